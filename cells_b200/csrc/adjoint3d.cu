@@ -14,12 +14,9 @@
 // Inflow: dJ/du_n from the inlet's feq(1, u_n) and the absorbing layer's target u_n, summed per
 // step in f64 with a fixed order.
 #include <algorithm>
-#include <atomic>
 #include <cmath>
 #include <cstring>
-#include <numeric>
 #include <string>
-#include <thread>
 #include <vector>
 
 #include "adjoint3d.h"
@@ -33,87 +30,150 @@ __host__ __device__ __forceinline__ long long off3(int i, int W, int H) {
   return (long long)cx3(i) + (long long)W * ((long long)cy3(i) + (long long)H * cz3(i));
 }
 
-template <class R>
-struct XRow {
-  R omP, omM, sigma;
+// Arithmetic on one cell's values (float, double) or on those of two x-neighbours (float2: the packed
+// f32x2 instructions of sm_100, each component rounding as the scalar instruction would).
+template <class V>
+struct Lane {
+  using R = V;
+  __device__ __forceinline__ static V bc(R v) { return v; }
+  __device__ __forceinline__ static V add(V a, V b) { return a + b; }
+  __device__ __forceinline__ static V sub(V a, V b) { return a - b; }
+  __device__ __forceinline__ static V mul(V a, V b) { return a * b; }
+  __device__ __forceinline__ static V fma(V a, V b, V c) { return ::fma(a, b, c); }
+  // f32: the hardware reciprocal (branch-free, within 2 ulp)
+  __device__ __forceinline__ static V recip(V a) {
+    if constexpr (sizeof(V) == 4)
+      return __fdividef(V(1), a);
+    else
+      return V(1) / a;
+  }
+  __device__ __forceinline__ static bool positive(V a) { return a > V(0); }
 };
+template <>
+struct Lane<float2> {
+  using R = float;
+  __device__ __forceinline__ static float2 bc(float v) { return make_float2(v, v); }
+  __device__ __forceinline__ static float2 add(float2 a, float2 b) { return __fadd2_rn(a, b); }
+  __device__ __forceinline__ static float2 sub(float2 a, float2 b) { return __ffma2_rn(b, make_float2(-1.0f, -1.0f), a); }
+  __device__ __forceinline__ static float2 mul(float2 a, float2 b) { return __fmul2_rn(a, b); }
+  __device__ __forceinline__ static float2 fma(float2 a, float2 b, float2 c) { return __ffma2_rn(a, b, c); }
+  __device__ __forceinline__ static float2 recip(float2 a) {
+    return make_float2(__fdividef(1.0f, a.x), __fdividef(1.0f, a.y));
+  }
+  __device__ __forceinline__ static bool positive(float2 a) { return a.x > 0.0f || a.y > 0.0f; }
+};
+
+// c_p . v for direction p
+template <class V>
+__device__ __forceinline__ V dot_c3(int p, const V (&v)[3]) {
+  using L = Lane<V>;
+  V r = L::bc(0);
+  bool any = false;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int c = k == 0 ? cx3(p) : (k == 1 ? cy3(p) : cz3(p));
+    if (c == 0) continue;
+    if (!any)
+      r = v[k];  // the first component of a pair's lower member is +1
+    else
+      r = c > 0 ? L::add(r, v[k]) : L::sub(r, v[k]);
+    any = true;
+  }
+  return r;
+}
 
 // (dC/dg)^T lp for the TRT collision with sponge rate omP/omM and absorbing strength sigma toward
 // the inflow speed ut (src/shaders/step3d.ts:38-102, Smagorinsky off). Also returns dJ/dut.
-// ABS = false: a cell known to lie outside the absorbing layer, compiled without its terms (as a
-// run-time branch the compiler evaluates them for every cell). f32 takes the hardware reciprocal.
-template <class R, bool ABS = true>
-__device__ __forceinline__ void collide_adjoint3(const R g[Q3], const R lp[Q3], R omP, R omM, R sigma, R ut,
-                                                 R lg[Q3], R& dut) {
-  R drho = R(0);
-#pragma unroll
-  for (int i = 0; i < Q3; i++) drho += g[i];
-  const R rho = R(1) + drho;
-  R inv;
-  if constexpr (sizeof(R) == 4)
-    inv = __fdividef(R(1), rho);
-  else
-    inv = R(1) / rho;
-  R jx = R(0), jy = R(0), jz = R(0);
-#pragma unroll
-  for (int i = 1; i < Q3; i++) {
-    jx += R(cx3(i)) * g[i];
-    jy += R(cy3(i)) * g[i];
-    jz += R(cz3(i)) * g[i];
-  }
-  const R ux = jx * inv, uy = jy * inv, uz = jz * inv;
-  const R uu = ux * ux + uy * uy + uz * uz;
-  const R usq = R(1.5) * uu;
-  const R w0 = w3<R>(0);
-  R rhoB = R(0), usqB = R(0), uxB = R(0), uyB = R(0), uzB = R(0), dqB = R(0), utB = R(0);
-  lg[0] = lp[0] * (R(1) - omP);
+// ABS = false: a cell known to lie outside the absorbing layer, compiled without its terms.
+//
+// With S, D = lp_a +- lp_b of each pair (a, b), s = omega+ w S, d = omega- w D and cu = 3 c_a . u:
+//   d/drho:  (1 - 3u^2/2) sum s + sum cu (s cu / 2 + d)      (s of the rest direction included)
+//   d/du:    3 rho sum c_a (s cu + d) - 3 u rho sum s
+//   lg_a, lg_b = (1 - omega+)/2 S + rhoB +- ((1 - omega-)/2 D + c_a . jB)
+// so a pair costs about 16 operations; written per direction with the pair's sums formed twice, the
+// kernel issued 850 thread instructions per cell and was bound by them.
+template <class V, bool ABS = true>
+__device__ __forceinline__ void collide_adjoint3(const V g[Q3], const V lp[Q3], V omP, V omM, V sigma,
+                                                 typename Lane<V>::R utS, V lg[Q3], V& dut) {
+  using L = Lane<V>;
+  using R = typename L::R;
+  const R w0 = w3<R>(0), w1 = w3<R>(1), w7 = w3<R>(7);
+  V u[3], rho, inv;
   {
-    const R e0 = omP * lp[0];
-    rhoB += e0 * w0 * (R(1) - usq);
-    usqB -= e0 * w0 * rho;
-  }
-  const bool absorb = ABS && sigma > R(0);
-  if (absorb) dqB -= lp[0] * sigma * w0;
+    V sum = g[0];
+    V j[3] = {L::bc(0), L::bc(0), L::bc(0)};
 #pragma unroll
-  for (int a = 1; a < Q3; a += 2) {
-    const int b = a + 1;
-    const R wa = w3<R>(a);
-    const R cu = R(3) * (R(cx3(a)) * ux + R(cy3(a)) * uy + R(cz3(a)) * uz);
-    const R S = lp[a] + lp[b];
-    const R Dd = lp[a] - lp[b];
-    lg[a] = lp[a] - R(0.5) * omP * S - R(0.5) * omM * Dd;
-    lg[b] = lp[b] - R(0.5) * omP * S + R(0.5) * omM * Dd;
-    const R eS = omP * S, eA = omM * Dd;
-    rhoB += eS * wa * (R(1) + R(0.5) * cu * cu - usq) + eA * wa * cu;
-    R cuB = eS * wa * rho * cu + eA * wa * rho;
-    usqB -= eS * wa * rho;
-    if (absorb) {
-      const R cut = R(3) * R(cx3(a)) * ut;
-      const R sw = sigma * wa;
-      rhoB += S * sw * R(0.5) * (cut * cut - cu * cu) + Dd * sw * (cut - cu);
-      cuB -= S * sw * rho * cu + Dd * sw * rho;
-      dqB -= S * sw;
-      utB += R(3) * R(cx3(a)) * (S * sw * rho * cut + Dd * sw * rho);
+    for (int p = 1; p < Q3; p += 2) {
+      sum = L::add(sum, L::add(g[p], g[p + 1]));
+      const V d = L::sub(g[p], g[p + 1]);
+      if (cx3(p) != 0) j[0] = cx3(p) > 0 ? L::add(j[0], d) : L::sub(j[0], d);
+      if (cy3(p) != 0) j[1] = cy3(p) > 0 ? L::add(j[1], d) : L::sub(j[1], d);
+      if (cz3(p) != 0) j[2] = cz3(p) > 0 ? L::add(j[2], d) : L::sub(j[2], d);
     }
-    uxB += R(3) * R(cx3(a)) * cuB;
-    uyB += R(3) * R(cy3(a)) * cuB;
-    uzB += R(3) * R(cz3(a)) * cuB;
-  }
-  if (absorb) {  // dq = 1.5 rho (ut^2 - |u|^2)
-    rhoB += dqB * R(1.5) * (ut * ut - uu);
-    uxB -= dqB * R(3) * rho * ux;
-    uyB -= dqB * R(3) * rho * uy;
-    uzB -= dqB * R(3) * rho * uz;
-    utB += dqB * R(3) * rho * ut;
-  }
-  uxB += R(3) * ux * usqB;
-  uyB += R(3) * uy * usqB;
-  uzB += R(3) * uz * usqB;
-  const R jxB = uxB * inv, jyB = uyB * inv, jzB = uzB * inv;
-  rhoB -= (ux * uxB + uy * uyB + uz * uzB) * inv;
+    rho = L::add(L::bc(1), sum);
+    inv = L::recip(rho);
 #pragma unroll
-  for (int i = 0; i < Q3; i++) lg[i] += rhoB + R(cx3(i)) * jxB + R(cy3(i)) * jyB + R(cz3(i)) * jzB;
-  dut = utB;
+    for (int k = 0; k < 3; k++) u[k] = L::mul(j[k], inv);
+  }
+  const V uu = L::fma(u[2], u[2], L::fma(u[1], u[1], L::mul(u[0], u[0])));
+  const V u3[3] = {L::mul(L::bc(3), u[0]), L::mul(L::bc(3), u[1]), L::mul(L::bc(3), u[2])};
+  const V sP[2] = {L::mul(omP, L::bc(w1)), L::mul(omP, L::bc(w7))};
+  const V sM[2] = {L::mul(omM, L::bc(w1)), L::mul(omM, L::bc(w7))};
+  const bool absorb = ABS && L::positive(sigma);
+  const V ut = L::bc(utS);
+  V S[Q3], D[Q3];  // entries p = 1, 3, .., 17
+  V sumS = L::mul(L::mul(omP, L::bc(w0)), lp[0]);
+  V rB = L::bc(0);
+  V T[3] = {L::bc(0), L::bc(0), L::bc(0)};
+  V dqB = L::bc(0), utA = L::bc(0);
+  if (absorb) dqB = L::mul(L::mul(L::bc(-w0), sigma), lp[0]);
+#pragma unroll
+  for (int p = 1; p < Q3; p += 2) {
+    const int k = p <= 5 ? 0 : 1;
+    S[p] = L::add(lp[p], lp[p + 1]);
+    D[p] = L::sub(lp[p], lp[p + 1]);
+    const V cu = dot_c3<V>(p, u3);
+    const V s = L::mul(sP[k], S[p]), d = L::mul(sM[k], D[p]);
+    sumS = L::add(sumS, s);
+    rB = L::fma(cu, L::fma(L::mul(L::bc(R(0.5)), s), cu, d), rB);
+    V t = L::fma(s, cu, d);
+    if (absorb) {
+      const V sw = L::mul(sigma, L::bc(k == 0 ? w1 : w7));
+      const V as = L::mul(sw, S[p]), ad = L::mul(sw, D[p]);
+      const V cut = L::mul(L::bc(R(3) * R(cx3(p))), ut);
+      const V dc = L::sub(cut, cu);
+      // as (cut^2 - cu^2) / 2 + ad (cut - cu)
+      rB = L::fma(dc, L::fma(L::mul(L::bc(R(0.5)), as), L::add(cut, cu), ad), rB);
+      t = L::sub(t, L::fma(as, cu, ad));
+      dqB = L::sub(dqB, as);
+      if (cx3(p) != 0) utA = L::fma(L::bc(R(cx3(p))), L::fma(as, cut, ad), utA);
+    }
+    if (cx3(p) != 0) T[0] = cx3(p) > 0 ? L::add(T[0], t) : L::sub(T[0], t);
+    if (cy3(p) != 0) T[1] = cy3(p) > 0 ? L::add(T[1], t) : L::sub(T[1], t);
+    if (cz3(p) != 0) T[2] = cz3(p) > 0 ? L::add(T[2], t) : L::sub(T[2], t);
+  }
+  const V rho3 = L::mul(L::bc(3), rho);
+  V rhoB = L::fma(L::fma(L::bc(R(-1.5)), uu, L::bc(1)), sumS, rB);
+  V uB[3];
+  // 3 rho (T - u sum s), and the absorbing layer's dq = 1.5 rho (ut^2 - |u|^2)
+  const V usq = absorb ? L::add(sumS, dqB) : sumS;
+#pragma unroll
+  for (int k = 0; k < 3; k++) uB[k] = L::mul(rho3, L::sub(T[k], L::mul(u[k], usq)));
+  dut = L::bc(0);
+  if (absorb) {
+    rhoB = L::fma(L::mul(L::bc(R(1.5)), dqB), L::sub(L::mul(ut, ut), uu), rhoB);
+    dut = L::mul(rho3, L::fma(dqB, ut, utA));
+  }
+  const V jB[3] = {L::mul(uB[0], inv), L::mul(uB[1], inv), L::mul(uB[2], inv)};
+  rhoB = L::sub(rhoB, L::fma(u[2], jB[2], L::fma(u[1], jB[1], L::mul(u[0], jB[0]))));
+  lg[0] = L::fma(L::sub(L::bc(1), omP), lp[0], rhoB);
+  const V hP = L::fma(L::bc(R(-0.5)), omP, L::bc(R(0.5))), hM = L::fma(L::bc(R(-0.5)), omM, L::bc(R(0.5)));
+#pragma unroll
+  for (int p = 1; p < Q3; p += 2) {
+    const V a = L::fma(hP, S[p], rhoB), b = L::fma(hM, D[p], dot_c3<V>(p, jB));
+    lg[p] = L::add(a, b);
+    lg[p + 1] = L::sub(a, b);
+  }
 }
 
 // (d feq(1, u(g)) / dg)^T lp: the outlet stores feq(1, u) with u the velocity of the pulled values.
@@ -147,12 +207,7 @@ __device__ __forceinline__ void outlet_adjoint3(const R g[Q3], const R lp[Q3], R
   for (int i = 0; i < Q3; i++) lg[i] = rhoB + R(cx3(i)) * jxB + R(cy3(i)) * jyB + R(cz3(i)) * jzB;
 }
 
-// The recorded step this adjoint step undoes: the segment's first step (device memory, written
-// before the segment's kernels run, so one captured graph serves every segment) plus the kernel's
-// position t within the segment.
-__device__ __forceinline__ int adj_step(const AdjLaunch3& a) { return __ldg(a.n0Dev) + a.t; }
-
-// The block's f64 sum of dJ/du_n into part[slot] (the rows kernel sums the slots in order).
+// The block's f64 sum of dJ/du_n into part[slot] (adj_du3_kernel sums the slots in order).
 __device__ __forceinline__ void block_du_partial(double du, double* part, int slot, double* red, int tid) {
   for (int o = 16; o > 0; o >>= 1) du += __shfl_down_sync(0xffffffffu, du, o);
   if ((tid & 31) == 0) red[tid >> 5] = du;
@@ -164,365 +219,755 @@ __device__ __forceinline__ void block_du_partial(double du, double* part, int sl
   }
 }
 
+// One adjoint step, one launch: blocks of 128 threads in a grid of z slices. The first roleZ slices
+// hold the listed flagged fluid cells (adj_slow_role) and, with x-pairs, the face rows
+// (adj_face_pairs_role), the others the rows y = 1 .. H-2 of the planes z = 1 .. D-2 in tiles of 4 rows of
+// 32 cells or pairs (every cell of the remaining rows is flagged). The roles write disjoint elements. The launch and the boundary-element kernel after it are programmatic
+// dependents of their predecessors: their blocks take the slots a finishing grid frees.
+//
+// What bounds it: memory. An adjoint step moves 228 bytes per f32 cell and the recompute beside it 152;
+// the adjoint states and the recomputed state together are larger than L2 at 128x64x64, where all of it
+// at the copy bandwidth takes 31 us. Per adjoint step there, recompute included (6,000 steps, K = 100):
+// 53 us with all 40k flagged cells in the list on a second stream, the per-direction collision and
+// the sum of dJ/du_n in the boundary-element kernel; 49 us as one launch with loads batched; 44 us with
+// the face rows as x-pairs, the packed collision, direct stores for links that are their source's only
+// reader, and f^n asked for before the dependency wait.
+
+// Programmatic dependent launch: waits for the boundary-element kernel of the step before to complete.
+// f^n, the tables and the flags do not depend on it (the recompute that wrote f^n ended before the
+// segment's first adjoint step, which follows an ordinary event), so the roles ask for them first.
+__device__ __forceinline__ void adj_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 template <class R>
-__global__ void __launch_bounds__(kAdjThreads) adj_cells3_kernel(AdjLaunch3 a) {
-  __shared__ double red[kAdjThreads / 32];
+__device__ __forceinline__ double adj_cells_role(const AdjLaunch3& a, int tz) {
   // a tile of x-rows per block (no division per cell); 32-bit element indices (19 N < 2^31)
   const int W = a.W, H = a.H;
   const int N = (int)a.N;
   const int x = blockIdx.x * blockDim.x + threadIdx.x;
-  const int y = blockIdx.y * blockDim.y + threadIdx.y;
-  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+  const int y = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+  if (x >= W || y >= H - 1) return 0.0;
   const R* __restrict__ f = (const R*)a.f;
   const R* __restrict__ lamNext = (const R*)a.lamNext;
   R* __restrict__ lamOut = (R*)a.lamOut;
-  double du = 0.0;
-  const int idx = x + W * (y + H * (int)blockIdx.z);
-  const bool in = x < W && y < H;
-  // the plain pulls and lambda^{n+1} go out with the flag load rather than after it: for every cell
-  // of the grid each address lies inside the 19 N arrays (no D3Q19 direction reaches further than
-  // one plane, and the arrays of directions 1 and 18 are not the first and last), and flagged cells
-  // discard the values
+  const int idx = x + W * (y + H * (1 + tz));
+  // the plain pulls go out with the flag load rather than after it: the sources of an interior row
+  // lie inside the 19 N arrays, and flagged cells discard the values
   R g[Q3], lp[Q3];
-  if (in) {
 #pragma unroll
-    for (int i = 0; i < Q3; i++) {
-      const int o = i * N + idx;
-      lp[i] = __ldg(&lamNext[o]);
-      g[i] = __ldg(&f[o - (int)off3(i, W, H)]);
-    }
-  }
-  const uint32_t fl = in ? __ldg(&a.flags[idx]) : FLAG3_SOLID;
-  if (fl == 0u) {
-    // interior cell: plain pulls, the collision's transposed Jacobian, plain pushes
-    R lg[Q3];
-    const R* xt = (const R*)a.xTab + 4 * x;
-    R dut = R(0);
-    // block-uniform: tiles that end before the absorbing layer take the code without it
-    if ((int)((blockIdx.x + 1) * blockDim.x) > a.absorbX0)
-      collide_adjoint3<R, true>(g, lp, xt[0], xt[1], xt[2], (R)__ldg(&a.uDev[adj_step(a)]), lg, dut);
-    else
-      collide_adjoint3<R, false>(g, lp, xt[0], xt[1], xt[2], (R)__ldg(&a.uDev[adj_step(a)]), lg, dut);
-    du = (double)dut;
+  for (int i = 0; i < Q3; i++) g[i] = __ldg(&f[i * N + idx - (int)off3(i, W, H)]);
+  const uint32_t fl = __ldg(&a.flags[idx]);
+  adj_wait();
 #pragma unroll
-    for (int i = 0; i < Q3; i++) lamOut[i * N + idx - (int)off3(i, W, H)] = lg[i];
-  }
-  // flagged fluid cells (faces, inlet, outlet, body) are done by adj_slow3_kernel
-  block_du_partial(du, a.blockPart, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z), red, tid);
+  for (int i = 0; i < Q3; i++) lp[i] = __ldg(&lamNext[i * N + idx]);
+  if (fl != 0u) return 0.0;
+  // interior cell: plain pulls, the collision's transposed Jacobian, plain pushes
+  R lg[Q3];
+  const R* xt = (const R*)a.xTab + 4 * x;
+  R dut;
+  // block-uniform: tiles that end before the absorbing layer take the code without it
+  if ((int)((blockIdx.x + 1) * blockDim.x) > a.absorbX0)
+    collide_adjoint3<R, true>(g, lp, xt[0], xt[1], xt[2], (R)a.u, lg, dut);
+  else
+    collide_adjoint3<R, false>(g, lp, xt[0], xt[1], xt[2], (R)a.u, lg, dut);
+#pragma unroll
+  for (int i = 0; i < Q3; i++) lamOut[i * N + idx - (int)off3(i, W, H)] = lg[i];
+  return (double)dut;
 }
 
-// The flagged fluid cells (faces, inlet, outlet, body), kSlowCells per block in three phases so
-// that their many independent loads are in flight together: (cell, direction) items pull through
-// the cells' records into shared memory; one thread per cell applies the transposed Jacobian of its
-// collision (or of the outlet equilibrium; the inlet only feeds dJ/du_n); (cell, direction) items
-// push the plain pulls' adjoints and store the links' adjoints (with dJ/dq of Bouzidi links).
+// f32 and an even width: the x-pair (x0, x0 + 1), x0 even, per thread. lambda^{n+1} and the
+// directions with c_x = 0 move as 8-byte words, and both cells go through one packed instruction stream.
+__device__ __forceinline__ double adj_pairs_role(const AdjLaunch3& a, int tz) {
+  const int W = a.W, H = a.H;
+  const int N = (int)a.N;
+  const int x0 = blockIdx.x * (2 * blockDim.x) + 2 * threadIdx.x;
+  const int y = 1 + blockIdx.y * blockDim.y + threadIdx.y;
+  if (x0 >= W || y >= H - 1) return 0.0;
+  const float* __restrict__ f = (const float*)a.f;
+  const float* __restrict__ lamNext = (const float*)a.lamNext;
+  float* __restrict__ lamOut = (float*)a.lamOut;
+  const int idx = x0 + W * (y + H * (1 + tz));
+  float2 g[Q3], lp[Q3];
+#pragma unroll
+  for (int i = 0; i < Q3; i++) {
+    const float* p = f + (i * N + idx - (int)off3(i, W, H));
+    g[i] = cx3(i) == 0 ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(__ldg(p), __ldg(p + 1));
+  }
+  const uint2 fl = __ldg(reinterpret_cast<const uint2*>(a.flags + idx));
+  adj_wait();
+#pragma unroll
+  for (int i = 0; i < Q3; i++) lp[i] = __ldg(reinterpret_cast<const float2*>(lamNext + (i * N + idx)));
+  if (fl.x != 0u && fl.y != 0u) return 0.0;
+  const float4* xt = (const float4*)a.xTab + x0;
+  const float4 t0 = __ldg(xt), t1 = __ldg(xt + 1);
+  const float2 omP = make_float2(t0.x, t1.x), omM = make_float2(t0.y, t1.y), sigma = make_float2(t0.z, t1.z);
+  float2 lg[Q3], dut;
+  if ((int)((blockIdx.x + 1) * 2 * blockDim.x) > a.absorbX0)
+    collide_adjoint3<float2, true>(g, lp, omP, omM, sigma, (float)a.u, lg, dut);
+  else
+    collide_adjoint3<float2, false>(g, lp, omP, omM, sigma, (float)a.u, lg, dut);
+  if (fl.x == 0u && fl.y == 0u) {
+#pragma unroll
+    for (int i = 0; i < Q3; i++) {
+      float* p = lamOut + (i * N + idx - (int)off3(i, W, H));
+      if (cx3(i) == 0) {
+        *reinterpret_cast<float2*>(p) = lg[i];
+      } else {
+        p[0] = lg[i].x;
+        p[1] = lg[i].y;
+      }
+    }
+    return (double)dut.x + (double)dut.y;
+  }
+  const int k = fl.x == 0u ? 0 : 1;  // the other cell is flagged
+#pragma unroll
+  for (int i = 0; i < Q3; i++) lamOut[i * N + idx + k - (int)off3(i, W, H)] = k ? lg[i].y : lg[i].x;
+  return (double)(k ? dut.y : dut.x);
+}
+
+// The x-pairs of a face row with one outside side (rows y = 1 .. H-2 of the z = 0 / z = D-1 planes,
+// sides 0 / 1; the y = 0 / y = H-1 rows of the planes between, sides 2 / 3) away from bodies: a
+// direction that enters from outside pulls the mirrored population of the same plane or row
+// (foff[side], as the forward step's face tiles). No other cell reads that element, so its adjoint is a
+// plain store as well. The row's inlet and outlet cells, and all cells of rows that hold a body cell, are
+// in the flagged-cell list.
+__device__ __forceinline__ double adj_face_pairs_role(const AdjLaunch3& a, int fb) {
+  const int W = a.W, H = a.H, D = a.D;
+  const int tilesX = gridDim.x, perPlane = gridDim.x * gridDim.y;
+  int side, tx, y, z;
+  if (fb < 2 * perPlane) {
+    side = fb >= perPlane ? 1 : 0;
+    const int rem = fb - side * perPlane, ty = rem / tilesX;
+    tx = rem - ty * tilesX;
+    y = 1 + ty * blockDim.y + threadIdx.y;
+    z = side ? D - 1 : 0;
+    if (y >= H - 1) return 0.0;
+  } else {
+    fb -= 2 * perPlane;
+    const int perSide = (D - 2 + (int)blockDim.y - 1) / (int)blockDim.y * tilesX;
+    side = fb >= perSide ? 3 : 2;
+    const int rem = fb - (side - 2) * perSide, gz = rem / tilesX;
+    tx = rem - gz * tilesX;
+    y = side == 3 ? H - 1 : 0;
+    z = 1 + gz * blockDim.y + threadIdx.y;
+    if (z >= D - 1) return 0.0;
+  }
+  const int x0 = tx * (2 * blockDim.x) + 2 * threadIdx.x;
+  const int row = y + H * z;
+  if (x0 >= W || a.rowBody[row]) return 0.0;
+  const float* __restrict__ f = (const float*)a.f;
+  const float* __restrict__ lamNext = (const float*)a.lamNext;
+  float* __restrict__ lamOut = (float*)a.lamOut;
+  const int N = (int)a.N, idx = x0 + W * row;
+  float2 g[Q3], lp[Q3];
+#pragma unroll
+  for (int i = 0; i < Q3; i++) {
+    const float* p = f + (idx + a.foff[side][i]);
+    g[i] = cx3(i) == 0 ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(__ldg(p), __ldg(p + 1));
+  }
+  adj_wait();
+#pragma unroll
+  for (int i = 0; i < Q3; i++) lp[i] = __ldg(reinterpret_cast<const float2*>(lamNext + (i * N + idx)));
+  const float4* xt = (const float4*)a.xTab + x0;
+  const float4 t0 = __ldg(xt), t1 = __ldg(xt + 1);
+  float2 lg[Q3], dut;
+  collide_adjoint3<float2, true>(g, lp, make_float2(t0.x, t1.x), make_float2(t0.y, t1.y), make_float2(t0.z, t1.z),
+                                 (float)a.u, lg, dut);
+  const bool on0 = x0 > 0, on1 = x0 + 1 < W - 1;
+#pragma unroll
+  for (int i = 0; i < Q3; i++) {
+    float* p = lamOut + (idx + a.foff[side][i]);
+    if (on0) p[0] = lg[i].x;
+    if (on1) p[1] = lg[i].y;
+  }
+  return (on0 ? (double)dut.x : 0.0) + (on1 ? (double)dut.y : 0.0);
+}
+
+// L2 prefetch for the tile one plane later: one 128-byte line per thread and turn, of the 19 pulls
+// and of lambda^{n+1}, as the forward step does it (a hint: every address is a source of an interior
+// row of that plane).
+template <class R, int TILEX>
+__device__ __forceinline__ void adj_prefetch(const AdjLaunch3& a, int tz, int tid) {
+  constexpr int kPer = 128 / (int)sizeof(R), kLines = TILEX / kPer, kRows = kAdjThreads / kAdjTileX;
+  constexpr int kSlots = kLines * kRows;  // lines of a tile per array
+  const int l = tid % kLines, r = tid / kLines % kRows;
+  const int y = 1 + blockIdx.y * kRows + r;
+  const int x = (int)blockIdx.x * TILEX + l * kPer + kPer / 2;
+  if (y >= a.H - 1 || x >= a.W - 1) return;
+  const long long cell = x + (long long)a.W * (y + (long long)a.H * (1 + tz));
+#pragma unroll
+  for (int q0 = 0; q0 < Q3; q0 += kAdjThreads / kSlots) {
+    const int i = q0 + tid / kSlots;
+    if (i >= Q3) break;
+    const long long o = i * a.N + cell;
+    asm volatile("prefetch.global.L2 [%0];" ::"l"((const R*)a.lamNext + o));
+    asm volatile("prefetch.global.L2 [%0];" ::"l"((const R*)a.f + (o - a.off[i])));
+  }
+}
+
+// The flagged fluid cells (faces, inlet, outlet, body), kSlowCells per block in three phases:
+// (cell, direction) items pull through the cells' records into shared memory; one thread per cell
+// applies the transposed Jacobian of its collision (or of the outlet equilibrium; the inlet only
+// feeds dJ/du_n); (cell, direction) items push the plain pulls' adjoints and store the links'
+// adjoints (with dJ/dq of Bouzidi links). A thread's five items share a cell; their loads go out
+// together, and what the last phase needs of them stays in registers.
 constexpr int kSlowCells = 32;
 
 template <class R>
-__global__ void __launch_bounds__(kAdjThreads) adj_slow3_kernel(AdjLaunch3 a) {
-  __shared__ double red[kAdjThreads / 32];
+__device__ __forceinline__ double adj_slow_role(const AdjLaunch3& a, int block, int tid) {
+  constexpr int kItems = (Q3 * kSlowCells + kAdjThreads - 1) / kAdjThreads;
+  constexpr int kDirs = kAdjThreads / kSlowCells;  // directions a round of the block's threads covers
   __shared__ R sg[Q3][kSlowCells + 1];
   __shared__ R slp[Q3][kSlowCells + 1];
   __shared__ R slg[Q3][kSlowCells + 1];
-  __shared__ uint32_t sfl[kSlowCells];
   const int N = (int)a.N;
   const int n = a.nSlow;
-  const int tid = threadIdx.x;
-  const int c0 = blockIdx.x * kSlowCells;
+  const int c = tid % kSlowCells, i0 = tid / kSlowCells;
+  const int s = block * kSlowCells + c;
+  const bool on = s < n;
   const R* __restrict__ f = (const R*)a.f;
   const R* __restrict__ lamNext = (const R*)a.lamNext;
   R* __restrict__ lamOut = (R*)a.lamOut;
   const R* sA1 = (const R*)a.sA1;
   const R* sA2 = (const R*)a.sA2;
-  for (int it = tid; it < Q3 * kSlowCells; it += kAdjThreads) {
-    const int c = it % kSlowCells, i = it / kSlowCells, s = c0 + c;
-    if (s >= n) continue;
-    const int idx = a.slowCells[s];
-    const int r = i * n + s;
-    slp[i][c] = lamNext[i * N + idx];
-    const int e = a.sE1[r];
-    if (e >= 0) {  // one source with coefficient 1: plain pulls, copies, mirrors, bounce-back
-      sg[i][c] = f[e];
-    } else {       // Bouzidi interpolation: two sources
-      sg[i][c] = sA1[r] * f[e & 0x7fffffff] + sA2[r] * f[a.sE2[r]];
+  const int idx = on ? a.slowCells[s] : 0;
+  const uint32_t fl = on ? a.flags[idx] : FLAG3_INLET;
+  int e[kItems], tgt[kItems];
+  R fj[kItems], f2[kItems], lp[kItems];
+#pragma unroll
+  for (int k = 0; k < kItems; k++) {
+    const int i = i0 + k * kDirs;
+    const bool item = on && i < Q3;
+    e[k] = item ? a.sE1[i * n + s] : 0;
+    tgt[k] = item ? a.sTgt[i * n + s] : 0;
+  }
+#pragma unroll
+  for (int k = 0; k < kItems; k++) {
+    fj[k] = f[e[k] & 0x7fffffff];
+    f2[k] = R(0);
+  }
+  adj_wait();
+#pragma unroll
+  for (int k = 0; k < kItems; k++) {
+    const int i = i0 + k * kDirs;
+    lp[k] = on && i < Q3 ? lamNext[i * N + idx] : R(0);
+  }
+#pragma unroll
+  for (int k = 0; k < kItems; k++) {
+    const int i = i0 + k * kDirs;
+    if (!on || i >= Q3) continue;
+    slp[i][c] = lp[k];
+    R v = fj[k];  // one source with coefficient 1: plain pulls, copies, mirrors, bounce-back
+    if (e[k] < 0) {  // Bouzidi interpolation: two sources
+      const int r = i * n + s;
+      f2[k] = f[a.sE2[r]];
+      v = sA1[r] * v + sA2[r] * f2[k];
     }
+    sg[i][c] = v;
   }
   __syncthreads();
   double du = 0.0;
-  if (tid < kSlowCells && c0 + tid < n) {
-    const int idx = a.slowCells[c0 + tid];
-    const uint32_t fl = a.flags[idx];
-    sfl[tid] = fl;
-    R g[Q3], lp[Q3], lg[Q3];
+  if (tid < kSlowCells && on) {
+    R g[Q3], lpc[Q3], lg[Q3];
 #pragma unroll
     for (int i = 0; i < Q3; i++) {
       g[i] = sg[i][tid];
-      lp[i] = slp[i][tid];
+      lpc[i] = slp[i][tid];
     }
-    const R u = (R)__ldg(&a.uDev[adj_step(a)]);
+    const R u = (R)a.u;
     if (fl & FLAG3_INLET) {
       // f' = feq(1, u, 0, 0): d/du = w_i (3 c_ix + 9 c_ix^2 u - 3 u); the inlet reads nothing
       R sum = R(0);
 #pragma unroll
       for (int i = 0; i < Q3; i++) {
-        const R c = R(cx3(i));
-        sum += lp[i] * w3<R>(i) * (R(3) * c + R(9) * c * c * u - R(3) * u);
+        const R cx = R(cx3(i));
+        sum += lpc[i] * w3<R>(i) * (R(3) * cx + R(9) * cx * cx * u - R(3) * u);
         lg[i] = R(0);
       }
       du = (double)sum;
     } else if (fl & FLAG3_OUTLET) {
-      outlet_adjoint3<R>(g, lp, lg);
+      outlet_adjoint3<R>(g, lpc, lg);
     } else {
       const R* xt = (const R*)a.xTab + 4 * (idx % a.W);
       R dut = R(0);
-      collide_adjoint3<R>(g, lp, xt[0], xt[1], xt[2], u, lg, dut);
+      collide_adjoint3<R>(g, lpc, xt[0], xt[1], xt[2], u, lg, dut);
       du = (double)dut;
     }
 #pragma unroll
     for (int i = 0; i < Q3; i++) slg[i][tid] = lg[i];
   }
   __syncthreads();
-  const R* lcF = (const R*)a.lcF;
-  const R* lq = (const R*)a.lq;
-  R* lamG = (R*)a.lamG;
-  const R w = (R)__ldg(&a.wDev[adj_step(a)]);
-  for (int it = tid; it < Q3 * kSlowCells; it += kAdjThreads) {
-    const int c = it % kSlowCells, i = it / kSlowCells, s = c0 + c;
-    if (s >= n || (sfl[c] & FLAG3_INLET)) continue;
-    const R v = slg[i][c];
-    const int t = a.sTgt[i * n + s];
-    if (t >= 0) {  // a plain pull: the element's only regular reader
-      lamOut[t] = v;
-    } else {       // a link: its adjoint, and dJ/dq of a Bouzidi link
-      const int k = -t - 1;
-      lamG[k] = v;
-      const int qk = a.lqk[k];
-      if (qk) {
-        const R fj = f[a.le1[k]], f2 = f[a.le2[k]], q = lq[k];
-        const R dgdq = qk == 1 ? R(2) * (fj - f2) : (f2 - fj) / (R(2) * q * q);
-        a.dqAcc[k] += (double)((v + w * lcF[k]) * dgdq);
+  if (!(fl & FLAG3_INLET)) {
+    const R w = (R)a.w;
+#pragma unroll
+    for (int k = 0; k < kItems; k++) {
+      const int i = i0 + k * kDirs;
+      if (i >= Q3) continue;
+      const R v = slg[i][c];
+      if (tgt[k] >= 0) {  // a plain pull: the element's only regular reader
+        lamOut[tgt[k]] = v;
+      } else {            // a link: its adjoint, and dJ/dq of a Bouzidi link
+        const int l = -tgt[k] - 1;
+        ((R*)a.lamG)[l] = v;
+        const int qk = e[k] < 0 ? a.lqk[l] : 0;  // only a two-source pull depends on q
+        if (qk) {
+          const R q = ((const R*)a.lq)[l];
+          const R dgdq = qk == 1 ? R(2) * (fj[k] - f2[k]) : (f2[k] - fj[k]) / (R(2) * q * q);
+          a.dqAcc[l] += (double)((v + w * ((const R*)a.lcF)[l]) * dgdq);
+        }
       }
     }
   }
-  block_du_partial(du, a.blockPart, a.nCellBlocks + (int)blockIdx.x, red, tid);
+  return du;
+}
+
+// PAIR: f32 with an even width. Five blocks per SM for f32 (up to 102 registers).
+template <class R, bool PAIR>
+__global__ void __launch_bounds__(kAdjThreads, PAIR ? 4 : (sizeof(R) == 4 ? 5 : 3)) adj_step3_kernel(AdjLaunch3 a) {
+  __shared__ double red[kAdjThreads / 32];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  const int tid = threadIdx.x + blockDim.x * threadIdx.y;
+  if ((int)blockIdx.z < a.roleZ) {
+    const int r = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+    if (r >= a.nSlowBlocks + a.nFaceBlocks) return;
+    double du = 0.0;
+    if (r < a.nSlowBlocks) {
+      du = adj_slow_role<R>(a, r, tid);
+    } else if constexpr (PAIR) {
+      du = adj_face_pairs_role(a, r - a.nSlowBlocks);
+    }
+    block_du_partial(du, a.blockPart, a.nCellBlocks + r, red, tid);
+  } else {
+    const int tz = blockIdx.z - a.roleZ;
+    if (tz + 1 < a.D - 2) adj_prefetch<R, (PAIR ? 2 : 1) * kAdjTileX>(a, tz + 1, tid);
+    double du;
+    if constexpr (PAIR)
+      du = adj_pairs_role(a, tz);
+    else
+      du = adj_cells_role<R>(a, tz);
+    block_du_partial(du, a.blockPart, blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * tz), red, tid);
+  }
 }
 
 // Elements with an irregular reader or no regular reader: lambda^n[e] (= 0 when no regular reader
 // wrote it) plus each link's adjoint times its coefficient, plus the direct force terms.
 template <class R>
 __global__ void __launch_bounds__(256) adj_rows3_kernel(AdjLaunch3 a) {
-  if (blockIdx.x == gridDim.x - 1) {
-    // the extra last block: dJ/du_n = the cell kernel's block sums, strided per thread, then in order
-    __shared__ double red[8];
-    double s = 0.0;
-    for (int k = threadIdx.x; k < a.nParts; k += 256) s += a.blockPart[k];
-    for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
-    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-      double t = 0.0;
-      for (int k = 0; k < 8; k++) t += red[k];
-      a.dudn[adj_step(a)] = t;
-    }
-    return;
-  }
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int r = blockIdx.x * blockDim.x + threadIdx.x;
-  if (r >= a.nRows) return;
-  R* lamOut = (R*)a.lamOut;
+  const bool on = r < a.nRows;
+  // the row's own record does not depend on the step before: it goes out before the wait, with the first
+  // entries (few rows have more)
+  constexpr int kHead = 4;
+  const int e = on ? a.rowElem[r] : 0;
+  const int k0 = on ? a.rowStart[r] : 0, k1 = on ? a.rowStart[r + 1] : 0;
+  const bool set = on && a.rowSet[r];
+  const R phi = on ? ((const R*)a.rowPhi)[r] : R(0);
   const R* lamG = (const R*)a.lamG;
   const R* lcF = (const R*)a.lcF;
   const R* alpha = (const R*)a.entAlpha;
-  const R w = (R)__ldg(&a.wDev[adj_step(a)]);
-  const long long e = a.rowElem[r];
-  R v = a.rowSet[r] ? R(0) : lamOut[e];
-  for (int k = a.rowStart[r]; k < a.rowStart[r + 1]; k++) {
+  int link[kHead];
+  R al[kHead], cF[kHead];
+#pragma unroll
+  for (int k = 0; k < kHead; k++) {
+    link[k] = k0 + k < k1 ? a.entLink[k0 + k] : 0;
+    al[k] = k0 + k < k1 ? alpha[k0 + k] : R(0);
+  }
+#pragma unroll
+  for (int k = 0; k < kHead; k++) cF[k] = k0 + k < k1 ? lcF[link[k]] : R(0);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  if (!on) return;
+  R* lamOut = (R*)a.lamOut;
+  const R w = (R)a.w;
+  R v = set ? R(0) : lamOut[e];
+  R lam[kHead];
+#pragma unroll
+  for (int k = 0; k < kHead; k++) lam[k] = k0 + k < k1 ? lamG[link[k]] : R(0);
+#pragma unroll
+  for (int k = 0; k < kHead; k++)
+    if (k0 + k < k1) v += al[k] * (lam[k] + w * cF[k]);
+  for (int k = k0 + kHead; k < k1; k++) {
     const int L = a.entLink[k];
     v += alpha[k] * (lamG[L] + w * lcF[L]);
   }
-  v += w * ((const R*)a.rowPhi)[r];
+  v += w * phi;
   lamOut[e] = v;
 }
 
-template <class R>
-cudaError_t launch_adjoint_step3_t(const AdjLaunch3& a, cudaStream_t s, cudaStream_t side, cudaEvent_t fork,
-                                   cudaEvent_t join) {
-  const dim3 block(a.tileX, kAdjThreads / a.tileX);
-  const dim3 grid((unsigned)((a.W + block.x - 1) / block.x), (unsigned)((a.H + block.y - 1) / block.y),
-                  (unsigned)a.D);
-  if ((long long)grid.x * grid.y * grid.z != a.nCellBlocks) return cudaErrorInvalidValue;
-  const int slowBlocks = (a.nSlow + kSlowCells - 1) / kSlowCells;
-  if (a.nCellBlocks + slowBlocks != a.nParts) return cudaErrorInvalidValue;
-  cudaError_t e;
-  if (slowBlocks > 0) {  // the flagged cells on the side stream, beside the interior cells
-    if ((e = cudaEventRecord(fork, s)) != cudaSuccess) return e;
-    if ((e = cudaStreamWaitEvent(side, fork, 0)) != cudaSuccess) return e;
-    adj_slow3_kernel<R><<<slowBlocks, kAdjThreads, 0, side>>>(a);
-    if ((e = cudaGetLastError()) != cudaSuccess) return e;
-    if ((e = cudaEventRecord(join, side)) != cudaSuccess) return e;
+// After a segment: dJ/du_n of its steps, one block each, from the steps' block sums (strided per
+// thread, then in order).
+__global__ void __launch_bounds__(256) adj_du3_kernel(const double* __restrict__ part, int nParts,
+                                                      double* __restrict__ dudn) {
+  __shared__ double red[8];
+  const double* p = part + (size_t)blockIdx.x * nParts;
+  double s = 0.0;
+  for (int k = threadIdx.x; k < nParts; k += 256) s += p[k];
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = s;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    double t = 0.0;
+    for (int k = 0; k < 8; k++) t += red[k];
+    dudn[blockIdx.x] = t;
   }
-  adj_cells3_kernel<R><<<grid, block, 0, s>>>(a);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (slowBlocks > 0 && (e = cudaStreamWaitEvent(s, join, 0)) != cudaSuccess) return e;
-  adj_rows3_kernel<R><<<(unsigned)((a.nRows + 255) / 256) + 1, 256, 0, s>>>(a);
-  return cudaGetLastError();
+}
+
+template <class... Args>
+cudaError_t launch_dependent(void (*fn)(Args...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.stream = s;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, fn, args...);
+}
+
+// Interior-cell blocks of a step: x tiles of 32 cells (or 32 x-pairs), so each warp still reads
+// 128-byte rows and the tiles before the absorbing layer take the collision code without it.
+bool adj_pairs(int precision, int W) { return precision == 0 && W % 2 == 0; }
+
+dim3 adj_cell_grid(int precision, int W, int H, int D) {
+  const int tileY = kAdjThreads / kAdjTileX, tileX = adj_pairs(precision, W) ? 2 * kAdjTileX : kAdjTileX;
+  const unsigned gx = (unsigned)((W + tileX - 1) / tileX);
+  if (H < 3 || D < 3) return dim3(gx, 1, 0);  // every cell is flagged
+  return dim3(gx, (unsigned)((H - 2 + tileY - 1) / tileY), (unsigned)(D - 2));
+}
+
+// Blocks of the face rows: tiles of the two z planes, and of the two y rows of the planes between.
+int adj_face_blocks(int precision, int W, int H, int D, dim3 cells) {
+  if (!adj_pairs(precision, W) || H < 3 || D < 3) return 0;
+  const int rows = kAdjThreads / kAdjTileX;
+  return (int)(2 * cells.x * cells.y + 2 * cells.x * ((D - 2 + rows - 1) / rows));
+}
+
+template <class R>
+cudaError_t launch_adjoint_step3_t(AdjLaunch3 a, cudaStream_t s) {
+  const int precision = sizeof(R) == 4 ? 0 : 3;
+  const dim3 cells = adj_cell_grid(precision, a.W, a.H, a.D);
+  a.nCellBlocks = (int)(cells.x * cells.y * cells.z);
+  for (int i = 0; i < Q3; i++) a.off[i] = (int)off3(i, a.W, a.H);
+  a.nSlowBlocks = (a.nSlow + kSlowCells - 1) / kSlowCells;
+  a.nFaceBlocks = adj_face_blocks(precision, a.W, a.H, a.D, cells);
+  if (a.nCellBlocks + a.nSlowBlocks + a.nFaceBlocks != a.nParts) return cudaErrorInvalidValue;
+  for (int side = 0; side < 4; side++) {
+    for (int i = 0; i < Q3; i++) {
+      const bool out = side == 0 ? cz3(i) == 1 : (side == 1 ? cz3(i) == -1 : (side == 2 ? cy3(i) == 1 : cy3(i) == -1));
+      const int pop = !out ? i : (side < 2 ? mirror_z3(i) : mirror_y3(i));
+      const int off = !out ? a.off[i] : (side < 2 ? cx3(i) + a.W * cy3(i) : cx3(i) + a.W * a.H * cz3(i));
+      a.foff[side][i] = (int)((long long)pop * a.N - off);
+    }
+  }
+  const unsigned slice = cells.x * cells.y;
+  a.roleZ = (int)(((unsigned)(a.nSlowBlocks + a.nFaceBlocks) + slice - 1) / slice);
+  if (a.roleZ + cells.z > 0) {
+    void (*fn)(AdjLaunch3) = adj_step3_kernel<R, false>;
+    if constexpr (sizeof(R) == 4) {
+      if (adj_pairs(precision, a.W)) fn = adj_step3_kernel<R, true>;
+    }
+    const cudaError_t e = launch_dependent(fn, dim3(cells.x, cells.y, a.roleZ + cells.z),
+                                           dim3(kAdjTileX, kAdjThreads / kAdjTileX), s, a);
+    if (e != cudaSuccess) return e;
+  }
+  if (a.nRows == 0) return cudaSuccess;
+  return launch_dependent(adj_rows3_kernel<R>, dim3((unsigned)((a.nRows + 255) / 256)), dim3(256), s, a);
 }
 
 }  // namespace
 
 namespace cells {
-cudaError_t launch_adjoint_step3(int precision, const AdjLaunch3& a, cudaStream_t s, cudaStream_t side,
-                                 cudaEvent_t fork, cudaEvent_t join) {
-  if (precision == 0) return launch_adjoint_step3_t<float>(a, s, side, fork, join);
-  if (precision == 3) return launch_adjoint_step3_t<double>(a, s, side, fork, join);
+cudaError_t launch_adjoint_step3(int precision, const AdjLaunch3& a, cudaStream_t s) {
+  if (precision == 0) return launch_adjoint_step3_t<float>(a, s);
+  if (precision == 3) return launch_adjoint_step3_t<double>(a, s);
   return cudaErrorInvalidValue;
 }
 }  // namespace cells
 
-// ---------------- host: link resolution (the rules of pullSlow3, src/shaders/step3d.ts:119-168) ----
+// ---------------- the recorded run's tables, built on the device ----------------
+//
+// Once per recorded run (on the host they took 50 ms of a 128x64x64 gradient, more than the forward
+// run of 1,000 steps). The links follow the rules of pullSlow3 (src/shaders/step3d.ts:119-168).
+// Rows gather what several readers, or a reader with a coefficient, send to one element; their order
+// is of no account, and each row adds its entries in link order.
 
 namespace {
 
-// Host threads for the table builds: the machine's, at most 16.
-int table_threads() {
-  const unsigned n = std::thread::hardware_concurrency();
-  return (int)std::max(1u, std::min(16u, n));
+// Whether a flagged fluid cell is listed: all but those adj_face_pairs_role takes.
+__device__ __forceinline__ bool adj_listed(const AdjTables3& t, int x, int y, int z, uint32_t fl) {
+  if (fl == 0u || (fl & FLAG3_SOLID)) return false;
+  const bool zFace = z == 0 || z == t.D - 1, yFace = y == 0 || y == t.H - 1;
+  const bool face = t.facePairs && zFace != yFace && x > 0 && x < t.W - 1 && !t.rowBody[y + t.H * z];
+  return !face;
 }
 
-// Runs fn(t) for t = 0 .. n-1 on n host threads (t = 0 on the caller's).
-template <class F>
-void run_threads(int n, F fn) {
-  std::vector<std::thread> pool;
-  for (int t = 1; t < n; t++) pool.emplace_back(fn, t);
-  fn(0);
-  for (std::thread& th : pool) th.join();
+// Listed cells of each row, one warp per row: their number, or with `offset` the cells themselves.
+__global__ void adj_list3_kernel(AdjTables3 t, int* __restrict__ counts, const int* __restrict__ offset,
+                                 int* __restrict__ cells) {
+  const int row = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+  if (row >= t.H * t.D) return;
+  const int z = row / t.H, y = row - z * t.H;
+  int n = offset ? offset[row] : 0;
+  for (int x0 = 0; x0 < t.W; x0 += 32) {
+    const int x = x0 + lane;
+    const bool in = x < t.W && adj_listed(t, x, y, z, t.flags[x + t.W * row]);
+    const unsigned m = __ballot_sync(0xffffffffu, in);
+    if (in && offset) cells[n + __popc(m & ((1u << lane) - 1u))] = x + t.W * row;
+    n += __popc(m);
+  }
+  if (!offset && lane == 0) counts[row] = n;
 }
 
-// The links of the flagged fluid cells of planes z0 .. z1-1, in cell order; base[idx] is set to the
-// first link of each such cell, counted within this slab's links.
-template <class R>
-void resolve_links_slab(const Cells3D* h, const std::vector<uint32_t>& fl, const std::vector<float>& sdf, int comp,
-                        int z0, int z1, std::vector<int>& base, std::vector<AdjLink3Host>& links) {
-  const int W = h->W, H = h->H, D = h->D;
-  const long long N = h->N;
-  auto at = [&](int x, int y, int z) { return (long long)x + (long long)W * ((long long)y + (long long)H * z); };
-  auto solid = [&](long long c) { return (fl[(size_t)c] & FLAG3_SOLID) != 0u; };
-  auto cc = [&](int j) { return comp == 0 ? cx3(j) : (comp == 1 ? cy3(j) : cz3(j)); };
-  links.clear();
-  for (int z = z0; z < z1; z++)
-    for (int y = 0; y < H; y++)
-      for (int x = 0; x < W; x++) {
-        const long long idx = at(x, y, z);
-        const uint32_t f = fl[(size_t)idx];
-        if (f == 0u || (f & (FLAG3_SOLID | FLAG3_INLET))) continue;
-        const bool outlet = (f & FLAG3_OUTLET) != 0u;
-        bool any = false;
-        for (int i = 1; i < Q3; i++) {
-          if (!(f & (1u << i))) continue;
-          if (!any) {
-            base[(size_t)idx] = (int)links.size();
-            any = true;
-          }
-          AdjLink3Host L{};
-          L.e2 = -1;
-          L.a1 = 1.0;
-          L.a2 = 0.0;
-          L.cell = (int)idx;
-          L.solid = -1;
-          const int j = opp3(i);
-          const int sx = x - cx3(i), sy = y - cy3(i), sz = z - cz3(i);
-          const bool outX = sx < 0 || sx >= W, outY = sy < 0 || sy >= H, outZ = sz < 0 || sz >= D;
-          if (outX && outlet) {
-            L.e1 = i * N + at(W - 2, y, z);
-          } else if (outY && outZ) {
-            L.e1 = j * N + idx;
-          } else if (outY || outZ) {
-            int rx = sx, ry = sy, rz = sz, m = mirror_y3(i);
-            if (outY) {
-              ry = y;
-            } else {
-              rz = z;
-              m = mirror_z3(i);
-            }
-            const long long rs = at(rx, ry, rz);
-            if (solid(rs)) {  // a body meets a slip face: bounce-back with force 2 c_j f_j
-              L.e1 = j * N + idx;
-              L.cF = cc(j);
-            } else {
-              L.e1 = m * N + rs;
-            }
-          } else if (outX) {
-            L.e1 = j * N + idx;
-          } else {
-            const long long s = at(sx, sy, sz);
-            if (!solid(s)) {
-              L.e1 = i * N + s;
-            } else {
-              // Bouzidi: q in the arithmetic type, as the step kernel computes it
-              const R dF = (R)sdf[(size_t)idx], dS = (R)sdf[(size_t)s];
-              const R den = std::max(dF - dS, (R)1e-6);
-              const R raw = dF / den;
-              const R q = std::min(std::max(raw, (R)1e-3), R(1));
-              L.e1 = j * N + idx;
-              L.cF = cc(j);
-              L.q = (double)q;
-              L.cell = (int)idx;
-              L.solid = (int)s;
-              const bool free = raw > (R)1e-3 && raw < R(1) && (dF - dS) > (R)1e-6;
-              if (free) {
-                L.dqdF = -(double)dS / ((double)den * (double)den);
-                L.dqdS = (double)dF / ((double)den * (double)den);
-              }
-              if (q < R(0.5)) {
-                const int nx = x + cx3(i), ny = y + cy3(i), nz = z + cz3(i);
-                if (nx >= 0 && nx < W && ny >= 0 && ny < H && nz >= 0 && nz < D && !solid(at(nx, ny, nz))) {
-                  L.a1 = (double)(R(2) * q);
-                  L.e2 = j * N + at(nx, ny, nz);
-                  L.a2 = (double)(R(1) - R(2) * q);
-                  L.qKind = 1;
-                }
-              } else {
-                L.a1 = (double)(R(1) / (R(2) * q));
-                L.e2 = i * N + idx;
-                L.a2 = (double)((R(2) * q - R(1)) / (R(2) * q));
-                L.qKind = 2;
-              }
-            }
-          }
-          links.push_back(L);
-        }
+// Links of each listed cell: its flagged directions (the inlet reads nothing).
+__global__ void adj_link_count3_kernel(AdjTables3 t, const int* __restrict__ cells, int n, int* __restrict__ counts) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  if (c >= n) return;
+  const uint32_t fl = t.flags[cells[c]];
+  counts[c] = (fl & FLAG3_INLET) ? 0 : __popc(fl & (((1u << Q3) - 1u) & ~1u));
+}
+
+// Exclusive scan of n counts by one block, in place; the total to counts[n].
+__global__ void __launch_bounds__(1024) adj_scan3_kernel(int* __restrict__ counts, int n) {
+  __shared__ int warpSum[32];
+  __shared__ int carry;
+  const int tid = threadIdx.x, lane = tid & 31;
+  if (tid == 0) carry = 0;
+  __syncthreads();
+  for (int base = 0; base < n; base += 1024) {
+    const int k = base + tid;
+    const int v = k < n ? counts[k] : 0;
+    int s = v;
+    for (int o = 1; o < 32; o <<= 1) {
+      const int u = __shfl_up_sync(0xffffffffu, s, o);
+      if (lane >= o) s += u;
+    }
+    if (lane == 31) warpSum[tid >> 5] = s;
+    __syncthreads();
+    if (tid < 32) {
+      int w = warpSum[tid];
+      for (int o = 1; o < 32; o <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, w, o);
+        if (lane >= o) w += u;
       }
+      warpSum[tid] = w;
+    }
+    __syncthreads();
+    const int before = carry + (tid >= 32 ? warpSum[(tid >> 5) - 1] : 0) + s - v;
+    if (k < n) counts[k] = before;
+    __syncthreads();
+    if (tid == 1023) carry = before + v;
+    __syncthreads();
+  }
+  if (tid == 0) counts[n] = carry;
 }
 
-// The link records of every flagged fluid cell in cell order (the order a sequential pass gives),
-// built by slabs of planes on host threads and joined.
+// The pull records of each listed cell's 19 directions and its links, one thread per cell; every link's
+// sources are counted into cnt (per element).
 template <class R>
-void resolve_links(const Cells3D* h, const std::vector<uint32_t>& fl, const std::vector<float>& sdf, int comp,
-                   std::vector<int>& base, std::vector<AdjLink3Host>& links) {
-  const int D = h->D;
-  const long long plane = (long long)h->W * h->H;
-  base.assign((size_t)h->N, -1);
-  const int T = std::min(table_threads(), D);
-  std::vector<std::vector<AdjLink3Host>> part((size_t)T);
-  auto z_begin = [&](int t) { return (int)((long long)D * t / T); };
-  run_threads(T, [&](int t) { resolve_links_slab<R>(h, fl, sdf, comp, z_begin(t), z_begin(t + 1), base, part[(size_t)t]); });
-  std::vector<int> offset((size_t)T + 1, 0);
-  for (int t = 0; t < T; t++) offset[(size_t)t + 1] = offset[(size_t)t] + (int)part[(size_t)t].size();
-  run_threads(T, [&](int t) {
-    const int o = offset[(size_t)t];
-    if (o == 0) return;
-    for (long long c = z_begin(t) * plane; c < z_begin(t + 1) * plane; c++)
-      if (base[(size_t)c] >= 0) base[(size_t)c] += o;
-  });
-  links.clear();
-  links.reserve((size_t)offset[(size_t)T]);
-  for (auto& p : part) links.insert(links.end(), p.begin(), p.end());
+__global__ void adj_links3_kernel(AdjTables3 t, AdjLaunch3 a, const int* __restrict__ linkBase, AdjLinkQ3* __restrict__ linkQ,
+                                  int* __restrict__ sE1, int* __restrict__ sE2, int* __restrict__ sTgt,
+                                  R* __restrict__ sA1, R* __restrict__ sA2, R* __restrict__ lcF, R* __restrict__ lq,
+                                  signed char* __restrict__ lqk, int* __restrict__ cnt) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x;
+  const int n = a.nSlow;
+  if (c >= n) return;
+  const int W = t.W, H = t.H, D = t.D;
+  const int N = (int)t.N;  // 19 N < 2^31
+  const int idx = a.slowCells[c];
+  const int z = idx / (W * H), y = idx / W - z * H, x = idx % W;
+  const uint32_t fl = t.flags[idx];
+  const bool inlet = (fl & FLAG3_INLET) != 0u, outlet = (fl & FLAG3_OUTLET) != 0u;
+  auto at = [&](int qx, int qy, int qz) { return qx + W * (qy + H * qz); };
+  auto solid = [&](int cell) { return (t.flags[cell] & FLAG3_SOLID) != 0u; };
+  int k = linkBase[c];
+  for (int i = 0; i < Q3; i++) {
+    const int r = i * n + c;
+    if (inlet) {  // the inlet reads nothing
+      sE1[r] = sE2[r] = sTgt[r] = 0;
+      sA1[r] = sA2[r] = R(0);
+      continue;
+    }
+    if (i == 0 || !(fl & (1u << i))) {
+      const int e = i * N + idx - a.off[i];
+      sE1[r] = sE2[r] = sTgt[r] = e;
+      sA1[r] = R(1);
+      sA2[r] = R(0);
+      continue;
+    }
+    const int j = opp3(i);
+    const int sx = x - cx3(i), sy = y - cy3(i), sz = z - cz3(i);
+    const bool outX = sx < 0 || sx >= W, outY = sy < 0 || sy >= H, outZ = sz < 0 || sz >= D;
+    const int comp = t.component;
+    const int cc = comp == 0 ? cx3(j) : (comp == 1 ? cy3(j) : cz3(j));
+    int e1, e2 = -1, cF = 0, qKind = 0;
+    R a1 = R(1), a2 = R(0), q = R(0);
+    AdjLinkQ3 Q{0.0, 0.0, -1, -1};
+    if (outX && outlet) {
+      e1 = i * N + at(W - 2, y, z);
+    } else if (outY && outZ) {
+      e1 = j * N + idx;
+    } else if (outY || outZ) {
+      const int rs = at(sx, outY ? y : sy, outY ? sz : z);
+      if (solid(rs)) {  // a body meets a slip face: bounce-back with force 2 c_j f_j
+        e1 = j * N + idx;
+        cF = cc;
+      } else {
+        e1 = (outY ? mirror_y3(i) : mirror_z3(i)) * N + rs;
+      }
+    } else if (outX) {
+      e1 = j * N + idx;
+    } else {
+      const int s = at(sx, sy, sz);
+      if (!solid(s)) {
+        e1 = i * N + s;
+      } else {
+        // Bouzidi: q in the arithmetic type, as the step kernel computes it
+        const R dF = (R)t.sdf[idx], dS = (R)t.sdf[s];
+        const R den = max(dF - dS, (R)1e-6);
+        const R raw = dF / den;
+        q = min(max(raw, (R)1e-3), R(1));
+        e1 = j * N + idx;
+        cF = cc;
+        Q.cell = idx;
+        Q.solid = s;
+        if (raw > (R)1e-3 && raw < R(1) && (dF - dS) > (R)1e-6) {
+          Q.dqdF = -(double)dS / ((double)den * (double)den);
+          Q.dqdS = (double)dF / ((double)den * (double)den);
+        }
+        if (q < R(0.5)) {
+          const int nx = x + cx3(i), ny = y + cy3(i), nz = z + cz3(i);
+          if (nx >= 0 && nx < W && ny >= 0 && ny < H && nz >= 0 && nz < D && !solid(at(nx, ny, nz))) {
+            a1 = R(2) * q;
+            e2 = j * N + at(nx, ny, nz);
+            a2 = R(1) - R(2) * q;
+            qKind = 1;
+          }
+        } else {
+          a1 = R(1) / (R(2) * q);
+          e2 = i * N + idx;
+          a2 = (R(2) * q - R(1)) / (R(2) * q);
+          qKind = 2;
+        }
+        if (qKind == 0) Q.solid = -1;  // its pull does not depend on q
+      }
+    }
+    // one source with coefficient 1 is the plain index; else the sign bit marks the two sources
+    sE1[r] = e2 < 0 ? e1 : (int)((uint32_t)e1 | 0x80000000u);
+    sE2[r] = e2 >= 0 ? e2 : e1;
+    sA1[r] = a1;
+    sA2[r] = a2;
+    sTgt[r] = -(k + 1);
+    lcF[k] = (R)cF;
+    lq[k] = q;
+    lqk[k] = (signed char)qKind;
+    linkQ[k] = Q;
+    atomicAdd(cnt + e1, 1);
+    if (e2 >= 0) atomicAdd(cnt + e2, 1);
+    k++;
+  }
+}
+
+// Whether a plain store writes element e's adjoint: its regular reader is a fluid cell that pulls e's
+// direction without a rule, or e leaves the grid through a slip face and the cell that pulls its mirror
+// image is one of adj_face_pairs_role's.
+__device__ __forceinline__ bool adj_regular(const AdjTables3& t, int e) {
+  const int i = e / (int)t.N, cell = e - i * (int)t.N;
+  const int z = cell / (t.W * t.H), y = cell / t.W - z * t.H, x = cell % t.W;
+  const int rx = x + cx3(i), ry = y + cy3(i), rz = z + cz3(i);
+  if (rx < 0 || rx >= t.W) return false;
+  const bool outY = ry < 0 || ry >= t.H, outZ = rz < 0 || rz >= t.D;
+  if (outY || outZ) {
+    if (!t.facePairs || (outY && outZ)) return false;
+    const int my = outY ? y : ry, mz = outZ ? z : rz;
+    const uint32_t m = t.flags[rx + t.W * (my + t.H * mz)];
+    return m != 0u && !(m & FLAG3_SOLID) && !adj_listed(t, rx, my, mz, m);
+  }
+  const uint32_t g = t.flags[rx + t.W * (ry + t.H * rz)];
+  return !(g & (FLAG3_SOLID | FLAG3_INLET)) && (i == 0 || !(g & (1u << i)));
+}
+
+// Links whose only source has no other reader store their adjoint there (their target becomes the
+// element). The elements of the others become rows: the first of an element's readers to come takes
+// the row's number. Elements that nothing reads keep the zero of the cleared adjoint states.
+template <class R>
+__global__ void adj_claim3_kernel(AdjTables3 t, int n, const int* __restrict__ sE1, const int* __restrict__ sE2,
+                                  int* __restrict__ sTgt, const R* __restrict__ lcF, const int* __restrict__ cnt,
+                                  int* __restrict__ rowOf, int* __restrict__ rowElem, int* __restrict__ rowStart,
+                                  int* __restrict__ nRows) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+  if (c >= n) return;
+  const int r = i * n + c;
+  if (sTgt[r] >= 0) return;
+  const bool two = sE1[r] < 0;
+  const int e1 = sE1[r] & 0x7fffffff;
+  if (!two && cnt[e1] == 1 && lcF[-sTgt[r] - 1] == R(0) && !adj_regular(t, e1)) {
+    sTgt[r] = e1;
+    return;
+  }
+  for (int s = 0; s < (two ? 2 : 1); s++) {
+    const int e = s ? sE2[r] : e1;
+    if (atomicCAS(rowOf + e, 0, -1) != 0) continue;
+    const int row = atomicAdd(nRows, 1);
+    rowElem[row] = e;
+    rowStart[row] = cnt[e];
+    rowOf[e] = row + 1;
+  }
 }
 
 template <class R>
-void upload_typed(cells::Device& dev, void* d, const std::vector<double>& v) {
-  std::vector<R> t(v.begin(), v.end());
-  if (!t.empty()) dev.h2d(d, t.data(), t.size() * sizeof(R));
-  dev.sync();
+__global__ void adj_entries3_kernel(int n, const int* __restrict__ sE1, const int* __restrict__ sE2,
+                                    const int* __restrict__ sTgt, const R* __restrict__ sA1, const R* __restrict__ sA2,
+                                    const int* __restrict__ rowOf, const int* __restrict__ rowStart,
+                                    int* __restrict__ fill, int* __restrict__ entLink, R* __restrict__ entAlpha) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+  if (c >= n) return;
+  const int r = i * n + c;
+  if (sTgt[r] >= 0) return;
+  const bool two = sE1[r] < 0;
+  for (int s = 0; s < (two ? 2 : 1); s++) {
+    const int row = rowOf[s ? sE2[r] : (sE1[r] & 0x7fffffff)] - 1;
+    const int p = rowStart[row] + atomicAdd(fill + row, 1);
+    entLink[p] = -sTgt[r] - 1;
+    entAlpha[p] = s ? sA2[r] : (two ? sA1[r] : R(1));
+  }
+}
+
+// Each row's entries in link order (a row has a handful), the sum of its force links' coefficients
+// (those that read the element as f_j, their first source), and whether a plain pull writes it.
+template <class R>
+__global__ void adj_rows_build3_kernel(AdjTables3 t, int nRows, const int* __restrict__ rowElem,
+                                       const int* __restrict__ rowStart, int* __restrict__ entLink,
+                                       R* __restrict__ entAlpha, const int* __restrict__ le1, const R* __restrict__ lcF,
+                                       R* __restrict__ rowPhi, unsigned char* __restrict__ rowSet) {
+  const int row = blockIdx.x * blockDim.x + threadIdx.x;
+  if (row >= nRows) return;
+  const int k0 = rowStart[row], k1 = rowStart[row + 1], e = rowElem[row];
+  for (int k = k0 + 1; k < k1; k++) {
+    const int l = entLink[k];
+    const R al = entAlpha[k];
+    int q = k;
+    for (; q > k0 && entLink[q - 1] > l; q--) {
+      entLink[q] = entLink[q - 1];
+      entAlpha[q] = entAlpha[q - 1];
+    }
+    entLink[q] = l;
+    entAlpha[q] = al;
+  }
+  double phi = 0.0;
+  for (int k = k0; k < k1; k++)
+    if (le1[entLink[k]] == e) phi += (double)lcF[entLink[k]];
+  rowPhi[row] = (R)phi;
+  rowSet[row] = adj_regular(t, e) ? 0 : 1;
+}
+
+// First source of each link, for adj_rows_build3_kernel.
+__global__ void adj_first_source3_kernel(int n, const int* __restrict__ sE1, const int* __restrict__ sTgt,
+                                         int* __restrict__ le1) {
+  const int c = blockIdx.x * blockDim.x + threadIdx.x, i = blockIdx.y;
+  if (c >= n) return;
+  const int r = i * n + c;
+  if (sTgt[r] < 0) le1[-sTgt[r] - 1] = sE1[r] & 0x7fffffff;
 }
 
 // A device buffer of the recorded run: from the handle's table block while it has room (256-byte
@@ -561,298 +1006,129 @@ void release_adjoint(Cells3D* h) {
   // the checkpoints, recompute buffers and adjoint states live in h->adjStore and the tables in
   // h->adjTab, which both stay; only the run's own buffers go
   if (!h->dev.fake) h->dev.sync();
-  if (A->side) cudaStreamSynchronize(A->side);
   if (A->side2) cudaStreamSynchronize(A->side2);
-  for (auto& row : A->segGraph)
-    for (auto& g : row)
-      if (g) cudaGraphExecDestroy(g);
   if (A->fork2) cudaEventDestroy(A->fork2);
   if (A->join2) cudaEventDestroy(A->join2);
   if (A->side2) cudaStreamDestroy(A->side2);
-  if (A->fork) cudaEventDestroy(A->fork);
-  if (A->join) cudaEventDestroy(A->join);
-  if (A->side) cudaStreamDestroy(A->side);
-  if (A->n0Host) h->dev.free_host_pinned(A->n0Host);
   for (void* p : A->own) h->dev.release(p);
   h->adj.reset();
 }
 
-// Link tables and the transposed element map for the current flags and SDF.
-void build_tables(Cells3D* h, Adjoint3D* A) {
+// Block sums of one adjoint step.
+int adj_parts(const Cells3D* h, int nSlow) {
+  const dim3 cells = adj_cell_grid(h->prec, h->W, h->H, h->D);
+  return (int)(cells.x * cells.y * cells.z) + (nSlow + kSlowCells - 1) / kSlowCells +
+         adj_face_blocks(h->prec, h->W, h->H, h->D, cells);
+}
+
+unsigned blocks_of(size_t n, unsigned b) { return (unsigned)((n + b - 1) / b); }
+
+// The list of flagged cells, their pull records, the links and the rows for the current flags and SDF.
+// Two ints come back to the host: the links with the cells' number, then the rows'. The per-element
+// scratch (one count and one row number per population element) lies in the recompute buffers, which
+// the sweep fills later.
+template <class R>
+void build_tables(Cells3D* h, Adjoint3D* A, int* cnt, int* rowOf) {
   cells::Device& dev = h->dev;
-  const long long N = h->N;
-  const int W = h->W, H = h->H, D = h->D;
-  std::vector<uint32_t> fl((size_t)N);
-  std::vector<float> sdf((size_t)N);
-  dev.d2h(fl.data(), h->flags, (size_t)N * 4);
-  dev.d2h(sdf.data(), h->sdf, (size_t)N * 4);
+  cudaStream_t st = dev.stream;
+  const int W = h->W, H = h->H, D = h->D, nRowsXY = H * D;
+  AdjTables3 t;
+  t.flags = h->flags;
+  t.sdf = h->sdf;
+  t.rowBody = h->rowBody;
+  t.N = h->N;
+  t.W = W;
+  t.H = H;
+  t.D = D;
+  t.component = A->component;
+  t.facePairs = adj_face_blocks(h->prec, W, H, D, adj_cell_grid(h->prec, W, H, D)) > 0;
+  // the cell list, and the links of each cell, counted and scanned in scratch
+  int* rowCount = rowOf;                     // H D + 1
+  adj_list3_kernel<<<blocks_of((size_t)nRowsXY * 32, 256), 256, 0, st>>>(t, rowCount, nullptr, nullptr);
+  adj_scan3_kernel<<<1, 1024, 0, st>>>(rowCount, nRowsXY);
+  int host[2] = {0, 0};
+  dev.d2h(host, rowCount + nRowsXY, 4);
   dev.sync();
-  std::vector<int> base;
-  if (h->prec == 3)
-    resolve_links<double>(h, fl, sdf, A->component, base, A->hostLinks);
-  else
-    resolve_links<float>(h, fl, sdf, A->component, base, A->hostLinks);
-  const std::vector<AdjLink3Host>& L = A->hostLinks;
-  A->nLinks = (int)L.size();
-  // transposed map: (element, link, alpha) entries, direct force terms, and elements without a
-  // regular reader
-  struct Ent {
-    long long e;
-    int link;  // -1: no regular reader; -2: a force term
-    double alpha;
-  };
-  // the links' entries, sorted by element (ties keep their order of insertion: link order, then
-  // e1, e2, force within a link)
-  std::vector<Ent> lent;
-  lent.reserve(L.size() * 3);
-  for (int k = 0; k < A->nLinks; k++) {
-    lent.push_back({L[k].e1, k, L[k].a1});
-    if (L[k].e2 >= 0) lent.push_back({L[k].e2, k, L[k].a2});
-    if (L[k].cF != 0.0) lent.push_back({L[k].e1, -2, L[k].cF});
-  }
-  // entry indices in element order, ties in insertion order: a stable LSD radix sort on the
-  // element index (below 19 N < 2^31), 8 bits a pass, as many passes as the largest element needs
-  std::vector<int> key(lent.size()), tmp(lent.size());
-  for (size_t p = 0; p < lent.size(); p++) key[p] = (int)p;
-  {
-    long long maxE = 0;
-    for (const Ent& en : lent) maxE = std::max(maxE, en.e);
-    for (int shift = 0; shift < 32 && (maxE >> shift) != 0; shift += 8) {
-      size_t count[257] = {0};
-      for (int p : key) count[(((uint32_t)lent[(size_t)p].e >> shift) & 255u) + 1]++;
-      for (int d = 0; d < 256; d++) count[d + 1] += count[d];
-      for (int p : key) tmp[count[((uint32_t)lent[(size_t)p].e >> shift) & 255u]++] = p;
-      key.swap(tmp);
-    }
-  }
-  // elements without a regular reader, generated in increasing element order (direction outer)
-  auto at = [&](int x, int y, int z) { return (long long)x + (long long)W * ((long long)y + (long long)H * z); };
-  std::vector<std::vector<long long>> irr(Q3);  // per direction, on host threads
-  {
-    const int T = std::min(table_threads(), Q3);
-    run_threads(T, [&](int t) {
-      for (int i = t; i < Q3; i += T) {
-        std::vector<long long>& out = irr[(size_t)i];
-        for (int z = 0; z < D; z++)
-          for (int y = 0; y < H; y++) {
-            const int ry = y + cy3(i), rz = z + cz3(i);
-            const bool rowIn = ry >= 0 && ry < H && rz >= 0 && rz < D;
-            for (int x = 0; x < W; x++) {
-              const long long c = at(x, y, z);
-              if (fl[(size_t)c] & FLAG3_SOLID) continue;
-              const int rx = x + cx3(i);
-              bool regular = rowIn && rx >= 0 && rx < W;
-              if (regular) {
-                const uint32_t g = fl[(size_t)at(rx, ry, rz)];
-                regular = !(g & (FLAG3_SOLID | FLAG3_INLET)) && (i == 0 || !(g & (1u << i)));
-              }
-              if (!regular) out.push_back(i * N + c);
-            }
-          }
-      }
-    });
-  }
-  std::vector<long long> irregular;
-  for (auto& v : irr) irregular.insert(irregular.end(), v.begin(), v.end());
-  // merge: for one element the link entries come before its no-reader mark
-  std::vector<Ent> ents;
-  ents.reserve(lent.size() + irregular.size());
-  {
-    size_t p = 0, q = 0;
-    while (p < key.size() || q < irregular.size()) {
-      if (q >= irregular.size() || (p < key.size() && lent[(size_t)key[p]].e <= irregular[q]))
-        ents.push_back(lent[(size_t)key[p++]]);
-      else
-        ents.push_back({irregular[q++], -1, 0.0});
-    }
-  }
-  std::vector<long long> rowElem;
-  std::vector<unsigned char> rowSet;
-  std::vector<int> rowStart, entLink;
-  std::vector<double> entAlpha, rowPhi;
-  rowElem.reserve(ents.size());
-  rowSet.reserve(ents.size());
-  rowStart.reserve(ents.size() + 1);
-  rowPhi.reserve(ents.size());
-  entLink.reserve(lent.size());
-  entAlpha.reserve(lent.size());
-  for (size_t p = 0; p < ents.size();) {
-    const long long e = ents[p].e;
-    unsigned char set = 0;
-    double phi = 0.0;
-    rowElem.push_back(e);
-    rowStart.push_back((int)entLink.size());
-    for (; p < ents.size() && ents[p].e == e; p++) {
-      if (ents[p].link == -1) {
-        set = 1;
-      } else if (ents[p].link == -2) {
-        phi += ents[p].alpha;
-      } else {
-        entLink.push_back(ents[p].link);
-        entAlpha.push_back(ents[p].alpha);
-      }
-    }
-    rowSet.push_back(set);
-    rowPhi.push_back(phi);
-  }
-  rowStart.push_back((int)entLink.size());
-  A->nRows = (int)rowElem.size();
-  const size_t rb = h->prec == 3 ? 8 : 4;
-  auto up_r = [&](void* d, const std::vector<double>& v) {
-    if (h->prec == 3)
-      upload_typed<double>(dev, d, v);
-    else
-      upload_typed<float>(dev, d, v);
-  };
-  const size_t nl = std::max<size_t>(1, L.size());
-  std::vector<int> slow;
-  for (long long c = 0; c < N; c++) {
-    const uint32_t v = fl[(size_t)c];
-    if (v != 0u && !(v & FLAG3_SOLID)) slow.push_back((int)c);
-  }
+  A->nSlow = host[0];
+  const size_t ns = (size_t)A->nSlow, nsr = std::max<size_t>(1, 19 * ns);
+  int* cells = cnt;                          // the list, then each cell's first link (n + 1)
+  int* linkBase = cnt + ns;
+  adj_list3_kernel<<<blocks_of((size_t)nRowsXY * 32, 256), 256, 0, st>>>(t, nullptr, rowCount, cells);
+  if (ns) adj_link_count3_kernel<<<blocks_of(ns, 256), 256, 0, st>>>(t, cells, A->nSlow, linkBase);
+  adj_scan3_kernel<<<1, 1024, 0, st>>>(linkBase, A->nSlow);
+  dev.d2h(host, linkBase + ns, 4);
+  dev.sync();
+  A->nLinks = host[0];
+  const size_t nl = std::max<size_t>(1, (size_t)A->nLinks), ne = 2 * nl;  // at most two entries per link
   {
     // every device buffer of the run, as adj_alloc rounds them (these tables, then the forward
     // run's): the handle's table block grows to hold them all before the first is taken
     auto al = [](size_t b) { return (std::max<size_t>(b, 1) + 255) / 256 * 256; };
-    const size_t ns = slow.size(), nsr = std::max<size_t>(1, 19 * ns);
-    const size_t nr = std::max<size_t>(1, rowElem.size()), ne = std::max<size_t>(1, entLink.size());
-    const size_t nSeg = (size_t)((A->steps + A->K - 1) / A->K);
-    const int tileY = kAdjThreads / 32;
-    const size_t nBlocks = (size_t)((W + 31) / 32) * (size_t)((H + tileY - 1) / tileY) * (size_t)D;
-    const size_t nParts = nBlocks + (ns + kSlowCells - 1) / kSlowCells;
-    const size_t need = al((size_t)N * 4) + al(ns * 4) + 3 * al(nsr * 4) + 2 * al(nsr * rb) + 2 * al(nl * 8) +
-                        5 * al(nl * rb) + al(nl) + al(nl * 8) + al(nr * 8) + al(nr) + al((nr + 1) * 4) +
-                        al(nr * rb) + al(ne * 4) + al(ne * rb) + al(nSeg * sizeof(DevState3)) +
-                        al(sizeof(DevState3)) + al(nParts * 8) + 2 * al(64) + 3 * al((size_t)A->steps * 8);
+    const size_t nSeg = (size_t)((A->steps + A->K - 1) / A->K), rb = sizeof(R);
+    const size_t segSteps = (size_t)std::min<int64_t>(A->K, A->steps);
+    const size_t need = al(ns * 4) + al((ns + 1) * 4) + 3 * al(nsr * 4) + 2 * al(nsr * rb) + al(nl * 4) + 3 * al(nl * rb) +
+                        al(nl) + al(nl * sizeof(AdjLinkQ3)) + al(nl * 8) + 2 * al(ne * 4) + al((ne + 1) * 4) + al(ne) +
+                        2 * al(ne * rb) + al(ne * 4) + al(64) + al(nSeg * sizeof(DevState3)) + al(sizeof(DevState3)) +
+                        al((size_t)adj_parts(h, A->nSlow) * segSteps * 8) + al((size_t)A->steps * 8);
     reserve_adj_tables(h, A, need);
   }
-  A->linkBase = (int*)adj_alloc(h, A, (size_t)N * 4, "adjoint link base");
-  dev.h2d(A->linkBase, base.data(), (size_t)N * 4);
-  dev.sync();
-  A->nSlow = (int)slow.size();
-  A->slowCells = (int*)adj_alloc(h, A, std::max<size_t>(1, slow.size()) * 4, "adjoint flagged cells");
-  if (!slow.empty()) {
-    dev.h2d(A->slowCells, slow.data(), slow.size() * 4);
-    dev.sync();
-  }
-  // per flagged cell and direction, [i][cell]: the pull's sources and coefficients, and where its
-  // adjoint goes (an element index, or -(link + 1))
-  const size_t ns = slow.size();
-  std::vector<int> sE1(19 * ns), sE2(19 * ns), sTgt(19 * ns);
-  std::vector<double> sA1(19 * ns), sA2(19 * ns);
-  std::atomic<bool> mismatch(false);
-  // each cell's 19 records are independent: chunks of cells on host threads
-  const int TS = (int)std::min<size_t>((size_t)table_threads(), std::max<size_t>(1, ns / 4096));
-  run_threads(TS, [&](int t) {
-    for (size_t c = ns * t / TS; c < ns * (t + 1) / TS; c++) {
-      const int idx = slow[c];
-      const uint32_t v = fl[(size_t)idx];
-      if (v & FLAG3_INLET) {  // the inlet reads nothing (and has no link records)
-        for (int i = 0; i < Q3; i++) {
-          const size_t r = (size_t)i * ns + c;
-          sE1[r] = sE2[r] = sTgt[r] = 0;
-          sA1[r] = sA2[r] = 0.0;
-        }
-        continue;
-      }
-      const int bse = base[(size_t)idx];
-      int rank = 0;
-      for (int i = 0; i < Q3; i++) {
-        const size_t r = (size_t)i * ns + c;
-        sA2[r] = 0.0;
-        if (i == 0 || !(v & (1u << i))) {
-          const int e = (int)(i * N + idx - off3(i, W, H));
-          sE1[r] = sE2[r] = sTgt[r] = e;
-          sA1[r] = 1.0;
-        } else {
-          const int k = bse + rank++;
-          if (bse < 0 || k >= A->nLinks) {
-            mismatch = true;
-            sE1[r] = sE2[r] = sTgt[r] = 0;
-            sA1[r] = 0.0;
-            continue;
-          }
-          const AdjLink3Host& Lk = A->hostLinks[(size_t)k];
-          const bool single = Lk.e2 < 0 && Lk.a1 == 1.0;
-          // a single source with coefficient 1 is the plain index; otherwise the sign bit marks the
-          // record's two sources and coefficients
-          sE1[r] = single ? (int)Lk.e1 : (int)((uint32_t)Lk.e1 | 0x80000000u);
-          sE2[r] = Lk.e2 >= 0 ? (int)Lk.e2 : (int)Lk.e1;
-          sA1[r] = Lk.a1;
-          sA2[r] = Lk.e2 >= 0 ? Lk.a2 : 0.0;
-          sTgt[r] = -(k + 1);
-        }
-      }
-    }
-  });
-  if (mismatch) throw Error(CELLS_E_INVALID, "adjoint link table does not match the flags");
-  const size_t nsr = std::max<size_t>(1, 19 * ns);
+  A->slowCells = (int*)adj_alloc(h, A, ns * 4, "adjoint flagged cells");
+  int* base = (int*)adj_alloc(h, A, (ns + 1) * 4, "adjoint link base");
   A->sE1 = (int*)adj_alloc(h, A, nsr * 4, "adjoint flagged-cell records");
   A->sE2 = (int*)adj_alloc(h, A, nsr * 4, "adjoint flagged-cell records");
   A->sTgt = (int*)adj_alloc(h, A, nsr * 4, "adjoint flagged-cell records");
-  A->sA1 = adj_alloc(h, A, nsr * (h->prec == 3 ? 8 : 4), "adjoint flagged-cell records");
-  A->sA2 = adj_alloc(h, A, nsr * (h->prec == 3 ? 8 : 4), "adjoint flagged-cell records");
+  A->sA1 = adj_alloc(h, A, nsr * sizeof(R), "adjoint flagged-cell records");
+  A->sA2 = adj_alloc(h, A, nsr * sizeof(R), "adjoint flagged-cell records");
+  int* le1 = (int*)adj_alloc(h, A, nl * 4, "adjoint links");
+  A->lcF = adj_alloc(h, A, nl * sizeof(R), "adjoint links");
+  A->lq = adj_alloc(h, A, nl * sizeof(R), "adjoint links");
+  A->lqk = (signed char*)adj_alloc(h, A, nl, "adjoint links");
+  A->linkQ = (AdjLinkQ3*)adj_alloc(h, A, nl * sizeof(AdjLinkQ3), "adjoint links");
+  A->lamG = adj_alloc(h, A, nl * sizeof(R), "adjoint link values");
+  A->dqAcc = (double*)adj_alloc(h, A, nl * 8, "adjoint dJ/dq");
+  A->rowElem = (int*)adj_alloc(h, A, ne * 4, "adjoint rows");
+  int* fill = (int*)adj_alloc(h, A, ne * 4, "adjoint rows");
+  A->rowStart = (int*)adj_alloc(h, A, (ne + 1) * 4, "adjoint rows");
+  A->rowSet = (unsigned char*)adj_alloc(h, A, ne, "adjoint rows");
+  A->rowPhi = adj_alloc(h, A, ne * sizeof(R), "adjoint rows");
+  A->entAlpha = adj_alloc(h, A, ne * sizeof(R), "adjoint rows");
+  A->entLink = (int*)adj_alloc(h, A, ne * 4, "adjoint rows");
+  int* nRows = (int*)adj_alloc(h, A, 64, "adjoint rows");
+  A->nRows = 0;
   if (ns) {
-    dev.h2d(A->sE1, sE1.data(), sE1.size() * 4);
-    dev.h2d(A->sE2, sE2.data(), sE2.size() * 4);
-    dev.h2d(A->sTgt, sTgt.data(), sTgt.size() * 4);
+    check_cuda(cudaMemcpyAsync(A->slowCells, cells, ns * 4, cudaMemcpyDeviceToDevice, st), "adjoint cell list");
+    check_cuda(cudaMemcpyAsync(base, linkBase, (ns + 1) * 4, cudaMemcpyDeviceToDevice, st), "adjoint link base");
+    dev.memset0(cnt, 19 * (size_t)h->N * 4);
+    dev.memset0(rowOf, 19 * (size_t)h->N * 4);
+    dev.memset0(nRows, 4);
+    dev.memset0(fill, ne * 4);
+    AdjLaunch3 a;
+    std::memset(&a, 0, sizeof(a));
+    a.nSlow = A->nSlow;
+    a.slowCells = A->slowCells;
+    for (int i = 0; i < Q3; i++) a.off[i] = (int)off3(i, W, H);
+    const dim3 items(blocks_of(ns, 256), Q3);
+    adj_links3_kernel<R><<<blocks_of(ns, 128), 128, 0, st>>>(t, a, base, A->linkQ, A->sE1, A->sE2, A->sTgt, (R*)A->sA1,
+                                                             (R*)A->sA2, (R*)A->lcF, (R*)A->lq, A->lqk, cnt);
+    adj_first_source3_kernel<<<items, 256, 0, st>>>(A->nSlow, A->sE1, A->sTgt, le1);
+    adj_claim3_kernel<R><<<items, 256, 0, st>>>(t, A->nSlow, A->sE1, A->sE2, A->sTgt, (const R*)A->lcF, cnt, rowOf,
+                                                A->rowElem, A->rowStart, nRows);
+    check_cuda(cudaGetLastError(), "adjoint table kernels");
+    dev.d2h(host, nRows, 4);
     dev.sync();
-    if (h->prec == 3) {
-      upload_typed<double>(dev, A->sA1, sA1);
-      upload_typed<double>(dev, A->sA2, sA2);
-    } else {
-      upload_typed<float>(dev, A->sA1, sA1);
-      upload_typed<float>(dev, A->sA2, sA2);
+    A->nRows = host[0];
+    if (A->nRows > 0) {
+      adj_scan3_kernel<<<1, 1024, 0, st>>>(A->rowStart, A->nRows);
+      adj_entries3_kernel<R><<<items, 256, 0, st>>>(A->nSlow, A->sE1, A->sE2, A->sTgt, (const R*)A->sA1,
+                                                    (const R*)A->sA2, rowOf, A->rowStart, fill, A->entLink,
+                                                    (R*)A->entAlpha);
+      adj_rows_build3_kernel<R><<<blocks_of((size_t)A->nRows, 256), 256, 0, st>>>(
+          t, A->nRows, A->rowElem, A->rowStart, A->entLink, (R*)A->entAlpha, le1, (const R*)A->lcF, (R*)A->rowPhi,
+          A->rowSet);
     }
   }
-  std::vector<long long> e1(L.size()), e2(L.size());
-  std::vector<double> a1(L.size()), a2(L.size()), cF(L.size()), q(L.size());
-  std::vector<signed char> qk(L.size());
-  for (size_t k = 0; k < L.size(); k++) {
-    e1[k] = L[k].e1;
-    e2[k] = L[k].e2;
-    a1[k] = L[k].a1;
-    a2[k] = L[k].a2;
-    cF[k] = L[k].cF;
-    q[k] = L[k].q;
-    qk[k] = (signed char)L[k].qKind;
-  }
-  A->le1 = (long long*)adj_alloc(h, A, nl * 8, "adjoint links");
-  A->le2 = (long long*)adj_alloc(h, A, nl * 8, "adjoint links");
-  A->la1 = adj_alloc(h, A, nl * rb, "adjoint links");
-  A->la2 = adj_alloc(h, A, nl * rb, "adjoint links");
-  A->lcF = adj_alloc(h, A, nl * rb, "adjoint links");
-  A->lq = adj_alloc(h, A, nl * rb, "adjoint links");
-  A->lqk = (signed char*)adj_alloc(h, A, nl, "adjoint links");
-  A->lamG = adj_alloc(h, A, nl * rb, "adjoint link values");
-  A->dqAcc = (double*)adj_alloc(h, A, nl * 8, "adjoint dJ/dq");
-  if (!L.empty()) {
-    dev.h2d(A->le1, e1.data(), L.size() * 8);
-    dev.h2d(A->le2, e2.data(), L.size() * 8);
-    dev.h2d(A->lqk, qk.data(), L.size());
-    dev.sync();
-    up_r(A->la1, a1);
-    up_r(A->la2, a2);
-    up_r(A->lcF, cF);
-    up_r(A->lq, q);
-  }
-  const size_t nr = std::max<size_t>(1, rowElem.size());
-  const size_t ne = std::max<size_t>(1, entLink.size());
-  A->rowElem = (long long*)adj_alloc(h, A, nr * 8, "adjoint rows");
-  A->rowSet = (unsigned char*)adj_alloc(h, A, nr, "adjoint rows");
-  A->rowStart = (int*)adj_alloc(h, A, (nr + 1) * 4, "adjoint rows");
-  A->rowPhi = adj_alloc(h, A, nr * rb, "adjoint rows");
-  A->entLink = (int*)adj_alloc(h, A, ne * 4, "adjoint rows");
-  A->entAlpha = adj_alloc(h, A, ne * rb, "adjoint rows");
-  if (!rowElem.empty()) {
-    dev.h2d(A->rowElem, rowElem.data(), rowElem.size() * 8);
-    dev.h2d(A->rowSet, rowSet.data(), rowSet.size());
-    dev.h2d(A->rowStart, rowStart.data(), rowStart.size() * 4);
-    if (!entLink.empty()) dev.h2d(A->entLink, entLink.data(), entLink.size() * 4);
-    dev.sync();
-    up_r(A->rowPhi, rowPhi);
-    if (!entAlpha.empty()) up_r(A->entAlpha, entAlpha);
-  }
+  check_cuda(cudaGetLastError(), "adjoint table kernels");
+  dev.launches += 10;
 }
 
 }  // namespace
@@ -860,31 +1136,23 @@ void build_tables(Cells3D* h, Adjoint3D* A) {
 namespace {
 
 // The launch arguments of the adjoint step kernels for the recorded run (all but f, the adjoint
-// buffers and the step position t, which enqueue_segment sets per step).
+// buffers, the block sums and the step's inlet speed and objective weight, which enqueue_sweep sets).
 AdjLaunch3 adj_args(Cells3D* h, Adjoint3D* A) {
   AdjLaunch3 a;
   std::memset(&a, 0, sizeof(a));
   a.flags = h->flags;
   a.xTab = h->xTab;
-  a.linkBase = A->linkBase;
-  a.le1 = A->le1;
-  a.le2 = A->le2;
-  a.la1 = A->la1;
-  a.la2 = A->la2;
+  a.rowBody = h->rowBody;
   a.lcF = A->lcF;
   a.lq = A->lq;
   a.lqk = A->lqk;
   a.lamG = A->lamG;
   a.dqAcc = A->dqAcc;
-  a.blockPart = A->blockPart;
-  a.counter = A->counter;
   a.N = h->N;
   a.W = h->W;
   a.H = h->H;
   a.D = h->D;
-  a.tileX = A->tileX;
   a.absorbX0 = h->absorbX0;
-  a.nCellBlocks = A->nBlocks;
   a.slowCells = A->slowCells;
   a.nSlow = A->nSlow;
   a.sE1 = A->sE1;
@@ -900,10 +1168,6 @@ AdjLaunch3 adj_args(Cells3D* h, Adjoint3D* A) {
   a.entLink = A->entLink;
   a.entAlpha = A->entAlpha;
   a.rowPhi = A->rowPhi;
-  a.n0Dev = A->n0Dev;
-  a.uDev = A->uDev;
-  a.wDev = A->wDev;
-  a.dudn = A->dudn;
   return a;
 }
 
@@ -915,74 +1179,55 @@ void enqueue_recompute(Cells3D* h, Adjoint3D* A, int set, int len, int par0, cud
   }
 }
 
-// The adjoint steps of a segment whose states are in set `set`, from the last to the first,
-// starting from adjoint buffer c; with `next`, the next (earlier) segment's recompute into the
-// other set runs beside them on side2.
-void enqueue_sweep(Cells3D* h, Adjoint3D* A, AdjLaunch3& a, int set, int len, int c, bool next, int nextLen,
-                   int nextPar0) {
+// The adjoint steps of segment sgi (len steps, states in set `set`), from the last to the first,
+// starting from adjoint buffer c; the next (earlier) segment's recompute into the other set, when there
+// is one, runs beside them on side2.
+void enqueue_sweep(Cells3D* h, Adjoint3D* A, AdjLaunch3& a, int64_t sgi, int set, int len, int c, bool next,
+                   int nextLen, int nextPar0, bool terminal) {
   cudaStream_t s = h->dev.stream;
   if (next) {
     check_cuda(cudaEventRecord(A->fork2, s), "cudaEventRecord");
     check_cuda(cudaStreamWaitEvent(A->side2, A->fork2, 0), "cudaStreamWaitEvent");
-    enqueue_recompute(h, A, set ^ 1, nextLen, nextPar0, A->side2);
-    check_cuda(cudaEventRecord(A->join2, A->side2), "cudaEventRecord");
   }
   for (int t = len - 1; t >= 0; t--) {
+    const int64_t n = sgi * A->K + t, label = A->s0 + n + 1;
     a.f = A->seg[set][(size_t)t];
     a.lamNext = A->lam[c];
     a.lamOut = A->lam[c ^ 1];
-    a.t = t;
-    check_cuda(launch_adjoint_step3(h->prec, a, s, A->side, A->fork, A->join), "adjoint step kernel");
-    h->dev.launches += 3;
+    a.blockPart = A->blockPart + (size_t)t * A->nParts;
+    a.u = A->uStep[(size_t)n];
+    a.w = label >= A->w0 && label <= A->w1 ? A->scale / (double)(A->w1 - A->w0 + 1) : 0.0;
+    check_cuda(launch_adjoint_step3(h->prec, a, s), "adjoint step kernel");
+    h->dev.launches += 2;
+    // elements that nothing reads keep zero, which a terminal adjoint in the first buffer is not
+    if (terminal && n + 1 == A->steps) h->dev.memset0(A->lam[c], 19 * h->bpp * (size_t)h->N);
     c ^= 1;
+    // the recompute's steps go out between the adjoint steps, so neither stream waits for the host
+    const int k = len - 1 - t;
+    if (next && k + 1 < nextLen) {
+      h->enqueue_step_between(A->seg[set ^ 1][(size_t)k], A->seg[set ^ 1][(size_t)k + 1], nextPar0 ^ (k & 1), false,
+                              A->side2);
+      h->dev.launches++;
+    }
   }
+  if (next) {
+    for (int k = len; k + 1 < nextLen; k++) {
+      h->enqueue_step_between(A->seg[set ^ 1][(size_t)k], A->seg[set ^ 1][(size_t)k + 1], nextPar0 ^ (k & 1), false,
+                              A->side2);
+      h->dev.launches++;
+    }
+    check_cuda(cudaEventRecord(A->join2, A->side2), "cudaEventRecord");
+  }
+  adj_du3_kernel<<<len, 256, 0, s>>>(A->blockPart, A->nParts, A->dudn + sgi * A->K);
+  check_cuda(cudaGetLastError(), "adjoint du kernel");
+  h->dev.launches++;
   if (next) check_cuda(cudaStreamWaitEvent(s, A->join2, 0), "cudaStreamWaitEvent");
-}
-
-// Full segments replay graphs when K is even (the parity pattern and buffers repeat).
-bool segment_graphs(const Cells3D* h, const Adjoint3D* A) { return h->useGraphs && A->K % 2 == 0; }
-
-void build_segment_graph(Cells3D* h, Adjoint3D* A, int set, int next, int cur) {
-  cudaGraphExec_t& g = A->segGraph[set][next];
-  if (g) cudaGraphExecDestroy(g);
-  g = nullptr;
-  AdjLaunch3 a = adj_args(h, A);
-  const int par0 = A->parity0 & 1;  // the parity at every full segment's start (K even)
-  const int64_t before = h->dev.launches;
-  check_cuda(cudaStreamBeginCapture(h->dev.stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-  enqueue_sweep(h, A, a, set, A->K, cur, next != 0, A->K, par0);
-  cudaGraph_t graph = nullptr;
-  check_cuda(cudaStreamEndCapture(h->dev.stream, &graph), "cudaStreamEndCapture");
-  cudaError_t e = cudaGraphInstantiate(&g, graph, 0);
-  cudaGraphDestroy(graph);
-  check_cuda(e, "cudaGraphInstantiate");
-  A->segGraphLaunches[set][next] = h->dev.launches - before;
-  h->dev.launches = before;
 }
 
 // The state set of segment s: the sweep alternates sets, starting with set 0 at the last segment.
 int seg_set(const Adjoint3D* A, int64_t s) {
   const int64_t nSeg = (A->steps + A->K - 1) / A->K;
   return (int)((nSeg - 1 - s) & 1);
-}
-
-// The sweep reaches its full segments with adjoint buffer 0, or 1 after an odd-length last segment.
-int full_segment_cur(const Adjoint3D* A) {
-  const int64_t nSeg = (A->steps + A->K - 1) / A->K;
-  const int64_t lenLast = A->steps - (nSeg - 1) * A->K;
-  return (lenLast < A->K && (lenLast & 1)) ? 1 : 0;
-}
-
-void build_segment_graphs(Cells3D* h, Adjoint3D* A) {
-  const int64_t nSeg = (A->steps + A->K - 1) / A->K;
-  const int cur = full_segment_cur(A);
-  for (int64_t s = nSeg - 1; s >= 0; s--) {
-    const int64_t len = std::min<int64_t>(A->K, A->steps - s * A->K);
-    if (len != A->K) continue;
-    const int set = seg_set(A, s), next = s > 0 ? 1 : 0;
-    if (!A->segGraph[set][next]) build_segment_graph(h, A, set, next, cur);
-  }
-  A->segGraphCur = cur;
 }
 
 }  // namespace
@@ -1024,32 +1269,21 @@ int cells3d_adjoint_forward(Cells3D* h, const Cells3DAdjointSpec* spec, double* 
   const int64_t nWin = spec->window_end - spec->window_begin + 1;
   if (nWin > HISTORY_LEN) throw Error(CELLS_E_INVALID, "the objective window exceeds the 8192-sample force ring");
   if (19ll * h->N >= (1ll << 31)) throw Error(CELLS_E_INVALID, "the adjoint supports grids of fewer than 2^31 / 19 cells");
-  // the previous run's streams, events and pinned segment slots carry over (detached here, after
-  // their work has finished, so release_adjoint keeps them)
+  // the previous run's stream and events carry over (detached here, after their work has finished,
+  // so release_adjoint keeps them)
   Adjoint3D carry;
   if (Adjoint3D* old = h->adj.get()) {
-    if (old->side) cudaStreamSynchronize(old->side);
     if (old->side2) cudaStreamSynchronize(old->side2);
-    std::swap(carry.side, old->side);
     std::swap(carry.side2, old->side2);
-    std::swap(carry.fork, old->fork);
-    std::swap(carry.join, old->join);
     std::swap(carry.fork2, old->fork2);
     std::swap(carry.join2, old->join2);
-    std::swap(carry.n0Host, old->n0Host);
-    std::swap(carry.n0Cap, old->n0Cap);
   }
   release_adjoint(h);
   h->adj.reset(new Adjoint3D());
   Adjoint3D* A = h->adj.get();
-  std::swap(A->side, carry.side);
   std::swap(A->side2, carry.side2);
-  std::swap(A->fork, carry.fork);
-  std::swap(A->join, carry.join);
   std::swap(A->fork2, carry.fork2);
   std::swap(A->join2, carry.join2);
-  std::swap(A->n0Host, carry.n0Host);
-  std::swap(A->n0Cap, carry.n0Cap);
   A->s0 = s0;
   A->steps = spec->steps;
   A->w0 = spec->window_begin;
@@ -1078,43 +1312,29 @@ int cells3d_adjoint_forward(Cells3D* h, const Cells3DAdjointSpec* spec, double* 
     h->adjStore = dev.alloc(need, "adjoint checkpoints");
     h->adjStoreBytes = need;
   }
-  build_tables(h, A);
   char* store = (char*)h->adjStore;
-  A->ckStateBlock = (DevState3*)adj_alloc(h, A, (size_t)nSeg * sizeof(DevState3), "adjoint checkpoint");
-  for (int64_t k = 0; k < nSeg; k++) {
-    A->ck.push_back(store + (size_t)k * stride);
-    A->ckState.push_back(A->ckStateBlock + k);
-  }
+  for (int64_t k = 0; k < nSeg; k++) A->ck.push_back(store + (size_t)k * stride);
   for (int set = 0; set < 2; set++)
     for (int k = 0; k < segBufs; k++) A->seg[set].push_back(store + (size_t)(nSeg + set * segBufs + k) * stride);
+  // the per-element scratch: the last checkpoint-sized places of the store (an f32 element is as wide as a
+  // count)
+  if (h->prec == CELLS_FP64)
+    build_tables<double>(h, A, (int*)(store + (size_t)(nSeg + 2 * segBufs) * stride),
+                         (int*)(store + (size_t)(nSeg + 2 * segBufs + 1) * stride));
+  else
+    build_tables<float>(h, A, (int*)(store + (size_t)(nSeg + 2 * segBufs) * stride),
+                        (int*)(store + (size_t)(nSeg + 2 * segBufs + 1) * stride));
+  A->ckStateBlock = (DevState3*)adj_alloc(h, A, (size_t)nSeg * sizeof(DevState3), "adjoint checkpoint");
+  for (int64_t k = 0; k < nSeg; k++) A->ckState.push_back(A->ckStateBlock + k);
   A->endState = adj_alloc(h, A, sizeof(DevState3), "adjoint end state");
   A->lam[0] = store + (size_t)(nSeg + 2 * segBufs) * stride;
   A->lam[1] = store + (size_t)(nSeg + 2 * segBufs + 1) * stride;
-  // 32-cell x tiles: each warp still reads 128-byte rows, and the tiles before the absorbing layer
-  // take the collision code without it
-  A->tileX = 32;
-  const int tileY = kAdjThreads / A->tileX;
-  A->nBlocks = ((h->W + A->tileX - 1) / A->tileX) * ((h->H + tileY - 1) / tileY) * h->D;
-  A->nParts = A->nBlocks + (A->nSlow + kSlowCells - 1) / kSlowCells;
-  A->blockPart = (double*)adj_alloc(h, A, (size_t)A->nParts * 8, "adjoint partials");
-  A->counter = (unsigned*)adj_alloc(h, A, 64, "adjoint counter");
+  A->nParts = adj_parts(h, A->nSlow);
+  A->blockPart = (double*)adj_alloc(h, A, (size_t)A->nParts * segBufs * 8, "adjoint partials");
   A->dudn = (double*)adj_alloc(h, A, (size_t)A->steps * 8, "adjoint du");
-  A->uDev = (double*)adj_alloc(h, A, (size_t)A->steps * 8, "adjoint step speeds");
-  A->wDev = (double*)adj_alloc(h, A, (size_t)A->steps * 8, "adjoint step weights");
-  A->n0Dev = (int*)adj_alloc(h, A, 64, "adjoint segment index");
-  if (A->n0Cap < (size_t)nSeg) {
-    if (A->n0Host) dev.free_host_pinned(A->n0Host);
-    A->n0Host = nullptr;
-    A->n0Cap = 0;
-    A->n0Host = (int*)dev.host_pinned((size_t)nSeg * sizeof(int));
-    A->n0Cap = (size_t)nSeg;
-  }
-  if (!A->side) check_cuda(cudaStreamCreateWithFlags(&A->side, cudaStreamNonBlocking), "cudaStreamCreate");
   if (!A->side2) check_cuda(cudaStreamCreateWithFlags(&A->side2, cudaStreamNonBlocking), "cudaStreamCreate");
   if (!A->fork2) check_cuda(cudaEventCreateWithFlags(&A->fork2, cudaEventDisableTiming), "cudaEventCreate");
   if (!A->join2) check_cuda(cudaEventCreateWithFlags(&A->join2, cudaEventDisableTiming), "cudaEventCreate");
-  if (!A->fork) check_cuda(cudaEventCreateWithFlags(&A->fork, cudaEventDisableTiming), "cudaEventCreate");
-  if (!A->join) check_cuda(cudaEventCreateWithFlags(&A->join, cudaEventDisableTiming), "cudaEventCreate");
   // the recorded run: a checkpoint at the start of every segment, force samples in the window
   const uint64_t written0 = h->forceSamplesRead + h->forceSteps.size();
   A->uStep.resize((size_t)A->steps);
@@ -1124,68 +1344,25 @@ int cells3d_adjoint_forward(Cells3D* h, const Cells3DAdjointSpec* spec, double* 
     A->uStep[(size_t)n] = h->uin_at(s);
     A->rampStep[(size_t)n] = h->rampKind ? (h->rampTarget != 0.0 ? h->ramp_speed(s) / h->rampTarget : 0.0) : 1.0;
   }
-  // Segments of K steps (K even) that are all sampled or all unsampled replay a graph of K steps
-  // captured once per recorded run: with K even every segment starts at the parity of the first.
-  cudaGraphExec_t recGraph[2] = {nullptr, nullptr};  // [sampled]
-  int64_t recGraphLaunches[2] = {0, 0};
-  const bool recGraphs = h->useGraphs && A->K % 2 == 0;
-  auto record_graph = [&](int sampled) {
-    const int64_t before = dev.launches;
-    const int p0 = h->parity;
-    check_cuda(cudaStreamBeginCapture(dev.stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
-    for (int t = 0; t < A->K; t++) {
-      const int p = p0 ^ (t & 1);
-      h->enqueue_step_between(h->f[p], h->f[p ^ 1], p, sampled != 0);
-      dev.launches++;
+  // (launched step by step: a step takes the GPU several times as long as its launch takes the host,
+  // and capturing K-step graphs anew for every recorded run cost more than they saved)
+  for (int64_t n = 0; n < A->steps; n++) {
+    if (n % A->K == 0) {
+      const int64_t k = n / A->K;
+      check_cuda(cudaMemcpyAsync(A->ck[(size_t)k], h->f[h->parity], fBytes, cudaMemcpyDeviceToDevice, dev.stream),
+                 "checkpoint copy");
+      check_cuda(cudaMemcpyAsync(A->ckState[(size_t)k], h->st, sizeof(DevState3), cudaMemcpyDeviceToDevice,
+                                 dev.stream),
+                 "checkpoint copy");
     }
-    cudaGraph_t graph = nullptr;
-    check_cuda(cudaStreamEndCapture(dev.stream, &graph), "cudaStreamEndCapture");
-    const cudaError_t e = cudaGraphInstantiate(&recGraph[sampled], graph, 0);
-    cudaGraphDestroy(graph);
-    check_cuda(e, "cudaGraphInstantiate");
-    recGraphLaunches[sampled] = dev.launches - before;
-    dev.launches = before;
-  };
-  try {
-    for (int64_t n = 0; n < A->steps;) {
-      if (n % A->K == 0) {
-        const int64_t k = n / A->K;
-        check_cuda(cudaMemcpyAsync(A->ck[(size_t)k], h->f[h->parity], fBytes, cudaMemcpyDeviceToDevice, dev.stream),
-                   "checkpoint copy");
-        check_cuda(cudaMemcpyAsync(A->ckState[(size_t)k], h->st, sizeof(DevState3), cudaMemcpyDeviceToDevice,
-                                   dev.stream),
-                   "checkpoint copy");
-        const int64_t first = s0 + n + 1, last = s0 + n + A->K;  // the segment's step labels
-        const bool all = first >= A->w0 && last <= A->w1, none = last < A->w0 || first > A->w1;
-        if (recGraphs && n + A->K <= A->steps && (all || none)) {
-          const int sampled = all ? 1 : 0;
-          if (!recGraph[sampled]) record_graph(sampled);
-          check_cuda(cudaGraphLaunch(recGraph[sampled], dev.stream), "cudaGraphLaunch");
-          dev.launches += recGraphLaunches[sampled];
-          for (int t = 0; t < A->K; t++) {
-            h->step++;
-            if (all) h->forceSteps.push_back((uint32_t)h->step);
-          }
-          n += A->K;
-          continue;
-        }
-      }
-      const int64_t label = s0 + n + 1;
-      const bool sample = label >= A->w0 && label <= A->w1;
-      h->enqueue_step_between(h->f[h->parity], h->f[h->parity ^ 1], h->parity, sample);
-      dev.launches++;
-      h->parity ^= 1;
-      h->step++;
-      if (sample) h->forceSteps.push_back((uint32_t)h->step);
-      n++;
-    }
-  } catch (...) {
-    for (cudaGraphExec_t g : recGraph)
-      if (g) cudaGraphExecDestroy(g);
-    throw;
+    const int64_t label = s0 + n + 1;
+    const bool sample = label >= A->w0 && label <= A->w1;
+    h->enqueue_step_between(h->f[h->parity], h->f[h->parity ^ 1], h->parity, sample);
+    dev.launches++;
+    h->parity ^= 1;
+    h->step++;
+    if (sample) h->forceSteps.push_back((uint32_t)h->step);
   }
-  for (cudaGraphExec_t g : recGraph)
-    if (g) cudaGraphExecDestroy(g);
   check_cuda(cudaMemcpyAsync(A->endState, h->st, sizeof(DevState3), cudaMemcpyDeviceToDevice, dev.stream),
              "end state copy");
   // the objective from the window's samples (ring slots written0 .. written0 + nWin - 1)
@@ -1202,18 +1379,8 @@ int cells3d_adjoint_forward(Cells3D* h, const Cells3DAdjointSpec* spec, double* 
   double sum = 0.0;
   for (const double4& v : hist) sum += A->component == 0 ? v.x : (A->component == 1 ? v.y : v.z);
   A->objective = A->scale * sum / (double)nWin;
-  std::vector<double> wStep((size_t)A->steps, 0.0);
-  for (int64_t n = 0; n < A->steps; n++) {
-    const int64_t label = s0 + n + 1;
-    if (label >= A->w0 && label <= A->w1) wStep[(size_t)n] = A->scale / (double)nWin;
-  }
-  dev.h2d(A->uDev, A->uStep.data(), (size_t)A->steps * 8);
-  dev.h2d(A->wDev, wStep.data(), (size_t)A->steps * 8);
-  dev.sync();
   A->endStep = h->step;
   A->argGen = h->argGen;
-  // the backward sweep's segment graphs, built now (record time) rather than inside the sweep
-  if (segment_graphs(h, A)) build_segment_graphs(h, A);
   if (objective) *objective = A->objective;
   ADJ_CATCH(h)
 }
@@ -1233,7 +1400,6 @@ int cells3d_adjoint_backward(Cells3D* h, const void* terminal_adjoint, double* d
   dev.memset0(A->lam[1], fBytes);
   dev.memset0(A->dqAcc, (size_t)std::max(1, A->nLinks) * 8);
   dev.memset0(A->dudn, (size_t)A->steps * 8);
-  dev.memset0(A->counter, 4);
   int cur = 0;
   if (terminal_adjoint) {
     dev.h2d(A->lam[0], terminal_adjoint, fBytes);
@@ -1241,8 +1407,6 @@ int cells3d_adjoint_backward(Cells3D* h, const void* terminal_adjoint, double* d
   }
   const int64_t nSeg = (A->steps + A->K - 1) / A->K;
   AdjLaunch3 a = adj_args(h, A);
-  const bool graphs = segment_graphs(h, A);
-  if (graphs && A->segGraphCur != full_segment_cur(A)) build_segment_graphs(h, A);
   // restore a segment's device state and first state (its checkpoint) into its state set
   auto restore = [&](int64_t s) {
     check_cuda(cudaMemcpyAsync(h->st, A->ckState[(size_t)s], sizeof(DevState3), cudaMemcpyDeviceToDevice,
@@ -1262,30 +1426,25 @@ int cells3d_adjoint_backward(Cells3D* h, const void* terminal_adjoint, double* d
     const int len = seg_len(sgi);
     const int set = seg_set(A, sgi);
     const bool next = sgi > 0;
-    A->n0Host[sgi] = (int)(sgi * A->K);
-    check_cuda(cudaMemcpyAsync(A->n0Dev, A->n0Host + sgi, sizeof(int), cudaMemcpyHostToDevice, dev.stream),
-               "segment index copy");
     if (next) restore(sgi - 1);
-    if (graphs && len == A->K && cur == A->segGraphCur) {
-      check_cuda(cudaGraphLaunch(A->segGraph[set][next ? 1 : 0], dev.stream), "cudaGraphLaunch");
-      dev.launches += A->segGraphLaunches[set][next ? 1 : 0];
-    } else {
-      enqueue_sweep(h, A, a, set, len, cur, next, next ? seg_len(sgi - 1) : 0, next ? seg_par0(sgi - 1) : 0);
-    }
+    enqueue_sweep(h, A, a, sgi, set, len, cur, next, next ? seg_len(sgi - 1) : 0, next ? seg_par0(sgi - 1) : 0,
+                  terminal_adjoint != nullptr);
     if (len & 1) cur ^= 1;
   }
   check_cuda(cudaMemcpyAsync(h->st, A->endState, sizeof(DevState3), cudaMemcpyDeviceToDevice, dev.stream),
              "end state restore");
   if (adjoint_out) dev.d2h(adjoint_out, A->lam[cur], fBytes);
   std::vector<double> dq((size_t)std::max(1, A->nLinks)), dudn((size_t)A->steps);
+  std::vector<AdjLinkQ3> linkQ((size_t)(dJ_dsdf ? A->nLinks : 0));
   dev.d2h(dq.data(), A->dqAcc, dq.size() * 8);
   dev.d2h(dudn.data(), A->dudn, dudn.size() * 8);
+  if (!linkQ.empty()) dev.d2h(linkQ.data(), A->linkQ, linkQ.size() * sizeof(AdjLinkQ3));
   dev.sync();
   if (dJ_dsdf) {
     std::fill(dJ_dsdf, dJ_dsdf + N, 0.0);
     for (int k = 0; k < A->nLinks; k++) {
-      const AdjLink3Host& L = A->hostLinks[(size_t)k];
-      if (L.qKind == 0 || L.solid < 0) continue;
+      const AdjLinkQ3& L = linkQ[(size_t)k];
+      if (L.solid < 0) continue;
       dJ_dsdf[L.cell] += dq[(size_t)k] * L.dqdF;
       dJ_dsdf[L.solid] += dq[(size_t)k] * L.dqdS;
     }

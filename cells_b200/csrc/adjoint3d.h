@@ -16,16 +16,11 @@
 
 #include "kernels3d.h"
 
-// A resolved pull of a flagged fluid cell's direction: g = a1 f[e1] + a2 f[e2] (e2 < 0: one source).
-// Force links add cF (fj + g) to the objective's force component, fj = f[ej] with ej = e1.
-struct AdjLink3Host {
-  long long e1, e2;
-  double a1, a2;
-  double cF;      // c_{j, component} for force links (Bouzidi, slip face meeting a solid), else 0
-  int qKind;      // 0: g does not depend on q; 1: q < 1/2 with a fluid node behind; 2: q >= 1/2
-  double q;       // link fraction in the arithmetic type, for dg/dq
-  double dqdF, dqdS;  // dq/dsdf at the cell and at the solid node (0 where q is clamped)
-  int cell, solid;    // node indices of the SDF values q reads
+// How a link's fraction q depends on the SDF: dq/dsdf at the cell and at the solid node (0 where q is
+// clamped). solid < 0: the link's pull does not depend on q.
+struct AdjLinkQ3 {
+  double dqdF, dqdS;
+  int cell, solid;
 };
 
 struct Adjoint3D {
@@ -50,23 +45,19 @@ struct Adjoint3D {
   void* endState = nullptr;  // device state after the run (restored after the backward sweep)
   std::vector<void*> seg[2];  // two sets of K recomputed states: the segment being swept and the next
 
-  // link tables (device)
+  // link tables (device). A link is a flagged direction of a listed cell: g = a1 f[e1] + a2 f[e2].
+  // Force links add cF (f[e1] + g) to the objective's force component, cF = c_{j, component}.
   int nLinks = 0;
-  std::vector<AdjLink3Host> hostLinks;
-  int* linkBase = nullptr;      // N: first link of a flagged fluid cell, -1 otherwise
-  long long* le1 = nullptr;
-  long long* le2 = nullptr;
-  void* la1 = nullptr;          // R
-  void* la2 = nullptr;          // R
-  void* lcF = nullptr;          // R
+  AdjLinkQ3* linkQ = nullptr;
+  void* lcF = nullptr;          // R, 0 for a link without force
   void* lq = nullptr;           // R
-  signed char* lqk = nullptr;
+  signed char* lqk = nullptr;   // 0: g does not depend on q; 1: q < 1/2 with a fluid node behind; 2: q >= 1/2
   void* lamG = nullptr;         // R, the adjoint of each link's pulled value in the current step
   double* dqAcc = nullptr;      // dJ/dq per link, summed over the steps
 
-  // transposed map: elements with irregular readers or no regular reader
+  // transposed map: elements that a link reads beside other readers, with a coefficient or for a force
   int nRows = 0;
-  long long* rowElem = nullptr;
+  int* rowElem = nullptr;
   unsigned char* rowSet = nullptr;  // 1: the element has no regular reader (its adjoint is set, not added)
   int* rowStart = nullptr;          // nRows + 1
   int* entLink = nullptr;
@@ -75,36 +66,22 @@ struct Adjoint3D {
 
   // adjoint state
   void* lam[2] = {nullptr, nullptr};  // R, 19 N each
-  double* blockPart = nullptr;
-  unsigned* counter = nullptr;
+  double* blockPart = nullptr;       // dJ/du_n block sums of a segment's steps: K x nParts
   double* dudn = nullptr;            // dJ/du_n per recorded step
-  int nBlocks = 0;  // blocks of the cell kernel
-  int tileX = 128;
-  double* uDev = nullptr;    // inlet speed of each recorded step (device)
-  double* wDev = nullptr;    // objective weight of each recorded step (device)
-  int* n0Dev = nullptr;      // first step of the segment being swept (device)
-  int* n0Host = nullptr;     // pinned, one slot per segment (the source of each n0Dev copy)
-  size_t n0Cap = 0;          // slots n0Host holds
   // device buffers of this run: carved from the handle's adjTab block while it has room (tabUsed
   // bytes taken), else allocated on their own (own, freed with the run); tabNeed is the total
   size_t tabUsed = 0, tabNeed = 0;
   std::vector<void*> own;
-  cudaStream_t side = nullptr;
-  cudaEvent_t fork = nullptr, join = nullptr;
   cudaStream_t side2 = nullptr;          // the next segment's recompute, beside the sweep
   cudaEvent_t fork2 = nullptr, join2 = nullptr;
-  // full segments replay captured graphs: [state set of the swept segment][with the next recompute]
-  cudaGraphExec_t segGraph[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
-  int64_t segGraphLaunches[2][2] = {{0, 0}, {0, 0}};
-  int segGraphCur = -1;                 // the adjoint buffer the graphs start from
-  int* slowCells = nullptr;  // flagged fluid cells (device), in index order
+  int* slowCells = nullptr;  // listed flagged fluid cells (device), in index order: all but the face rows'
   int nSlow = 0;
   int* sE1 = nullptr;        // [19][nSlow] pull records of the flagged cells
   int* sE2 = nullptr;
   int* sTgt = nullptr;
   void* sA1 = nullptr;       // R
   void* sA2 = nullptr;       // R
-  int nParts = 0;            // entries of blockPart
+  int nParts = 0;            // block sums of one adjoint step
 };
 
 namespace cells {
@@ -115,28 +92,21 @@ struct AdjLaunch3 {
   void* lamOut;          // lambda^n
   const uint32_t* flags;
   const void* xTab;      // per x: omega+, omega-, sigma, 0
-  const int* linkBase;
-  const long long* le1;
-  const long long* le2;
-  const void* la1;
-  const void* la2;
+  const uint8_t* rowBody;
   const void* lcF;
   const void* lq;
   const signed char* lqk;
   void* lamG;
   double* dqAcc;
-  double* blockPart;
-  unsigned* counter;
-  const int* n0Dev;      // first recorded step of the current segment (device)
-  int t;                 // this step's position in the segment: step n = *n0Dev + t
-  const double* uDev;    // inlet speed of each recorded step
-  const double* wDev;    // objective weight of each recorded step's force
-  double* dudn;          // dJ/du_n of each recorded step
+  double* blockPart;     // the step's dJ/du_n block sums
+  double u, w;           // the step's inlet speed, and the objective weight of its force
   long long N;
   int W, H, D;
-  int tileX;             // cell kernel block: tileX x (kAdjThreads / tileX) cells of x-rows
+  int off[cells::Q3];    // cell offset of each direction
   int absorbX0;          // first x of the absorbing layer (W when there is none)
-  int nCellBlocks;       // blocks of the cell kernel
+  int nCellBlocks, nSlowBlocks, nFaceBlocks;  // blocks of the roles
+  int roleZ;                                  // grid slices of the last two
+  int foff[4][cells::Q3];                     // face rows: element offset of direction i's source from the cell
   const int* slowCells;  // the flagged fluid cells, in index order
   int nSlow;
   const int* sE1;        // [19][nSlow]: the source of a one-source pull (coefficient 1), or the first
@@ -145,10 +115,10 @@ struct AdjLaunch3 {
   const int* sTgt;       // [19][nSlow]: element of a plain pull's adjoint, or -(link + 1)
   const void* sA1;       // R: coefficients (a2 = 0 for one source)
   const void* sA2;
-  int nParts;            // blockPart entries: nCellBlocks + blocks of the flagged-cell kernel
+  int nParts;            // blockPart entries: nCellBlocks + nSlowBlocks + nFaceBlocks
   // transposed map
   int nRows;
-  const long long* rowElem;
+  const int* rowElem;
   const unsigned char* rowSet;
   const int* rowStart;
   const int* entLink;
@@ -156,11 +126,21 @@ struct AdjLaunch3 {
   const void* rowPhi;
 };
 
+// What the table kernels read.
+struct AdjTables3 {
+  const uint32_t* flags;
+  const float* sdf;
+  const uint8_t* rowBody;
+  long long N;
+  int W, H, D;
+  int component;
+  int facePairs;  // the face rows go to the x-pair role
+};
+
 constexpr int kAdjThreads = 128;
-// One adjoint step (precision 0 or 3): the interior-cell kernel on `s` and the flagged-cell kernel
-// on `side` run concurrently (they write disjoint elements), then the boundary-element kernel on
-// `s`. fork and join are events used to order the two streams.
-cudaError_t launch_adjoint_step3(int precision, const AdjLaunch3& a, cudaStream_t s, cudaStream_t side,
-                                 cudaEvent_t fork, cudaEvent_t join);
+constexpr int kAdjTileX = 32;
+// One adjoint step (precision 0 or 3): the interior and flagged cells in one launch, then the
+// boundary-element kernel.
+cudaError_t launch_adjoint_step3(int precision, const AdjLaunch3& a, cudaStream_t s);
 
 }  // namespace cells
