@@ -55,7 +55,8 @@ struct StepLaunch3 {
   int rampKind, rampEvery;
   double rampTarget, rampSteps;
   double lambda, smagC2;
-  int par, sample;
+  int par;
+  int sample;            // 1: the step's force goes to the ring, 2: the body blocks' partials only, 0: neither
 };
 
 // One time step: one launch of the step kernel. precision: cells_precision (0 f32, 1 f16, 2 bf16,
@@ -63,10 +64,16 @@ struct StepLaunch3 {
 namespace fast {
 cudaError_t launch_step3(int precision, const StepLaunch3& a, cudaStream_t s);
 int body_blocks3(int nBody);
+// The force samples of a run of steps from their partials (perStep of each), into the ring.
+cudaError_t launch_sum_samples3(const double4* partials, int perStep, int nSamples, double4* history, DevState3* st,
+                                cudaStream_t s);
 }
 namespace exact {
 cudaError_t launch_step3(int precision, const StepLaunch3& a, cudaStream_t s);
 int body_blocks3(int nBody);
+// The force samples of a run of steps from their partials (perStep of each), into the ring.
+cudaError_t launch_sum_samples3(const double4* partials, int perStep, int nSamples, double4* history, DevState3* st,
+                                cudaStream_t s);
 }
 
 struct AuxLaunch3 {

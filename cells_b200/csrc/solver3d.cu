@@ -192,15 +192,68 @@ void Cells3D::rebuild_flags() {
   argGen++;  // the body list and links are baked into step graphs
 }
 
-// Enqueues the step kernel of one step of parity par on `main`; returns the kernels launched.
-int Cells3D::enqueue_step(int par, bool sample, cudaStream_t main) {
-  (void)main;
-  enqueue_step_between(f[par], f[par ^ 1], par, sample);
-  return 1;
+// The force partials of a run of `samples` sampled steps: the sum over the body blocks then runs once
+// per run, off the steps' critical path (the block count, the fences and the last block's sum cost
+// about 3.6 us of every sampled step). False when they would take too much memory.
+bool Cells3D::run_partials(int samples) {
+  const size_t need = (size_t)samples * (size_t)(nBody > 0 ? fast::body_blocks3(nBody) : 0);
+  if (dev.fake || runPartialsOff || need * sizeof(double4) > kRunPartialBytes) return false;
+  if (need > runPartialCap) {
+    dev.release(runPartials);
+    runPartials = nullptr;
+    runPartialCap = 0;
+    argGen++;  // step graphs bake the address
+    try {
+      runPartials = (double4*)dev.alloc(need * sizeof(double4), "force partials of a run");
+    } catch (const AllocError&) {
+      runPartialsOff = true;
+      return false;
+    }
+    runPartialCap = need;
+  }
+  return true;
+}
+
+void Cells3D::sum_samples(int samples) {
+  const int perStep = nBody > 0 ? fast::body_blocks3(nBody) : 0;
+  check_cuda(fast::launch_sum_samples3(runPartials, perStep, samples, history, st, dev.stream), "force sum kernel");
+}
+
+void Cells3D::enqueue_step(int par, bool sample, int sampled) {
+  StepLaunch3 a = step_launch(f[par], f[par ^ 1], par, sample);
+  if (sample && sampled >= 0) {
+    a.sample = 2;
+    a.partials = runPartials + (size_t)sampled * (size_t)(nBody > 0 ? fast::body_blocks3(nBody) : 0);
+  }
+  launch_step(a, dev.stream);
+}
+
+// The next step of a run of steps launched one by one, `samples` of which wait for their sum; the
+// last one adds them up.
+void Cells3D::enqueue_run_step(bool sample, bool last, int& samples) {
+  const bool split = sample && (!last || samples > 0) && run_partials(kGraphSteps);
+  enqueue_step(parity, sample, split ? samples : -1);
+  dev.launches++;
+  if (split) samples++;
+  if (samples == kGraphSteps || (last && samples > 0)) {
+    sum_samples(samples);
+    dev.launches++;
+    samples = 0;
+  }
+}
+
+void Cells3D::launch_step(const StepLaunch3& a, cudaStream_t stream) {
+  check_cuda(cfg.arithmetic == CELLS_ARITH_EXACT ? exact::launch_step3(prec, a, stream)
+                                                 : fast::launch_step3(prec, a, stream),
+             "step kernel");
 }
 
 void Cells3D::enqueue_step_between(const void* src, void* dst, int par, bool sample, cudaStream_t stream) {
-  cudaStream_t main = stream ? stream : dev.stream;
+  launch_step(step_launch(src, dst, par, sample), stream ? stream : dev.stream);
+}
+
+// The arguments of one step.
+StepLaunch3 Cells3D::step_launch(const void* src, void* dst, int par, bool sample) const {
   StepLaunch3 a;
   a.src = src;
   a.dst = dst;
@@ -230,9 +283,7 @@ void Cells3D::enqueue_step_between(const void* src, void* dst, int par, bool sam
   a.smagC2 = cfg.smagorinsky * cfg.smagorinsky;
   a.par = par;
   a.sample = sample ? 1 : 0;
-  check_cuda(cfg.arithmetic == CELLS_ARITH_EXACT ? exact::launch_step3(prec, a, main)
-                                                 : fast::launch_step3(prec, a, main),
-             "step kernel");
+  return a;
 }
 
 // Steps repeat with period lcm(2, force_every) in their launch arguments (parity and sampling);
@@ -248,15 +299,22 @@ void Cells3D::build_graph(int phase) {
   if (g.exec) cudaGraphExecDestroy(g.exec);
   g.exec = nullptr;
   const int every = cfg.force_every;
-  int launches = 0;
+  const bool split = every > 0 && run_partials(kGraphSteps);
+  int launches = 0, samples = 0;
   check_cuda(cudaStreamBeginCapture(dev.stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
   int par = phase % 2;
   int64_t s = phase;
   for (int k = 0; k < kGraphSteps; k++) {
     const bool sample = every > 0 && ((s + 1) % every) == 0;
-    launches += enqueue_step(par, sample, dev.stream);
+    enqueue_step(par, sample, split ? samples : -1);
+    launches++;
+    samples += sample;
     par ^= 1;
     s++;
+  }
+  if (split && samples > 0) {
+    sum_samples(samples);
+    launches++;
   }
   cudaGraph_t graph = nullptr;
   check_cuda(cudaStreamEndCapture(dev.stream, &graph), "cudaStreamEndCapture");
@@ -270,6 +328,7 @@ void Cells3D::build_graph(int phase) {
 void Cells3D::launch_steps(int64_t n) {
   const int every = cfg.force_every;
   const int period = graph_period();
+  int samples = 0;  // sampled steps launched one by one, whose partials wait for their sum
   while (n > 0) {
     if (!dev.fake && useGraphs && period <= kMaxGraphPeriod && n >= kGraphSteps) {
       // kGraphSteps steps as one graph launch: parity and sampling depend on step % period only
@@ -294,7 +353,8 @@ void Cells3D::launch_steps(int64_t n) {
         st->sample = s + 1;
       }
     } else {
-      dev.launches += enqueue_step(parity, sample, dev.stream);
+      // a single step reduces its force itself; the partials of a run are summed once
+      enqueue_run_step(sample, n == 1, samples);
     }
     parity ^= 1;
     step++;

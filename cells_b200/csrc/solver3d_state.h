@@ -78,6 +78,12 @@ struct Cells3D : cells::HandleBase {
   void* adjTab = nullptr;
   size_t adjTabBytes = 0;
 
+  // force partials of the sampled steps of one run (a step graph, or steps launched one by one)
+  double4* runPartials = nullptr;
+  size_t runPartialCap = 0;
+  bool runPartialsOff = false;  // they did not fit
+  static constexpr size_t kRunPartialBytes = 64u << 20;
+
   // device scratch of the macro-field products (fields3d.cu), grown on demand
   void* scratch = nullptr;
   size_t scratchBytes = 0;
@@ -118,7 +124,14 @@ struct Cells3D : cells::HandleBase {
   void upload_xtab();
   void rebuild_flags();
   void build_body_list();
-  int enqueue_step(int par, bool sample, cudaStream_t main);
+  // the step of parity par; sampled steps of a run write their force partials to slot `sampled` of
+  // runPartials (run_partials), or reduce them in the step itself when sampled is -1
+  void enqueue_step(int par, bool sample, int sampled);
+  bool run_partials(int samples);
+  void enqueue_run_step(bool sample, bool last, int& samples);
+  void sum_samples(int samples);
+  cells::StepLaunch3 step_launch(const void* src, void* dst, int par, bool sample) const;
+  void launch_step(const cells::StepLaunch3& a, cudaStream_t stream);
   // one step from src to dst (any buffers of 19 N populations), parity par of the device state, on
   // `stream` (nullptr: the handle's stream)
   void enqueue_step_between(const void* src, void* dst, int par, bool sample, cudaStream_t stream = nullptr);
