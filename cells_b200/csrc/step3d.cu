@@ -29,7 +29,9 @@
 //     from a W-entry table that the host fills with the reference's f32 arithmetic;
 //   * every block first asks L2 for the pull sources of the interior tile a few z planes ahead of
 //     its own (prefetch.global.L2, one 128-byte line per thread, no registers held), so the loads
-//     of the blocks that start later find their lines in L2 instead of waiting for DRAM.
+//     of the blocks that start later find their lines in L2 instead of waiting for DRAM;
+//   * consecutive steps take the interior planes in opposite order, so a step starts on the planes that
+//     the step before it wrote last.
 #include <algorithm>
 
 #include "kernels3d.h"
@@ -82,6 +84,7 @@ struct StepArgs3 {
   int roleZ;                     // grid z-slices holding the face and body roles
   int absorbX0;                  // first x of the absorbing layer (W when there is none)
   int pfPlanes;                  // L2 prefetch distance in z planes of interior tiles (0: none)
+  int reverse;                   // interior planes from z = D-2 down to 1
   int pfShift, pfRowShift;       // log2 of the 128-byte stretches per tile row and of the rows
   // x-pair face tiles (facePairs = 1): the rows with one outside side -- rows y = 1 .. H-2 of the
   // z = 0 / z = D-1 planes (sides 0 / 1) and the y = 0 / y = H-1 rows of the planes between
@@ -1025,7 +1028,7 @@ __device__ __forceinline__ void prefetch_tile_ahead(const StepArgs3<C>& a) {
   if (bz < a.roleZ || bz >= (int)gridDim.z) return;
   const int tid = threadIdx.x + blockDim.x * threadIdx.y;
   const int perDir = a.pfRowShift + a.pfShift;  // log2 of the stretches per population
-  const long long plane = (long long)a.H * (1 + bz - a.roleZ);
+  const long long plane = (long long)a.H * (a.reverse ? a.D - 2 - (bz - a.roleZ) : 1 + bz - a.roleZ);
   for (int t = tid; t < (Q3 << perDir); t += kStepThreads) {
     const int i = t >> perDir;
     const int r = (t >> a.pfShift) & ((1 << a.pfRowShift) - 1);
@@ -1076,7 +1079,7 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR))
   // block-uniform choice of the code for tiles that overlap the absorbing layer or hold the outlet
   const int tx1 = (blockIdx.x + 1) * a.tileTX;  // end of the tile's x range
   const bool abs = tx1 > a.absorbX0, out = tx1 >= a.W;
-  const int tz = blockIdx.z - a.roleZ;
+  const int tz = a.reverse ? gridDim.z - 1 - blockIdx.z : blockIdx.z - a.roleZ;
   if constexpr (PAIR) {
     if (out)
       abs ? bulk_pair_role<C, SMAG, true, true>(a, tz) : bulk_pair_role<C, SMAG, false, true>(a, tz);
@@ -1167,6 +1170,13 @@ static cudaError_t launch_step3_t(const StepLaunch3& L, cudaStream_t s) {
   a.bodyBlocks = (L.nBody > 0 || L.sample == 1) ? body_blocks3(L.nBody) : 0;
   a.roleZ = (a.shellBlocks + a.bodyBlocks + a.faceBlocks + perSlice - 1) / perSlice;
   const dim3 grid(tilesX, tilesY, a.roleZ + zInterior);
+  // Steps of odd parity take the planes from the far end: a step then starts where the one before it
+  // ended, on planes that are still in L2. B200, us per step forward -> alternating: f32 192x96x96
+  // 43.1 -> 41.4, 160x80x80 27.9 -> 25.8, 161x83x75 36.9 -> 35.5; f16 192x96x96 28.9 -> 27.6, 160x80x80
+  // 18.9 -> 17.7; f64 128x64x64 29.5 -> 27.7. A buffer of several times L2 gains nothing (f32
+  // 256x128x128, 319 MB: 100.6 -> 99.9), and f64 loses where the buffer no longer fits L2 (160x80x80,
+  // 156 MB: 50.2 -> 51.7; 192x96x96: 85.4 -> 87.4), so f64 stops at 100 MB and the others at 320 MB.
+  a.reverse = L.par && 19ull * (unsigned long long)L.N * sizeof(S) <= (sizeof(S) == 8 ? 100ull << 20 : 320ull << 20);
   // prefetch distance, measured on B200 at 192x96x96 and 256x128x128 (sphere tunnel, 1000 steps):
   // 16-bit storage 4 planes (+1.5-3% and +6.5-8%), f32 1 plane (+0.5-1.5%), f64 the plane count
   // nearest 270 tiles (+5% and +2%); farther prefetches lost to the demand loads
