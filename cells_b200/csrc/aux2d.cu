@@ -103,6 +103,71 @@ __global__ void flags2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, uint3
   }
 }
 
+// The rules of pullSlow (src/shaders/step.ts:119-175) for every flagged direction, as words (Rule2).
+template <class R, class R2>
+__global__ void rules2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, const uint32_t* __restrict__ flags,
+                              uint32_t* __restrict__ code, R2* __restrict__ qCoef, int qCap) {
+  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (idx >= a.N) return;
+  const uint32_t fl = flags[idx];
+  if (fl == 0u || (fl & FLAG2_SOLID)) {
+    code[idx] = fl == 0u ? 0u : CODE2_SOLID;
+    return;
+  }
+  const int W = a.W, H = a.H;
+  const int y = (int)(idx / W);
+  const int x = (int)(idx - (long long)y * W);
+  const int slot = (int)(fl >> BIDX2_SHIFT);
+  uint32_t w = ((fl & FLAG2_INLET) ? CODE2_INLET : 0u) | ((fl & FLAG2_OUTLET) ? CODE2_OUTLET : 0u) |
+               (slot ? CODE2_SLOT : 0u);
+  // an inlet (outlet) cell whose only flagged directions are the three that Zou-He replaces needs no rule
+  constexpr uint32_t kInletPlain = FLAG2_INLET | (1u << 1) | (1u << 5) | (1u << 8);
+  constexpr uint32_t kOutletPlain = FLAG2_OUTLET | (1u << 3) | (1u << 6) | (1u << 7);
+  for (int i = 1; i < Q2 && fl != kInletPlain && fl != kOutletPlain; i++) {
+    if (!(fl & (1u << i))) continue;
+    int sx = x - cx2(i), sy = y - cy2(i);
+    wrap2a(a, sx, sy);
+    const bool inX = sx >= 0 && sx < W, inY = sy >= 0 && sy < H;
+    uint32_t rule = RULE2_BOUNCE;
+    if (inX && inY) {
+      const long long s = (long long)sy * W + sx;
+      if ((flags[s] & FLAG2_SOLID) == 0u) {
+        rule = RULE2_PULL;
+      } else if (slot == 0 || slot > qCap) {
+        w |= CODE2_GENERAL;
+      } else {
+        const R dF = (R)sdf[idx], dS = (R)sdf[s];
+        const R den = (dF - dS) < (R)1e-6 ? (R)1e-6 : (dF - dS);
+        R q = dF / den;
+        q = q < (R)1e-3 ? (R)1e-3 : (R(1) < q ? R(1) : q);
+        R2 c;
+        c.x = R(2) * q;
+        c.y = R(0);
+        if (q < R(0.5)) {
+          rule = RULE2_BODY_0;
+          int nx = x + cx2(i), ny = y + cy2(i);
+          wrap2a(a, nx, ny);
+          if (nx >= 0 && nx < W && ny >= 0 && ny < H && (flags[(long long)ny * W + nx] & FLAG2_SOLID) == 0u) {
+            rule = RULE2_BODY_N;
+            c.y = R(1) - R(2) * q;
+          }
+        } else {
+          rule = RULE2_BODY_H;
+          c.y = (R(2) * q - R(1)) / (R(2) * q);
+        }
+        qCoef[(long long)(slot - 1) * 8 + (i - 1)] = c;
+      }
+    } else if (!inY) {
+      const int mode = sy < 0 ? a.bottom : a.top;
+      if (mode == Y2_SLIP) rule = inX ? RULE2_SLIP : RULE2_SLIP_HERE;
+      if (mode == Y2_MOVING) rule = RULE2_MOVING;
+    }
+    w |= rule << (3 * (i - 1));
+  }
+  if (w & CODE2_GENERAL) w &= ~CODE2_RULES;
+  code[idx] = w;
+}
+
 // initShader, src/shaders/aux.ts:92-111
 template <class C>
 __global__ void init2_kernel(AuxLaunch2 a, const float4* __restrict__ mac, typename C::S* __restrict__ fA,
@@ -220,6 +285,15 @@ __global__ void set_state2_kernel(DevState2* st, int which, unsigned step, doubl
       return cudaErrorInvalidValue;                      \
     }                                                    \
   } while (0)
+
+cudaError_t launch_rules2(int precision, const AuxLaunch2& a, const float* sdf, const uint32_t* flags, uint32_t* code,
+                          void* qCoef, int qCap, cudaStream_t s) {
+  if (precision == 0)
+    rules2_kernel<float, float2><<<blocks_for2(a.N, 256), 256, 0, s>>>(a, sdf, flags, code, (float2*)qCoef, qCap);
+  else
+    rules2_kernel<double, double2><<<blocks_for2(a.N, 256), 256, 0, s>>>(a, sdf, flags, code, (double2*)qCoef, qCap);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_flags2(int precision, const AuxLaunch2& a, const float* sdf, uint32_t* flags, void* fA, void* fB,
                           const float4* mac, unsigned* counter, cudaStream_t s) {

@@ -36,6 +36,26 @@ __host__ __device__ __forceinline__ constexpr int mirror_y2(int i) {
   constexpr int v[Q2] = {0, 1, 4, 3, 2, 8, 7, 6, 5};
   return v[i];
 }
+// The block kernel's word per cell (Tunnel2::code): how each flagged direction i obtains its
+// population, resolved once per SDF or boundary mode (pullSlow, src/shaders/step.ts:119-175), 3 bits at
+// 3 (i - 1).
+enum Rule2 : uint32_t {
+  RULE2_PULL = 0,      // plain pull, across a periodic seam too
+  RULE2_BOUNCE = 1,    // f_j of the cell (j opposite to i): no-slip and x walls, open-boundary placeholders
+  RULE2_SLIP = 2,      // mirrored population of the row, from x - c_ix
+  RULE2_SLIP_HERE = 3, // the same from the cell itself (the row ends there)
+  RULE2_MOVING = 4,    // f_j plus the moving wall's momentum
+  RULE2_BODY_N = 5,    // Bouzidi, q < 1/2 with a fluid node behind: c1 f_j + c2 f_j(x + c_i), c1 = 2q, c2 = 1 - 2q
+  RULE2_BODY_0 = 6,    // Bouzidi, q < 1/2 without one: f_j
+  RULE2_BODY_H = 7     // Bouzidi, q >= 1/2: f_j / c1 + c2 f_i of the cell, c1 = 2q, c2 = (2q - 1) / (2q)
+};
+constexpr uint32_t CODE2_RULES = (1u << 24) - 1u;
+constexpr uint32_t CODE2_INLET = 1u << 24;
+constexpr uint32_t CODE2_OUTLET = 1u << 25;
+constexpr uint32_t CODE2_SLOT = 1u << 26;     // the cell has a force slot
+constexpr uint32_t CODE2_GENERAL = 1u << 27;  // more body cells than coefficient slots: the flag word's rules
+constexpr uint32_t CODE2_SOLID = 1u << 31;
+
 // 4/9, 1/9, 1/36: the WGSL literals of the JS doubles, rounded to R
 template <class R>
 __host__ __device__ __forceinline__ R w2(int i) {
@@ -73,6 +93,8 @@ struct Tunnel2 {
   void* f[2];             // populations A and B (storage type), f[i * N + x + W * y]
   const uint32_t* flags;  // N
   const float* sdf;       // N
+  const uint32_t* code;   // N, the block kernel's rules of each cell
+  const void* qCoef;      // (c1, c2) of the body rules, [slot - 1][direction - 1], in the arithmetic type
   double2* partials;      // one force partial per tile
   double2* history;       // HISTORY2_LEN force samples
   DevState2* st;

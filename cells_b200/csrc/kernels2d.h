@@ -24,13 +24,39 @@ struct Step2Launch {
                                      // (0; 1 only to test the time-out path)
 };
 
+// k steps of every tunnel of a batch in one launch, tiles in shared memory (block2d.cu). A tile is
+// (regionX - 2 K) x (regionY - 2 K) cells of one tunnel; the launch's k steps are odd and at most K.
+constexpr int kBlockSteps2 = 7;  // largest K
+struct Block2Tunnel {
+  int tilesX, tiles, first;  // tiles per row, of the tunnel, and its first in the batch
+};
+struct Block2Launch {
+  const Tunnel2* tunnels;
+  const Block2Tunnel* layout;        // device array, one per tunnel
+  const unsigned short* tileTunnel;  // device array: the tunnel of each tile
+  int nTiles;
+  int regionX, regionY, rows;        // region of a block and cell rows per thread
+  int K, k;
+  int par;                           // parity of the first step
+  double2* partials;                 // force partials [step of the run][tile]; NULL: no sampling
+  int j0;                            // the launch's first step in the run
+};
+
 // precision: 0 f32, 3 f64. fast: FMA contraction allowed; exact: every operation rounds as written.
 namespace fast {
+cudaError_t launch_block2(int precision, const Block2Launch& a, cudaStream_t s);
+// The force samples of a run of n steps that ended on parity par, from its partials.
+cudaError_t launch_sum_samples2(const Tunnel2* tunnels, const Block2Tunnel* layout, int nTunnels, const double2* partials,
+                                int tiles, int n, int par, cudaStream_t s);
 cudaError_t launch_step2(int precision, const Step2Launch& a, cudaStream_t s);
 cudaError_t launch_step2_persistent(int precision, const Step2Launch& a, cudaStream_t s);
 int persistent_blocks2(int precision, int threads);  // resident blocks of the persistent kernel
 }
 namespace exact {
+cudaError_t launch_block2(int precision, const Block2Launch& a, cudaStream_t s);
+// The force samples of a run of n steps that ended on parity par, from its partials.
+cudaError_t launch_sum_samples2(const Tunnel2* tunnels, const Block2Tunnel* layout, int nTunnels, const double2* partials,
+                                int tiles, int n, int par, cudaStream_t s);
 cudaError_t launch_step2(int precision, const Step2Launch& a, cudaStream_t s);
 cudaError_t launch_step2_persistent(int precision, const Step2Launch& a, cudaStream_t s);
 int persistent_blocks2(int precision, int threads);
@@ -47,6 +73,10 @@ struct AuxLaunch2 {
 // the refill of uncovered cells from mac.
 cudaError_t launch_flags2(int precision, const AuxLaunch2& a, const float* sdf, uint32_t* flags, void* fA, void* fB,
                           const float4* mac, unsigned* counter, cudaStream_t s);
+// The block kernel's rule words and Bouzidi coefficients from the flags and the SDF; cells whose force
+// slot exceeds qCap keep the general rules.
+cudaError_t launch_rules2(int precision, const AuxLaunch2& a, const float* sdf, const uint32_t* flags, uint32_t* code,
+                          void* qCoef, int qCap, cudaStream_t s);
 // initShader (src/shaders/aux.ts:92-111): both buffers to feq(rho, ux, uy) of mac.
 cudaError_t launch_init2(int precision, const AuxLaunch2& a, const float4* mac, void* fA, void* fB, cudaStream_t s);
 // macroShader (src/shaders/aux.ts:115-140); sets status bit 1 on a non-finite value.

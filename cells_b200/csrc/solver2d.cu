@@ -9,6 +9,7 @@
 // live in a device-side descriptor that the kernel reads every step, so parameter changes need no
 // graph rebuild; the inlet speed and step counter live in per-tunnel device state.
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <deque>
@@ -25,6 +26,7 @@ namespace {
 
 constexpr int kGraphSteps2 = 100;
 constexpr int kPersistentChunk = 500;
+constexpr int kRunSteps2 = 126;  // steps whose force partials wait for one sum: 18 launches of 7
 
 struct Shape2 {
   int tx, ty;
@@ -39,6 +41,9 @@ struct Tunnel2Host {
   void* f[2] = {nullptr, nullptr};
   uint32_t* flags = nullptr;
   float* sdf = nullptr;
+  uint32_t* code = nullptr;  // the block kernel's rules (Tunnel2::code, qCoef)
+  void* qCoef = nullptr;
+  int qCap = 0;
   float4* macro = nullptr;
   double2* partials = nullptr;
   int partialsCap = 0;
@@ -119,6 +124,21 @@ struct Cells2DBatch : HandleBase {
   unsigned barrierErrors = 0;
   unsigned barrierExtra = 0;  // test hook: arrivals a persistent launch waits for that never come
 
+  // several steps per launch (block2d.cu): the default way to take two steps or more, unless a launch
+  // shape was asked for or the autotuner found another one faster
+  bool blockWanted = false, blockOn = false;  // blockOn: wanted and possible (tables, periodic sides >= 3)
+  int blockK = 0, regionX = 0, regionY = 0, regionRows = 1;
+  int nBlockTiles = 0;
+  Block2Tunnel* dLayout = nullptr;
+  unsigned short* dBlockTiles = nullptr;
+  double2* runPartials = nullptr;  // force partials of a run of kRunSteps2 steps
+  bool runPartialsOff = false;     // they did not fit
+  void alloc_rules();
+  void choose_block();
+  bool samples_force() const;
+  bool run_partials();
+  void launch_blocks(int64_t n, int par, int allowSample);
+
   struct StepGraph {
     cudaGraphExec_t exec = nullptr;
     uint64_t gen = 0;
@@ -129,6 +149,7 @@ struct Cells2DBatch : HandleBase {
   void upload_tunnel(int k);
   void write_state(int k, int which);
   void rebuild_flags(int k);
+  void resolve_rules(int k);
   AuxLaunch2 aux(int k) const;
   void launch_raw(int64_t n, int par, int allowSample);
   void launch_steps(int64_t n);
@@ -235,6 +256,8 @@ void Cells2DBatch::upload_tunnel(int k) {
   d.f[1] = T.f[1];
   d.flags = T.flags;
   d.sdf = T.sdf;
+  d.code = T.code;
+  d.qCoef = T.qCoef;
   d.partials = T.partials;
   d.history = T.history;
   d.st = T.st;
@@ -307,10 +330,191 @@ void Cells2DBatch::rebuild_flags(int k) {
   dev.memset0(dCounter, sizeof(unsigned));
   check_cuda(launch_flags2(prec, a, T.sdf, T.flags, T.f[0], T.f[1], T.macro, dCounter, dev.stream), "flags kernel");
   dev.launches += 2;
+  resolve_rules(k);
+}
+
+// The block kernel's tables. A device without room for them steps one launch at a time.
+void Cells2DBatch::alloc_rules() {
+  if (dev.fake) return;
+  unsigned long long total = 1u << 22;
+  for (Tunnel2Host& T : t) {
+    // coefficient slots for the cells around a body: a few times the grid's outline (further body cells
+    // keep the general rules)
+    T.qCap = (int)std::min<long long>(T.N, 4LL * (T.W + T.H));
+    total += (unsigned long long)T.N * 4 + (unsigned long long)T.qCap * 16 * bpp;
+  }
+  if (total > dev.free_bytes()) return;
+  try {
+    for (Tunnel2Host& T : t) {
+      T.qCoef = dev.alloc((size_t)T.qCap * 16 * bpp, "boundary coefficients");
+      T.code = (uint32_t*)dev.alloc((size_t)T.N * 4, "boundary rules");
+    }
+  } catch (const AllocError&) {
+    for (Tunnel2Host& T : t) {
+      if (T.qCoef) dev.release(T.qCoef);
+      if (T.code) dev.release(T.code);
+      T.qCoef = nullptr;
+      T.code = nullptr;
+    }
+  }
+}
+
+// The block kernel's rules follow the flags and the SDF.
+void Cells2DBatch::resolve_rules(int k) {
+  Tunnel2Host& T = t[(size_t)k];
+  if (!T.code) return;
+  check_cuda(launch_rules2(prec, aux(k), T.sdf, T.flags, T.code, T.qCoef, T.qCap, dev.stream), "rules kernel");
+  dev.launches++;
+}
+
+// A region of the block kernel, the steps K per launch, and the number of tiles up to which it is taken.
+struct Region2 {
+  int x, y, rows, K, maxTiles;
+};
+// us per step of one tunnel with a circle and Smagorinsky off, FP32 [one step per launch before]:
+//                 128x128  400x100  500x140  700x180  1000x250  1500x400  2000x500  4000x1000
+//   32x28x1 K=7     2.70     2.83     3.65     4.96      8.53     18.78     30.68     119.81
+//   32x32x1 K=5     3.14     3.19     3.16     3.75      6.36     13.85     22.07      86.06
+//   64x32x2 K=5     4.62     4.88     5.11     5.09      5.37     10.41     16.71      63.49
+//   64x48x3 K=5     6.51     5.97     6.42     7.55      7.63     10.29     15.18      57.63
+//   [before         9.48    12.13    11.98    14.47     21.72     29.90     45.48     192.38]
+// and for 64 NACA tunnels with Smagorinsky: 189, 138, 102 to 105, 95 [117]. A grid whose tiles fit on the SMs
+// at once pays for the latency of a launch, spread over its steps: small regions, many steps. A larger one
+// is bound by issue, and the margins are computed twice: (x - 2K)(y - 2K) / xy of the work is kept, so the
+// region grows with the number of tiles until shared memory is full (64x48 in two buffers).
+// FP64, same order: 32x24x2 K=7 3.62 (128x128), 4.26 (400x100), 7.89 (700x180), 14.3 (1000x250), 209 (4000x1000);
+// 32x32x2 K=5 4.35, 5.28, 5.15, 9.06, 129; 32x32x2 K=3 5.53, 4.32, 6.08, 8.58, 126 [9.09, 12.3, 15.9, 25.0, 312].
+constexpr Region2 kRegions32[] = {{32, 28, 1, 7, 222}, {32, 32, 1, 5, 296}, {64, 32, 2, 5, 444}, {64, 48, 3, 5, INT_MAX}};
+constexpr Region2 kRegions64[] = {{32, 24, 2, 7, 296}, {32, 32, 2, 5, 296}, {32, 32, 2, 3, INT_MAX}};
+
+// The block kernel's region and step count, its tiles numbered tunnel by tunnel, and the tile -> tunnel map.
+void Cells2DBatch::choose_block() {
+  const bool on = blockOn;
+  blockOn = false;
+  if (!t[0].code) return;
+  int limit = kBlockSteps2;
+  for (const Tunnel2Host& T : t) {
+    // a periodic margin is loaded from the other side once
+    if (T.cfg.left == CELLS_X_PERIODIC || T.cfg.right == CELLS_X_PERIODIC) limit = std::min(limit, T.W);
+    if (T.cfg.bottom == CELLS_Y_PERIODIC || T.cfg.top == CELLS_Y_PERIODIC) limit = std::min(limit, T.H);
+  }
+  limit = (limit - 1) | 1;  // the largest odd number up to it
+  if (limit < 3) return;
+  Region2 r = {};
+  int K = 0;
+  long long tiles = 0;
+  for (const Region2* c = prec == CELLS_FP64 ? kRegions64 : kRegions32;; c++) {
+    r = *c;
+    K = std::min(r.K, limit);
+    tiles = 0;
+    for (const Tunnel2Host& T : t)
+      tiles += (long long)((T.W + r.x - 2 * K - 1) / (r.x - 2 * K)) * ((T.H + r.y - 2 * K - 1) / (r.y - 2 * K));
+    if (tiles <= r.maxTiles || r.maxTiles == INT_MAX) break;
+  }
+  if (tiles > INT_MAX) return;
+  if (dLayout && r.x == regionX && r.y == regionY && K == blockK) {
+    blockOn = true;
+    return;
+  }
+  std::vector<unsigned short> map;
+  std::vector<Block2Tunnel> layout;
+  map.reserve((size_t)tiles);
+  const int tx = r.x - 2 * K, ty = r.y - 2 * K;
+  for (size_t k = 0; k < t.size(); k++) {
+    Block2Tunnel L;
+    L.tilesX = (t[k].W + tx - 1) / tx;
+    L.tiles = L.tilesX * ((t[k].H + ty - 1) / ty);
+    L.first = (int)map.size();
+    layout.push_back(L);
+    map.insert(map.end(), (size_t)L.tiles, (unsigned short)k);
+  }
+  if (on) dev.sync();  // launches that read the layout before
+  if (dLayout) dev.release(dLayout);
+  if (dBlockTiles) dev.release(dBlockTiles);
+  if (runPartials) dev.release(runPartials);
+  dLayout = nullptr;
+  dBlockTiles = nullptr;
+  runPartials = nullptr;
+  runPartialsOff = false;
+  try {
+    dLayout = (Block2Tunnel*)dev.alloc(layout.size() * sizeof(Block2Tunnel), "block layout");
+    dBlockTiles = (unsigned short*)dev.alloc(map.size() * sizeof(unsigned short), "block tile map");
+  } catch (const AllocError&) {
+    if (dLayout) dev.release(dLayout);
+    dLayout = nullptr;
+    return;  // one step per launch
+  }
+  regionX = r.x;
+  regionY = r.y;
+  regionRows = r.rows;
+  blockK = K;
+  nBlockTiles = (int)map.size();
+  dev.h2d(dLayout, layout.data(), layout.size() * sizeof(Block2Tunnel));
+  dev.h2d(dBlockTiles, map.data(), map.size() * sizeof(unsigned short));
+  dev.sync();  // the host vectors die here
+  blockOn = true;
+}
+
+bool Cells2DBatch::samples_force() const {
+  for (const Tunnel2Host& T : t)
+    if (T.cfg.force_every > 0) return true;
+  return false;
+}
+
+bool Cells2DBatch::run_partials() {
+  if (runPartials) return true;
+  if (runPartialsOff) return false;
+  try {
+    runPartials = (double2*)dev.alloc((size_t)nBlockTiles * kRunSteps2 * sizeof(double2), "force partials of a run");
+  } catch (const AllocError&) {
+    runPartialsOff = true;
+  }
+  return runPartials != nullptr;
+}
+
+// n steps from parity par, an odd number at most blockK per launch; the force partials of up to
+// kRunSteps2 steps are summed together.
+void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
+  const bool sampled = allowSample && samples_force();
+  const bool ex = arithmetic == CELLS_ARITH_EXACT;
+  Block2Launch a;
+  a.tunnels = dTunnels;
+  a.layout = dLayout;
+  a.tileTunnel = dBlockTiles;
+  a.nTiles = nBlockTiles;
+  a.regionX = regionX;
+  a.regionY = regionY;
+  a.rows = regionRows;
+  a.K = blockK;
+  a.partials = sampled ? runPartials : nullptr;
+  a.j0 = 0;
+  while (n > 0) {
+    a.k = (int)std::min<int64_t>(std::min<int64_t>(n, blockK), kRunSteps2 - a.j0);
+    if (a.k % 2 == 0) a.k--;
+    a.par = par;
+    check_cuda(ex ? exact::launch_block2(prec, a, dev.stream) : fast::launch_block2(prec, a, dev.stream),
+               "block step kernel");
+    dev.launches++;
+    par ^= 1;
+    n -= a.k;
+    a.j0 += a.k;
+    if (sampled && (n == 0 || a.j0 == kRunSteps2)) {
+      check_cuda(fast::launch_sum_samples2(dTunnels, dLayout, (int)t.size(), runPartials, nBlockTiles, a.j0, par,
+                                           dev.stream),
+                 "force sum kernel");
+      dev.launches++;
+      a.j0 = 0;
+    }
+    if (!sampled) a.j0 = 0;
+  }
 }
 
 // n steps from parity par on the device only (no host bookkeeping).
 void Cells2DBatch::launch_raw(int64_t n, int par, int allowSample) {
+  if (blockOn && n >= 2 && (!(allowSample && samples_force()) || run_partials())) {
+    launch_blocks(n, par, allowSample);
+    return;
+  }
   Step2Launch a;
   a.tunnels = dTunnels;
   a.tileTunnel = dTileTunnel;
@@ -530,9 +734,12 @@ static Cells2DBatch* create_batch(const Cells2DConfig* cfgs, int count) {
     // 64 x 2, which the autotuner picked for a single 400 x 100 tunnel (cells2d_batch_autotune
     // retunes a batch for its own sizes)
     const int wg = cfgs[0].workgroup_size;
-    if (wg == 0)
+    b->blockWanted = wg == 0;
+    b->alloc_rules();
+    if (wg == 0) {
       b->set_layout(64, 2, 0);
-    else
+      b->choose_block();
+    } else
       b->set_layout(32, wg == 64 ? 2 : (wg == 256 ? 8 : 4), 0);
     for (int k = 0; k < count; k++) {
       b->write_state(k, 1 | 2 | 4 | 8);
@@ -682,6 +889,7 @@ int cells2d_update(Cells2D* h, const Cells2DConfig* c) {
   // the boundary modes enter the flags (src/shaders/aux.ts:33-67); the reference rebuilds them on
   // the next setSdf only, which leaves flags that disagree with the new modes: rebuild now
   if (modes) h->b->rebuild_flags(h->k);
+  if (modes && h->b->blockWanted) h->b->choose_block();  // a periodic side bounds the steps per launch
   C2_CATCH(h, kAllocPrefix)
 }
 
@@ -765,6 +973,7 @@ static void brush_one(Cells2D* h, double cx, double cy, double r, int erase) {
                            y1 - y0 + 1, h->b->dev.stream),
              "brush kernel");
   h->b->dev.launches++;
+  h->b->resolve_rules(h->k);  // the links' fractions follow the SDF at once, the flags on the next rebuild
 }
 
 int cells2d_brush(Cells2D* h, double cx, double cy, double r, int erase, int rebuild) {
@@ -1180,6 +1389,7 @@ int cells2d_batch_set_launch(Cells2DBatch* b, int32_t tile_x, int32_t tile_y, in
   for (const Shape2& sh : kShapes) known = known || (sh.tx == tile_x && sh.ty == tile_y);
   if (!known) throw Error(CELLS_E_INVALID, "unsupported tile shape");
   b->dev.sync();
+  b->blockWanted = b->blockOn = false;
   b->set_layout(tile_x, tile_y, persistent ? 1 : 0);
   C2_CATCH(b, kAllocPrefix)
 }
@@ -1201,6 +1411,7 @@ int cells2d_batch_autotune(Cells2DBatch* b, int32_t trial_steps, Cells2DInfo* in
     b->dev.sync();
     const int par0 = b->parity;
     const int tx0 = b->tileX, ty0 = b->tileY, pers0 = b->persistent;
+    const bool block0 = b->blockOn;
     std::vector<void*> save;  // per tunnel: its populations and device state before the trials
     // copies the snapshots back into the current parity's buffers and releases them
     auto restore = [&]() {
@@ -1233,6 +1444,18 @@ int cells2d_batch_autotune(Cells2DBatch* b, int32_t trial_steps, Cells2DInfo* in
       Shape2 bestShape = {b->tileX, b->tileY};
       int bestPers = b->persistent;
       const int warm = std::min(trial_steps, 20);
+      // the block kernel first, then the one-step kernel's shapes (one of which serves single steps)
+      float blockMs = 1e30f;
+      b->choose_block();
+      if (b->blockOn) {
+        b->launch_blocks(warm, par0, 0);
+        check_cuda(cudaEventRecord(b->dev.ev0, b->dev.stream), "cudaEventRecord");
+        b->launch_blocks(trial_steps, par0 ^ (warm & 1), 0);
+        check_cuda(cudaEventRecord(b->dev.ev1, b->dev.stream), "cudaEventRecord");
+        check_cuda(cudaEventSynchronize(b->dev.ev1), "cudaEventSynchronize");
+        check_cuda(cudaEventElapsedTime(&blockMs, b->dev.ev0, b->dev.ev1), "cudaEventElapsedTime");
+      }
+      b->blockOn = false;
       for (const Shape2& sh : kShapes) {
         for (int pers = 0; pers <= 1; pers++) {
           b->set_layout(sh.tx, sh.ty, pers);
@@ -1264,10 +1487,12 @@ int cells2d_batch_autotune(Cells2DBatch* b, int32_t trial_steps, Cells2DInfo* in
           }
         }
       }
-      b->set_layout(bestShape.tx, bestShape.ty, bestPers);
+      b->blockWanted = b->blockOn = blockMs < best;
+      b->set_layout(bestShape.tx, bestShape.ty, b->blockOn ? 0 : bestPers);
       restore();
     } catch (...) {
       // a failed trial leaves the previous layout and the state before the call in place
+      b->blockOn = block0 && b->dLayout;
       try {
         b->set_layout(tx0, ty0, pers0);
         restore();

@@ -16,143 +16,10 @@
 //
 // This file is compiled twice: into cells::fast (contraction allowed) and, with
 // -fmad=false -DCELLS_EXACT_ARITH, into cells::exact.
-#include "kernels2d.h"
-
-#ifdef CELLS_EXACT_ARITH
-#define CELLS_NS exact
-constexpr bool kExact2 = true;
-#else
-#define CELLS_NS fast
-constexpr bool kExact2 = false;
-#endif
+#include "step2d.cuh"
 
 namespace cells {
 namespace CELLS_NS {
-
-// Storage type S, arithmetic type R, and how populations are loaded: through the read-only path
-// when a launch never writes what it reads (one step per launch), through L2 when it does (the
-// persistent kernel rewrites the buffer it read two steps earlier, which a stale read-only line
-// would miss).
-template <class S_, class R_, bool COHERENT>
-struct Store2 {
-  using S = S_;
-  using R = R_;
-  __device__ __forceinline__ static S ld(const S* p) { return COHERENT ? __ldcg(p) : __ldg(p); }
-};
-using Store2F32 = Store2<float, float, false>;
-using Store2F64 = Store2<double, double, false>;
-using Store2F32P = Store2<float, float, true>;
-using Store2F64P = Store2<double, double, true>;
-
-template <class R>
-__device__ __forceinline__ R prm(const Tunnel2& T, int k);
-template <>
-__device__ __forceinline__ float prm<float>(const Tunnel2& T, int k) {
-  return __ldg(&T.pf[k]);
-}
-template <>
-__device__ __forceinline__ double prm<double>(const Tunnel2& T, int k) {
-  return __ldg(&T.pd[k]);
-}
-
-template <class R>
-__device__ __forceinline__ R clampR(R v, R lo, R hi) {
-  return v < lo ? lo : (hi < v ? hi : v);
-}
-// 1 / v: IEEE in the exact build and for f64; the hardware reciprocal (within 2 ulp, no branch)
-// for f32 in the fast build
-template <class R>
-__device__ __forceinline__ R recip2(R v) {
-  if constexpr (!kExact2 && sizeof(R) == 4)
-    return __fdividef(R(1), v);
-  else
-    return R(1) / v;
-}
-template <class R>
-struct XTab2;
-template <>
-struct XTab2<float> {
-  using T = float4;
-};
-template <>
-struct XTab2<double> {
-  using T = double4;
-};
-
-struct Geo2 {
-  int W, H;
-  int left, right, bottom, top;
-};
-
-// wrapPeriodic, src/shaders/common.ts:48-57
-__device__ __forceinline__ void wrap2(const Geo2& g, int& x, int& y) {
-  if (x < 0 && g.left == X2_PERIODIC) x += g.W;
-  if (x >= g.W && g.right == X2_PERIODIC) x -= g.W;
-  if (y < 0 && g.bottom == Y2_PERIODIC) y += g.H;
-  if (y >= g.H && g.top == Y2_PERIODIC) y -= g.H;
-}
-
-// inletVelocity, src/shaders/common.ts:39-45
-template <class R>
-__device__ __forceinline__ R inlet_velocity2(int parabolic, R uIn, int H, int y) {
-  if (parabolic == 0) return uIn;
-  const R h = R(H);
-  const R s = R(y) + R(0.5);
-  return R(4) * uIn * s * (h - s) / (h * h);
-}
-
-// pullSlow, src/shaders/step.ts:119-175
-template <class C>
-__device__ __forceinline__ typename C::R pull_slow2(int i, const Geo2& g, const typename C::S* __restrict__ src,
-                                                    const uint32_t* __restrict__ flags, const float* __restrict__ sdf,
-                                                    long long N, int x, int y, long long idx, uint32_t fl,
-                                                    typename C::R uLid, typename C::R force[2]) {
-  using R = typename C::R;
-  const int j = opp2(i);
-  int sx = x - cx2(i);
-  int sy = y - cy2(i);
-  if ((fl & (1u << i)) == 0u) return (R)C::ld(&src[i * N + (long long)sy * g.W + sx]);
-  wrap2(g, sx, sy);
-  const bool inX = sx >= 0 && sx < g.W;
-  const bool inY = sy >= 0 && sy < g.H;
-  if (inX && inY) {
-    const long long s = (long long)sy * g.W + sx;
-    if ((__ldg(&flags[s]) & FLAG2_SOLID) == 0u) return (R)C::ld(&src[i * N + s]);
-    // Bouzidi linear interpolated bounce-back with q from the SDF
-    const R fj = (R)C::ld(&src[j * N + idx]);
-    const R dF = (R)__ldg(&sdf[idx]);
-    const R dS = (R)__ldg(&sdf[s]);
-    const R den = (dF - dS) < (R)1e-6 ? (R)1e-6 : (dF - dS);
-    const R q = clampR<R>(dF / den, (R)1e-3, R(1));
-    R fi = fj;
-    if (q < R(0.5)) {
-      int nx = x + cx2(i), ny = y + cy2(i);
-      wrap2(g, nx, ny);
-      if (nx >= 0 && nx < g.W && ny >= 0 && ny < g.H) {
-        const long long n = (long long)ny * g.W + nx;
-        if ((__ldg(&flags[n]) & FLAG2_SOLID) == 0u)
-          fi = R(2) * q * fj + (R(1) - R(2) * q) * (R)C::ld(&src[j * N + n]);
-      }
-    } else {
-      fi = fj / (R(2) * q) + (R(2) * q - R(1)) / (R(2) * q) * (R)C::ld(&src[i * N + idx]);
-    }
-    const R t = fj + fi;
-    force[0] += R(cx2(j)) * t;
-    force[1] += R(cy2(j)) * t;
-    return fi;
-  }
-  if (!inY) {
-    const int mode = sy < 0 ? g.bottom : g.top;
-    if (mode == Y2_SLIP) {
-      const int rx = sx < 0 ? 0 : (sx > g.W - 1 ? g.W - 1 : sx);
-      return (R)C::ld(&src[mirror_y2(i) * N + (long long)y * g.W + rx]);
-    }
-    if (mode == Y2_MOVING) return (R)C::ld(&src[j * N + idx]) + R(6) * w2<R>(i) * R(cx2(i)) * uLid;
-    return (R)C::ld(&src[j * N + idx]);
-  }
-  // walls, and placeholders that the open-boundary fix-up overwrites
-  return (R)C::ld(&src[j * N + idx]);
-}
 
 // The fields of a tunnel that every cell of a tile reads, loaded once per thread.
 template <class C>
@@ -180,154 +47,28 @@ __device__ __forceinline__ uint32_t load2(const Hot2<C>& h, int x, int y, typena
 }
 
 // main, src/shaders/step.ts:177-227, for the cell (x, y) of tunnel T, whose loads load2 made.
-// Returns whether the cell has a force slot (its force is then in force[0..1]). The x-dependent
-// rates come from the tunnel's x table; the exact build evaluates every other expression in the
-// reference's order.
+// Returns whether the cell has a force slot (its force is then in force[0..1]).
 template <class C>
 __device__ __forceinline__ bool cell2(const Tunnel2& T, const Hot2<C>& h, typename C::R uIn, int x, int y,
                                       uint32_t fl, typename C::R (&f)[Q2], typename C::R force[2]) {
   using R = typename C::R;
   using S = typename C::S;
-  const int W = h.W;
   const int N = h.N;  // 9 N < 2^31: checked when the tunnel is created
-  const S* __restrict__ src = h.src;
   S* __restrict__ dst = h.dst;
-  const int idx = y * W + x;
+  const int idx = y * h.W + x;
   bool slot = false;
   if (fl != 0u) {
     if (fl & FLAG2_SOLID) return false;
-    // pullSlow's first rule: a direction without its flag bit is the plain pull, which load2
-    // already made (same element), so the general rules run for the flagged directions only. An
-    // inlet (outlet) cell whose only flagged directions are the three entering from outside the
-    // grid skips them altogether: Zou-He replaces those three pulls.
-    constexpr uint32_t kInletPlain = FLAG2_INLET | (1u << 1) | (1u << 5) | (1u << 8);
-    constexpr uint32_t kOutletPlain = FLAG2_OUTLET | (1u << 3) | (1u << 6) | (1u << 7);
-    if (fl != kInletPlain && fl != kOutletPlain) {
-      Geo2 g;
-      g.W = W;
-      g.H = h.H;
-      g.left = T.left;
-      g.right = T.right;
-      g.bottom = T.bottom;
-      g.top = T.top;
-      const R uLid = prm<R>(T, P2_ULID);
-#pragma unroll
-      for (int i = 1; i < Q2; i++)
-        if (fl & (1u << i))
-          f[i] = pull_slow2<C>(i, g, src, h.flags, T.sdf, (long long)N, x, y, (long long)idx, fl, uLid, force);
-      slot = (fl >> BIDX2_SHIFT) != 0u;
-    }
-    // Zou-He (populations stored shifted by w_i)
-    if (fl & FLAG2_INLET) {
-      const R u = inlet_velocity2<R>(T.parabolic, uIn, h.H, y);
-      const R r = (R(1) + f[0] + f[2] + f[4] + R(2) * (f[3] + f[6] + f[7])) / (R(1) - u);
-      f[1] = f[3] + (R)(2.0 / 3.0) * r * u;
-      f[5] = f[7] - R(0.5) * (f[2] - f[4]) + (R)(1.0 / 6.0) * r * u;
-      f[8] = f[6] + R(0.5) * (f[2] - f[4]) + (R)(1.0 / 6.0) * r * u;
-    } else if (fl & FLAG2_OUTLET) {
-      const R u = f[0] + f[2] + f[4] + R(2) * (f[1] + f[5] + f[8]);
-      f[3] = f[1] - (R)(2.0 / 3.0) * u;
-      f[7] = f[5] + R(0.5) * (f[2] - f[4]) - (R)(1.0 / 6.0) * u;
-      f[6] = f[8] - R(0.5) * (f[2] - f[4]) - (R)(1.0 / 6.0) * u;
-    }
+    const Geo2 g{h.W, h.H, T.left, T.right, T.bottom, T.top};
+    const GridSource2<C> src{h.src, (long long)N, h.W};
+    slot = boundary2<C>(T, g, src, h.flags, uIn, x, y, (long long)idx, fl, f, force);
   }
-  // moments (src/shaders/step.ts:22-32)
-  const R drho = f[0] + f[1] + f[2] + f[3] + f[4] + f[5] + f[6] + f[7] + f[8];
-  const R rho = R(1) + drho;
-  const R invRho = recip2<R>(rho);
-  R ux = (f[1] - f[3] + f[5] - f[6] - f[7] + f[8]) * invRho;
-  R uy = (f[2] - f[4] + f[5] + f[6] - f[7] - f[8]) * invRho;
-  const int forcing = h.forcing;
-  R bfx = R(0), bfy = R(0);
-  if (forcing != 0) {
-    bfx = prm<R>(T, P2_FX);
-    bfy = prm<R>(T, P2_FY);
-    ux += R(0.5) * bfx * invRho;
-    uy += R(0.5) * bfy * invRho;
-  }
-  const R usq = R(1.5) * (ux * ux + uy * uy);
-  R cu[Q2];
-  cu[1] = R(3) * (ux);
-  cu[2] = R(3) * (uy);
-  cu[5] = R(3) * (ux + uy);
-  cu[6] = R(3) * (-ux + uy);
-  R eqS[Q2], eqA[Q2];
-#pragma unroll
-  for (int a : {1, 2, 5, 6}) {
-    eqS[a] = w2<R>(a) * (drho + rho * (R(0.5) * cu[a] * cu[a] - usq));
-    eqA[a] = w2<R>(a) * rho * cu[a];
-  }
-  // sponge and absorbing layers (src/shaders/step.ts:215-223), from the x table
+  R o[Q2];
   const auto xt = h.xtab[x];  // read-only for the whole launch
-  const R omegaBase = xt.x;
-  const R sigma = xt.z;
-  // Smagorinsky (src/shaders/step.ts:48-63)
-  R omP = omegaBase, omM = xt.y;
-  if (h.smagC2 > R(0)) {
-    R n[Q2];
+  collide2<C>(T, xt, h.forcing, h.smagC2, h.H, uIn, y, f, o);
 #pragma unroll
-    for (int a : {1, 2, 5, 6}) {
-      const int b = opp2(a);
-      n[a] = f[a] - (eqS[a] + eqA[a]);
-      n[b] = f[b] - (eqS[a] - eqA[a]);
-    }
-    const R pxx = n[1] + n[3] + n[5] + n[6] + n[7] + n[8];
-    const R pyy = n[2] + n[4] + n[5] + n[6] + n[7] + n[8];
-    const R pxy = n[5] - n[6] + n[7] - n[8];
-    const R pi = sqrt(pxx * pxx + pyy * pyy + R(2) * pxy * pxy);
-    const R t0 = xt.w;  // 1 / omegaBase
-    const R tEff = R(0.5) * (t0 + sqrt(t0 * t0 + (R)25.45584412271571 * h.smagC2 * pi * invRho));
-    omP = recip2<R>(tEff);
-    // the exact build divides 1 by omega+ again, as the reference does; the fast build uses tEff
-    const R tP = kExact2 ? R(1) / omP : tEff;
-    omM = recip2<R>(R(0.5) + prm<R>(T, P2_LAMBDA) / (tP - R(0.5)));
-  }
-  // absorbing-layer and Guo body-force sources (src/shaders/step.ts:65-91)
-  R s0 = R(0);
-  R sS[Q2], sA[Q2];
-#pragma unroll
-  for (int a : {1, 2, 5, 6}) {
-    sS[a] = R(0);
-    sA[a] = R(0);
-  }
-  if (sigma > R(0)) {
-    const R ut = inlet_velocity2<R>(T.parabolic, uIn, h.H, y);
-    const R dq = R(1.5) * rho * (ut * ut - ux * ux - uy * uy);
-    s0 += sigma * w2<R>(0) * -dq;
-#pragma unroll
-    for (int a : {1, 2, 5, 6}) {
-      const R cut = R(3) * R(cx2(a)) * ut;
-      sS[a] += sigma * w2<R>(a) * (R(0.5) * rho * (cut * cut - cu[a] * cu[a]) - dq);
-      sA[a] += sigma * w2<R>(a) * rho * (cut - cu[a]);
-    }
-  }
-  if (forcing != 0) {
-    const R uF = ux * bfx + uy * bfy;
-    s0 += (R(1) - R(0.5) * omP) * w2<R>(0) * (R(-3) * uF);
-#pragma unroll
-    for (int a : {1, 2, 5, 6}) {
-      const R cF = (R(cx2(a)) * bfx + R(cy2(a)) * bfy);
-      sS[a] += (R(1) - R(0.5) * omP) * w2<R>(a) * (R(-3) * uF + R(9) * (cu[a] / R(3)) * cF);
-      sA[a] += (R(1) - R(0.5) * omM) * w2<R>(a) * R(3) * cF;
-    }
-  }
-  // TRT collide + store (src/shaders/step.ts:93-103)
-  dst[idx] = (S)(f[0] - omP * (f[0] - w2<R>(0) * (drho - rho * usq)) + s0);
-#pragma unroll
-  for (int a : {1, 2, 5, 6}) {
-    const int b = opp2(a);
-    const R sym = omP * (R(0.5) * (f[a] + f[b]) - eqS[a]);
-    const R asym = omM * (R(0.5) * (f[a] - f[b]) - eqA[a]);
-    dst[a * N + idx] = (S)(f[a] - sym - asym + sS[a] + sA[a]);
-    dst[b * N + idx] = (S)(f[b] - sym + asym + sS[a] - sA[a]);
-  }
+  for (int i = 0; i < Q2; i++) dst[i * N + idx] = (S)o[i];
   return slot;
-}
-
-__device__ __forceinline__ double ramp_speed2(int kind, double target, double rampSteps, int every, unsigned step) {
-  const double sq = (double)((step / (unsigned)every) * (unsigned)every);
-  const double t = fmin(1.0, sq / rampSteps);
-  return kind == 1 ? target * t : target * (t * t * (3.0 - 2.0 * t));
 }
 
 // One tile (lb-th of its tunnel t) of the step of parity par.

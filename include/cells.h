@@ -313,8 +313,8 @@ int64_t cells_fake_live_buffers(void);
  * D2Q9: class Solver, src/solver.ts:50-340, and batches of independent 2D tunnels.
  *
  * A Cells2D handle is one tunnel. cells2d_create makes a batch of one and returns its tunnel;
- * cells2d_batch_create makes many tunnels of different sizes that advance together, one kernel
- * launch per step for all of them (or one persistent launch for many steps), and
+ * cells2d_batch_create makes many tunnels of different sizes that advance together, a kernel
+ * launch for up to seven steps of all of them, and
  * cells2d_batch_tunnel gives a handle to each for the per-tunnel calls (geometry, parameters,
  * readback). Stepping a tunnel of a batch of more than one is an error: step the batch.
  * Distributions are f[i*N + x + W*y], shifted by w_i (src/shaders/step.ts:7).
@@ -356,7 +356,7 @@ typedef struct {
   int32_t W, H, precision, force_every;
   int64_t N;
   int64_t step;
-  int32_t tile_x, tile_y;     /* block shape of the batch's step kernel */
+  int32_t tile_x, tile_y;     /* block shape of the batch's one-step kernel */
   int32_t persistent;         /* 1 when the batch steps with the persistent kernel */
   int32_t tunnels;            /* tunnels in the batch */
 } Cells2DInfo;
@@ -428,16 +428,17 @@ int cells2d_batch_create(const Cells2DConfig* cfgs, int32_t count, Cells2DBatch*
 void cells2d_batch_destroy(Cells2DBatch* b);
 /* A handle to tunnel k for the per-tunnel calls; valid until the batch is destroyed. */
 int cells2d_batch_tunnel(Cells2DBatch* b, int32_t k, Cells2D** out);
-/* n steps of every tunnel: one launch per step (replayed from CUDA graphs of 100 steps), or
- * persistent launches of many steps when the autotuner chose that. */
+/* n steps of every tunnel: up to seven steps per launch, or, after cells2d_batch_set_launch, with a
+ * workgroup_size, or when the autotuner found it faster, one launch per step (replayed from CUDA
+ * graphs of 100 steps) or persistent launches of many steps. */
 int cells2d_batch_step(Cells2DBatch* b, int64_t n);
 /* n steps, then every tunnel's macro refresh, then wait. */
 int cells2d_batch_run(Cells2DBatch* b, int64_t n);
 int cells2d_batch_synchronize(Cells2DBatch* b);
-/* Times trial_steps steps of each candidate launch shape (block shapes x per-step graphs or the
- * persistent kernel) on a copy of the current state, keeps the fastest, and restores the state:
- * populations, step counters, inlet speeds and force rings are as before the call. Writes the
- * chosen shape to *info when info is not NULL. */
+/* Times trial_steps steps of the multi-step launches and of each candidate shape of the one-step
+ * kernel (block shapes x per-step graphs or the persistent kernel) on a copy of the current state,
+ * keeps the fastest, and restores the state: populations, step counters, inlet speeds and force
+ * rings are as before the call. Writes the one-step kernel's shape to *info when info is not NULL. */
 int cells2d_batch_autotune(Cells2DBatch* b, int32_t trial_steps, Cells2DInfo* info);
 /* Fixes the launch shape by hand: tile_x * tile_y threads (64, 128 or 256, tile_x a multiple of 32),
  * persistent 0 or 1. A block covers tile_x x tile_y cells, or tile_x x 2 tile_y (two rows per
