@@ -1020,7 +1020,7 @@ constexpr int step_min_blocks(bool pair) {
 // middle so the pull's one-element x offset still names the stretch's own line. Every address is
 // the pull source of an interior cell, inside the source buffer. A hint only: it changes no
 // result. (One bulk prefetch per row instead measured 8-10% slower.)
-template <class C>
+template <class C, bool ALT>
 __device__ __forceinline__ void prefetch_tile_ahead(const StepArgs3<C>& a) {
   using S = typename C::S;
   constexpr int kLine = 128;
@@ -1028,7 +1028,7 @@ __device__ __forceinline__ void prefetch_tile_ahead(const StepArgs3<C>& a) {
   if (bz < a.roleZ || bz >= (int)gridDim.z) return;
   const int tid = threadIdx.x + blockDim.x * threadIdx.y;
   const int perDir = a.pfRowShift + a.pfShift;  // log2 of the stretches per population
-  const long long plane = (long long)a.H * (a.reverse ? a.D - 2 - (bz - a.roleZ) : 1 + bz - a.roleZ);
+  const long long plane = (long long)a.H * (ALT && a.reverse ? a.D - 2 - (bz - a.roleZ) : 1 + bz - a.roleZ);
   for (int t = tid; t < (Q3 << perDir); t += kStepThreads) {
     const int i = t >> perDir;
     const int r = (t >> a.pfShift) & ((1 << a.pfRowShift) - 1);
@@ -1040,7 +1040,10 @@ __device__ __forceinline__ void prefetch_tile_ahead(const StepArgs3<C>& a) {
   }
 }
 
-template <class C, bool SMAG, bool PAIR>
+// ALT: a.reverse may be set. f64 has kernels with and without it: what it changes in the interior code costs
+// grids that never reverse 3-4% (200x100x96 97.9 -> 102.5 us a step); the f32 kernel and the 16-bit x-pairs
+// lose nothing.
+template <class C, bool SMAG, bool PAIR, bool ALT>
 __global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR))
     step3d_kernel(const __grid_constant__ StepArgs3<C> a) {
   // Programmatic dependent launch: the next step's grid may be scheduled once every block of this
@@ -1050,7 +1053,7 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR))
   // returns at once.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  if (a.pfPlanes > 0) prefetch_tile_ahead<C>(a);
+  if (a.pfPlanes > 0) prefetch_tile_ahead<C, ALT>(a);
   // grid (tilesX, tilesY, roleZ + D - 2): the first roleZ slices of blocks hold the face and body
   // roles (dispatched first), the others the interior tiles, one z plane per slice
   if ((int)blockIdx.z < a.roleZ) {
@@ -1079,7 +1082,7 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR))
   // block-uniform choice of the code for tiles that overlap the absorbing layer or hold the outlet
   const int tx1 = (blockIdx.x + 1) * a.tileTX;  // end of the tile's x range
   const bool abs = tx1 > a.absorbX0, out = tx1 >= a.W;
-  const int tz = a.reverse ? gridDim.z - 1 - blockIdx.z : blockIdx.z - a.roleZ;
+  const int tz = ALT && a.reverse ? gridDim.z - 1 - blockIdx.z : blockIdx.z - a.roleZ;
   if constexpr (PAIR) {
     if (out)
       abs ? bulk_pair_role<C, SMAG, true, true>(a, tz) : bulk_pair_role<C, SMAG, false, true>(a, tz);
@@ -1171,12 +1174,18 @@ static cudaError_t launch_step3_t(const StepLaunch3& L, cudaStream_t s) {
   a.roleZ = (a.shellBlocks + a.bodyBlocks + a.faceBlocks + perSlice - 1) / perSlice;
   const dim3 grid(tilesX, tilesY, a.roleZ + zInterior);
   // Steps of odd parity take the planes from the far end: a step then starts where the one before it
-  // ended, on planes that are still in L2. B200, us per step forward -> alternating: f32 192x96x96
-  // 43.1 -> 41.4, 160x80x80 27.9 -> 25.8, 161x83x75 36.9 -> 35.5; f16 192x96x96 28.9 -> 27.6, 160x80x80
-  // 18.9 -> 17.7; f64 128x64x64 29.5 -> 27.7. A buffer of several times L2 gains nothing (f32
-  // 256x128x128, 319 MB: 100.6 -> 99.9), and f64 loses where the buffer no longer fits L2 (160x80x80,
-  // 156 MB: 50.2 -> 51.7; 192x96x96: 85.4 -> 87.4), so f64 stops at 100 MB and the others at 320 MB.
-  a.reverse = L.par && 19ull * (unsigned long long)L.N * sizeof(S) <= (sizeof(S) == 8 ? 100ull << 20 : 320ull << 20);
+  // ended, on planes that are still in L2 (126 MB). B200, us per step forward -> alternating:
+  //   f32   160x80x80 (78 MB a buffer) 27.9 -> 25.8, 192x96x96 (134 MB) 43.4 -> 41.6, 196x98x98 51.9 -> 50.5,
+  //         208x104x104 (171 MB) 56.7 -> 57.3; one cell per thread 201x101x95 (147 MB) 68.6 -> 65.9,
+  //         255x127x127 (313 MB) 133.6 -> 130.0
+  //   16    160x80x80 18.1 -> 17.6, 192x96x96 (67 MB) 28.9 -> 27.6, 224x112x112 (107 MB) 46.7 -> 47.1,
+  //         256x128x128 (159 MB) 61.0 -> 61.7; one cell per thread is bound by issue (fp16 255x127x127
+  //         121.5 -> 123.2)
+  //   f64   112x56x56 (53 MB) 23.5 -> 20.7, 128x64x64 (80 MB) 28.9 -> 27.9, 136x70x66 (96 MB) 34.6 -> 36.2
+  const unsigned long long altMax = sizeof(S) == 4 ? (pair ? 150ull << 20 : 320ull << 20)
+                                                   : (sizeof(S) == 8 || pair ? 84ull << 20 : 0ull);
+  const bool alternate = 19ull * (unsigned long long)L.N * sizeof(S) <= altMax;
+  a.reverse = L.par && alternate;
   // prefetch distance, measured on B200 at 192x96x96 and 256x128x128 (sphere tunnel, 1000 steps):
   // 16-bit storage 4 planes (+1.5-3% and +6.5-8%), f32 1 plane (+0.5-1.5%), f64 the plane count
   // nearest 270 tiles (+5% and +2%); farther prefetches lost to the demand loads
@@ -1194,9 +1203,11 @@ static cudaError_t launch_step3_t(const StepLaunch3& L, cudaStream_t s) {
   const bool smag = L.smagC2 > 0;
   void (*fn)(StepArgs3<C>) = nullptr;
   if (pair) {
-    if constexpr (sizeof(S) <= 4) fn = smag ? step3d_kernel<C, true, true> : step3d_kernel<C, false, true>;
+    if constexpr (sizeof(S) <= 4) fn = smag ? step3d_kernel<C, true, true, true> : step3d_kernel<C, false, true, true>;
+  } else if (sizeof(S) != 2 && (sizeof(S) == 4 || alternate)) {
+    if constexpr (sizeof(S) != 2) fn = smag ? step3d_kernel<C, true, false, true> : step3d_kernel<C, false, false, true>;
   } else {
-    fn = smag ? step3d_kernel<C, true, false> : step3d_kernel<C, false, false>;
+    if constexpr (sizeof(S) != 4) fn = smag ? step3d_kernel<C, true, false, false> : step3d_kernel<C, false, false, false>;
   }
   if (!fn) return cudaErrorInvalidValue;
   // launched with programmatic stream serialisation: consecutive steps on a stream (and in the
