@@ -95,7 +95,8 @@ void Cells3D::upload_xtab() {
     for (int x = W - 1; x >= 0; x--)
       if (t[4 * x + 2] > 0.0f) firstAbsorb = x;
     // the x-pair layout of the same values after the W per-x entries: entry x0 (even) holds
-    // (omega+ of x0, of x0 + 1, omega- of x0, of x0 + 1), entry x0 + 1 (sigma of x0, of x0 + 1, 0, 0)
+    // (omega+ of x0, of x0 + 1, omega- of x0, of x0 + 1), entry x0 + 1 (sigma of x0, of x0 + 1, 0, 0); with
+    // Smagorinsky omega- follows from the flow, and 1 / omega+ stands in its place
     t.resize(8 * (size_t)W, 0.0f);
     float* pairTab = t.data() + 4 * (size_t)W;
     for (int x0 = 0; x0 + 1 < W; x0 += 2) {
@@ -104,8 +105,8 @@ void Cells3D::upload_xtab() {
       float* e = pairTab + 4 * (size_t)x0;
       e[0] = c0[0];
       e[1] = c1[0];
-      e[2] = c0[1];
-      e[3] = c1[1];
+      e[2] = smag_on() ? 1.0f / c0[0] : c0[1];
+      e[3] = smag_on() ? 1.0f / c1[0] : c1[1];
       e[4] = c0[2];
       e[5] = c1[2];
     }
@@ -552,9 +553,12 @@ int cells3d_set_tau(Cells3D* h, double tau) {
 
 int cells3d_set_smagorinsky(Cells3D* h, double cs) {
   if (!h) return CELLS_E_INVALID;
+  CELLS_TRY(h)
+  const bool was = h->smag_on();
   h->cfg.smagorinsky = cs;
   h->argGen++;
-  return CELLS_OK;
+  if (h->smag_on() != was) h->upload_xtab();  // the x-pair table's second pair
+  CELLS_CATCH(h)
 }
 
 int cells3d_set_lambda(Cells3D* h, double lambda) {

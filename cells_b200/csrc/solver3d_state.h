@@ -121,6 +121,7 @@ struct Cells3D : cells::HandleBase {
   Cells3D();
   ~Cells3D();
   void choose_launch();
+  bool smag_on() const { return cfg.smagorinsky * cfg.smagorinsky > 0.0; }
   void upload_xtab();
   void rebuild_flags();
   void build_body_list();
