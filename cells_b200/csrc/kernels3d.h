@@ -48,7 +48,7 @@ struct StepLaunch3 {
   long long N;
   int W, H, D;
   int tileTX, tileTY;  // interior tile of the step kernel: tileTY rows of tileTX cells
-  int pairTiles;       // f32 / 16-bit storage with an even width: two cells per thread
+  int pairTiles;       // two cells per thread: f32 (exact build: even widths), 16-bit storage and an even width
   int absorbX0;        // first x of the absorbing layer (W when it is off): interior tiles before
                        // it compile without the absorbing sources
   int nBody;

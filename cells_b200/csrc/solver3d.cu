@@ -50,18 +50,19 @@ static void fill_xtab(std::vector<R>& t, int W, double tau, double lambda, doubl
     t[4 * x] = omegaBase;
     t[4 * x + 1] = R(1) / (R(0.5) + lamR / (R(1) / omegaBase - R(0.5)));
     t[4 * x + 2] = abR * sOut * sOut;
-    t[4 * x + 3] = R(0);
+    t[4 * x + 3] = R(1) / omegaBase;
   }
 }
 
-// Interior tile of the step kernel (128 threads per block): 128 cells, or 256 cells as x-pairs for
-// f32, f16 or bf16 storage with an even width (f64 and odd widths take one cell per thread). The
+// Interior tile of the step kernel (128 threads per block): 128 cells, or 256 cells two per thread for
+// f32, f16 or bf16 storage with an even width and for f32 in fast arithmetic with an odd one (f64 and
+// the other odd widths take one cell per thread). The
 // tile width is workgroup_size when given (the autotuner's knob), else the candidate that wastes
 // the fewest threads at the end of a row: the widest for one cell per thread, the narrowest (64
 // cells, 32 pairs x 4 rows) for pairs, so that more tiles fall wholly outside the absorbing layer
 // and the outlet column.
 void Cells3D::choose_launch() {
-  pairTiles = (bpp <= 4 && (W % 2) == 0) ? 1 : 0;
+  pairTiles = (bpp <= 4 && (W % 2 == 0 || (bpp == 4 && cfg.arithmetic != CELLS_ARITH_EXACT))) ? 1 : 0;
   const int cells = pairTiles ? 256 : 128;
   const int lo = pairTiles ? 64 : 32;
   int best = -1;

@@ -395,6 +395,8 @@ __device__ __noinline__ float2 smag_rates(float q, float ir, float t, float smag
   return make_float2(o, 1.0f / (0.5f + lambda / (1.0f / o - 0.5f)));
 }
 
+constexpr int kFarPair = 32;  // distance of the two cells of a thread at odd widths (f32)
+
 // The fast TRT collision of the two cells of an x-pair (cell x0 in .x, x0 + 1 in .y) with packed
 // f32x2 instructions, stored as one 32-bit word per population. It evaluates the lean pair form of
 // collide3 per component in f32: with s_p = f_p + f_p+1 and d_p = f_p - f_p+1 (exact for values
@@ -407,9 +409,21 @@ __device__ __noinline__ float2 smag_rates(float q, float ir, float t, float smag
 // same instructions: with omega+ = omega- = 1, rho = 1, drho = 0 and no absorbing source the update
 // is exactly the equilibrium feq(1, u), at u = (uIn, 0, 0) for the inlet (step3d.ts:190-193) and at
 // the node's own velocity for the outlet.
-template <class C, bool SMAG, bool ABS, bool IN, bool OUT>
+// DX: the distance of the two cells. 1: an x-pair, both stored as one word; kFarPair: cells of their own,
+// each stored when act0 / act1 is set (the other's values are computed and dropped).
+template <class C, int DX>
+__device__ __forceinline__ void store2(typename C::S* p, float2 v, bool act0, bool act1) {
+  if constexpr (DX == 1) {
+    C::st_pair_fast(p, v.x, v.y);
+  } else {
+    if (act0) p[0] = C::enc_raw(v.x);
+    if (act1) p[DX] = C::enc_raw(v.y);
+  }
+}
+
+template <class C, bool SMAG, bool ABS, bool IN, bool OUT, int DX>
 __device__ __forceinline__ void collide3x2_store(const StepArgs3<C>& a, const typename C::Pair (&r)[Q3], int x0,
-                                                 int idx) {
+                                                 int idx, bool act0, bool act1) {
   constexpr float IS = 1.0f / C::SCALE;
   float2 sp[Q3], dp[Q3];  // entries p = 1, 3, .., 17
   const float2 f0 = make_float2(C::lo(r[0]), C::hi(r[0]));
@@ -429,7 +443,8 @@ __device__ __forceinline__ void collide3x2_store(const StepArgs3<C>& a, const ty
   float2 ux = mul2(add2(add2(add2(dp[1], dp[7]), add2(dp[9], dp[13])), dp[15]), invRhoS);
   float2 uy = mul2(add2(add2(add2(dp[3], dp[7]), sub2(dp[11], dp[13])), dp[17]), invRhoS);
   float2 uz = mul2(sub2(add2(add2(dp[5], dp[9]), sub2(dp[11], dp[15])), dp[17]), invRhoS);
-  const bool inlet = IN && x0 == 0, outlet = OUT && x0 + 1 == a.W - 1;
+  const bool inlet = IN && x0 == 0, outlet = OUT && x0 + DX == a.W - 1;
+  const bool outlet0 = DX != 1 && OUT && x0 == a.W - 1;
   if (inlet) {
     ux.x = (float)a.st->uIn[a.par];
     uy.x = 0.0f;
@@ -438,8 +453,17 @@ __device__ __forceinline__ void collide3x2_store(const StepArgs3<C>& a, const ty
   const float2 u2 = fma2(uz, uz, fma2(uy, uy, mul2(ux, ux)));
   const float2 nusq = mul2(bc2(-1.5f), u2);  // -3u^2/2
   const float2 u3[3] = {mul2(bc2(3.0f), ux), mul2(bc2(3.0f), uy), mul2(bc2(3.0f), uz)};
-  const float4 t0 = a.xPair[x0];
-  float2 omP = make_float2(t0.x, t0.y), omM = make_float2(t0.z, t0.w);
+  float2 omP, omM, sigma = bc2(0.0f);
+  if constexpr (DX == 1) {
+    const float4 t0 = a.xPair[x0];
+    omP = make_float2(t0.x, t0.y);
+    omM = make_float2(t0.z, t0.w);
+  } else {
+    const float4 t0 = a.xTab[x0], t1 = a.xTab[min(x0 + DX, a.W - 1)];
+    omP = make_float2(t0.x, t1.x);
+    omM = SMAG ? make_float2(t0.w, t1.w) : make_float2(t0.y, t1.y);
+    if (ABS) sigma = make_float2(t0.z, t1.z);
+  }
   if (SMAG) {
     // second moments of the non-equilibrium part, per pair: n_p + n_p+1 = s_p - 2 w (rho cu^2/2 + K0)
     const float2 K0s = fma2(rho, nusq, drho);
@@ -489,13 +513,18 @@ __device__ __forceinline__ void collide3x2_store(const StepArgs3<C>& a, const ty
       omM = make_float2(r0.y, r1.y);
     }
   }
-  float2 sigma = bc2(0.0f);
-  if (ABS) {
+  if (ABS && DX == 1) {
     const float4 t1 = a.xPair[x0 + 1];
     sigma = make_float2(t1.x, t1.y);
   }
   // the boundary cells relax fully to feq(1, u)
   if (inlet) {
+    omP.x = omM.x = 1.0f;
+    rho.x = 1.0f;
+    drho.x = 0.0f;
+    sigma.x = 0.0f;
+  }
+  if (outlet0) {
     omP.x = omM.x = 1.0f;
     rho.x = 1.0f;
     drho.x = 0.0f;
@@ -526,7 +555,7 @@ __device__ __forceinline__ void collide3x2_store(const StepArgs3<C>& a, const ty
     // rest population: (1 - omega+) f0 + omega+ w0 K0
     float2 v0 = fma2(add2(aP, aP), f0, mul2(omP, mul2(bc2(ws3<C>(0)), K0)));
     if (absorb) v0 = fma2(mul2(sigma, bc2(ws3<C>(0))), ndq, v0);
-    C::st_pair_fast(a.out[0] + idx, v0.x, v0.y);
+    store2<C, DX>(a.out[0] + idx, v0, act0, act1);
   }
 #pragma unroll
   for (int p = 1; p < Q3; p += 2) {
@@ -542,8 +571,8 @@ __device__ __forceinline__ void collide3x2_store(const StepArgs3<C>& a, const ty
       T = fma2(mul2(sr, bc2(ws3<C>(p))), sub2(cut, cu), T);
     }
     const float2 oa = add2(S, T), ob = sub2(S, T);
-    C::st_pair_fast(a.out[p] + idx, oa.x, oa.y);
-    C::st_pair_fast(a.out[p + 1] + idx, ob.x, ob.y);
+    store2<C, DX>(a.out[p] + idx, oa, act0, act1);
+    store2<C, DX>(a.out[p + 1] + idx, ob, act0, act1);
   }
 }
 
@@ -948,7 +977,7 @@ __device__ __forceinline__ void pair_cells(const StepArgs3<C>& a, int x0, int y,
     // takes the per-cell code below
     if (act0 && act1) {
       // the inlet and outlet tests run per thread (one variant per ABS instead of four)
-      collide3x2_store<C, SMAG, ABS, true, true>(a, r, x0, idx);
+      collide3x2_store<C, SMAG, ABS, true, true, 1>(a, r, x0, idx, true, true);
       return;
     }
   }
@@ -986,19 +1015,70 @@ __device__ __forceinline__ void pair_cells(const StepArgs3<C>& a, int x0, int y,
   }
 }
 
+// f32 and an odd width: each thread updates the cells x0 and x0 + 32 of a row. An x-pair's words would be
+// misaligned in every other row and population; like this every load and store of a warp is one run of
+// 128 bytes, and both cells still share the packed collision. The second cell may lie beyond the row.
+// us per step, one cell per thread -> two: 33x32x32 6.6 -> 6.2, 97x49x51 9.8 -> 8.1, 161x83x75 30.8 -> 27.4
+// (with Smagorinsky 34.8 -> 28.5), 201x99x91 60.9 -> 52.8, 255x127x127 122.4 -> 110.1. The exact build keeps
+// one cell per thread, and 16-bit storage does because its results may not move by a rounding: stored at
+// 11 bits, one grows to 1e-4 of a velocity within some hundred steps.
+template <class C, bool SMAG, bool ABS, bool OUT, bool FACE>
+__device__ __forceinline__ void far_pair_cells(const StepArgs3<C>& a, int x0, int y, int z, int side) {
+  const int W = a.W;
+  const int row = y + a.H * z;
+  const int idx = x0 + W * row;
+  const bool out0 = OUT && x0 == W - 1, out1 = OUT && x0 + kFarPair == W - 1;
+  bool act0 = true, act1 = x0 + kFarPair < W;
+  const int d1 = act1 ? kFarPair : 0;
+  typename C::Pair r[Q3];
+#pragma unroll
+  for (int i = 0; i < Q3; i++) {
+    const typename C::S* p = (FACE ? a.fpull[side][i] : a.pull[i]) + idx;
+    int e0 = 0, e1 = d1;
+    // outlet: zero-gradient copy from (W-2, y, z) for the directions entering through x = W-1
+    if (cx3(i) == -1 && (out0 || out1)) {
+      const int o = FACE ? a.fout[side][i] - 1 : (int)(-2 + cy3(i) * (long long)W + cz3(i) * ((long long)W * a.H));
+      if (out0) e0 = o;
+      if (out1) e1 = kFarPair + o;
+    }
+    r[i] = C::ld_pair2(p + e0, p + e1);
+  }
+  if (a.rowBody[row]) {
+    act0 = __ldg(a.flags + idx) == 0u;
+    act1 = act1 && __ldg(a.flags + idx + d1) == 0u;
+    if (!act0 && !act1) return;
+  }
+  collide3x2_store<C, SMAG, ABS, true, true, kFarPair>(a, r, x0, idx, act0, act1);
+}
+
+template <class C, bool SMAG, bool ABS, bool OUT, bool FACE, int DX>
+__device__ __forceinline__ void two_cells(const StepArgs3<C>& a, int x0, int y, int z, int side) {
+  if constexpr (DX == 1)
+    pair_cells<C, SMAG, ABS, OUT, FACE>(a, x0, y, z, side);
+  else
+    far_pair_cells<C, SMAG, ABS, OUT, FACE>(a, x0, y, z, side);
+}
+
+// The first cell of this thread's two in a tile row that begins at x = t0.
+template <int DX>
+__device__ __forceinline__ int first_cell(int t0) {
+  const int t = threadIdx.x;
+  return t0 + (DX == 1 ? 2 * t : (t & 31) + 2 * (t & ~31));
+}
+
 // The interior pairs of tile (blockIdx.x, blockIdx.y) in plane z = 1 + tz.
-template <class C, bool SMAG, bool ABS, bool OUT>
+template <class C, bool SMAG, bool ABS, bool OUT, int DX>
 __device__ __forceinline__ void bulk_pair_role(const StepArgs3<C>& a, int tz) {
-  const int x0 = blockIdx.x * a.tileTX + 2 * threadIdx.x;
+  const int x0 = first_cell<DX>(blockIdx.x * a.tileTX);
   const int y = 1 + blockIdx.y * a.tileTY + threadIdx.y;
   if (x0 >= a.W || y >= a.H - 1) return;
-  pair_cells<C, SMAG, ABS, OUT, false>(a, x0, y, 1 + tz, 0);
+  two_cells<C, SMAG, ABS, OUT, false, DX>(a, x0, y, 1 + tz, 0);
 }
 
 // Face tile f: the first faceZTiles are the tiles of the z = 0 and z = D-1 planes (rows 1 .. H-2,
 // laid out as an interior plane), the others tileTY consecutive planes of the y = 0 / y = H-1 row.
 // The absorbing layer and the outlet column are decided per thread.
-template <class C, bool SMAG>
+template <class C, bool SMAG, int DX>
 __device__ __forceinline__ void face_pair_role(const StepArgs3<C>& a, int f) {
   const int tilesX = (a.W + a.tileTX - 1) / a.tileTX;
   int side, tx, y, z;
@@ -1022,15 +1102,15 @@ __device__ __forceinline__ void face_pair_role(const StepArgs3<C>& a, int f) {
     z = 1 + g * a.tileTY + threadIdx.y;
     if (z >= a.D - 1) return;
   }
-  const int x0 = tx * a.tileTX + 2 * threadIdx.x;
+  const int x0 = first_cell<DX>(tx * a.tileTX);
   if (x0 >= a.W) return;
-  pair_cells<C, SMAG, true, true, true>(a, x0, y, z, side);
+  two_cells<C, SMAG, true, true, true, DX>(a, x0, y, z, side);
 }
 
 // Resident blocks per SM the register allocation must allow: 16-bit x-pairs 6 (80 registers;
 // measured faster at 6 than at 7, 5 or 4), f32 x-pairs 5 (up to 102 registers, no spills; with
 // the L2 prefetch 3.5% faster at 192x96x96 than at 6, where 68 bytes spilled), 8 for one f32 cell
-// per thread (odd widths), 4 for f64.
+// per thread (the exact build's odd widths), 4 for f64.
 template <class C>
 constexpr int step_min_blocks(bool pair) {
   return pair ? (sizeof(typename C::S) == 4 ? 5 : 6) : (sizeof(typename C::R) == 8 ? 4 : 8);
@@ -1065,8 +1145,8 @@ __device__ __forceinline__ void prefetch_tile_ahead(const StepArgs3<C>& a) {
 // ALT: a.reverse may be set. f64 has kernels with and without it: what it changes in the interior code costs
 // grids that never reverse 3-4% (200x100x96 97.9 -> 102.5 us a step); the f32 kernel and the 16-bit x-pairs
 // lose nothing.
-template <class C, bool SMAG, bool PAIR, bool ALT>
-__global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR))
+template <class C, bool SMAG, int PAIR, bool ALT>
+__global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR != 0))
     step3d_kernel(const __grid_constant__ StepArgs3<C> a) {
   // Programmatic dependent launch: the next step's grid may be scheduled once every block of this
   // one has started, so its blocks fill the SMs this grid's tail leaves idle; each of them waits
@@ -1096,8 +1176,8 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR))
       shell_role<C, SMAG>(a, r, tid);
     else if (r < a.shellBlocks + a.bodyBlocks)
       body_role<C, SMAG>(a, r - a.shellBlocks, tid);
-    else if constexpr (PAIR) {
-      if (r < a.shellBlocks + a.bodyBlocks + a.faceBlocks) face_pair_role<C, SMAG>(a, r - a.shellBlocks - a.bodyBlocks);
+    else if constexpr (PAIR != 0) {
+      if (r < a.shellBlocks + a.bodyBlocks + a.faceBlocks) face_pair_role<C, SMAG, PAIR>(a, r - a.shellBlocks - a.bodyBlocks);
     }
     return;
   }
@@ -1105,11 +1185,11 @@ __global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR))
   const int tx1 = (blockIdx.x + 1) * a.tileTX;  // end of the tile's x range
   const bool abs = tx1 > a.absorbX0, out = tx1 >= a.W;
   const int tz = ALT && a.reverse ? gridDim.z - 1 - blockIdx.z : blockIdx.z - a.roleZ;
-  if constexpr (PAIR) {
+  if constexpr (PAIR != 0) {
     if (out)
-      abs ? bulk_pair_role<C, SMAG, true, true>(a, tz) : bulk_pair_role<C, SMAG, false, true>(a, tz);
+      abs ? bulk_pair_role<C, SMAG, true, true, PAIR>(a, tz) : bulk_pair_role<C, SMAG, false, true, PAIR>(a, tz);
     else
-      abs ? bulk_pair_role<C, SMAG, true, false>(a, tz) : bulk_pair_role<C, SMAG, false, false>(a, tz);
+      abs ? bulk_pair_role<C, SMAG, true, false, PAIR>(a, tz) : bulk_pair_role<C, SMAG, false, false, PAIR>(a, tz);
   } else {
     if (out)
       abs ? bulk_role<C, SMAG, true, true>(a, tz) : bulk_role<C, SMAG, false, true>(a, tz);
@@ -1159,7 +1239,7 @@ static cudaError_t launch_step3_t(const StepLaunch3& L, cudaStream_t s) {
   a.smagC2 = (R)L.smagC2;
   a.absorbX0 = L.absorbX0;
   // work split
-  const bool pair = sizeof(S) <= 4 && (L.W % 2) == 0 && L.tileTX >= 64 && L.pairTiles;
+  const bool pair = sizeof(S) <= 4 && (L.W % 2 == 0 || (sizeof(S) == 4 && !kExact)) && L.tileTX >= 64 && L.pairTiles;
   if (!pair && L.tileTX > kStepThreads) return cudaErrorInvalidValue;
   a.tileTX = L.tileTX;
   a.tileTY = L.tileTY;
@@ -1198,13 +1278,12 @@ static cudaError_t launch_step3_t(const StepLaunch3& L, cudaStream_t s) {
   // Steps of odd parity take the planes from the far end: a step then starts where the one before it
   // ended, on planes that are still in L2 (126 MB). B200, us per step forward -> alternating:
   //   f32   160x80x80 (78 MB a buffer) 27.9 -> 25.8, 192x96x96 (134 MB) 43.4 -> 41.6, 196x98x98 51.9 -> 50.5,
-  //         208x104x104 (171 MB) 56.7 -> 57.3; one cell per thread 201x101x95 (147 MB) 68.6 -> 65.9,
-  //         255x127x127 (313 MB) 133.6 -> 130.0
+  //         208x104x104 (171 MB) 56.7 -> 57.3
   //   16    160x80x80 18.1 -> 17.6, 192x96x96 (67 MB) 28.9 -> 27.6, 224x112x112 (107 MB) 46.7 -> 47.1,
   //         256x128x128 (159 MB) 61.0 -> 61.7; one cell per thread is bound by issue (fp16 255x127x127
   //         121.5 -> 123.2)
   //   f64   112x56x56 (53 MB) 23.5 -> 20.7, 128x64x64 (80 MB) 28.9 -> 27.9, 136x70x66 (96 MB) 34.6 -> 36.2
-  const unsigned long long altMax = sizeof(S) == 4 ? (pair ? 150ull << 20 : 320ull << 20)
+  const unsigned long long altMax = sizeof(S) == 4 ? 150ull << 20
                                                    : (sizeof(S) == 8 || pair ? 84ull << 20 : 0ull);
   const bool alternate = 19ull * (unsigned long long)L.N * sizeof(S) <= altMax;
   a.reverse = L.par && alternate;
@@ -1225,11 +1304,13 @@ static cudaError_t launch_step3_t(const StepLaunch3& L, cudaStream_t s) {
   const bool smag = L.smagC2 > 0;
   void (*fn)(StepArgs3<C>) = nullptr;
   if (pair) {
-    if constexpr (sizeof(S) <= 4) fn = smag ? step3d_kernel<C, true, true, true> : step3d_kernel<C, false, true, true>;
+    if constexpr (sizeof(S) <= 4) fn = smag ? step3d_kernel<C, true, 1, true> : step3d_kernel<C, false, 1, true>;
+    if constexpr (sizeof(S) == 4 && !kExact)
+      if (L.W % 2) fn = smag ? step3d_kernel<C, true, kFarPair, true> : step3d_kernel<C, false, kFarPair, true>;
   } else if (sizeof(S) != 2 && (sizeof(S) == 4 || alternate)) {
-    if constexpr (sizeof(S) != 2) fn = smag ? step3d_kernel<C, true, false, true> : step3d_kernel<C, false, false, true>;
+    if constexpr (sizeof(S) != 2) fn = smag ? step3d_kernel<C, true, 0, true> : step3d_kernel<C, false, 0, true>;
   } else {
-    if constexpr (sizeof(S) != 4) fn = smag ? step3d_kernel<C, true, false, false> : step3d_kernel<C, false, false, false>;
+    if constexpr (sizeof(S) != 4) fn = smag ? step3d_kernel<C, true, 0, false> : step3d_kernel<C, false, 0, false>;
   }
   if (!fn) return cudaErrorInvalidValue;
   // launched with programmatic stream serialisation: consecutive steps on a stream (and in the
