@@ -11,9 +11,15 @@
 // cylinder 5.0 us a step with them. The arithmetic is the one-step kernel's (step2d.cuh); k is odd, so
 // a launch ends in the other population buffer as a single step does.
 //
-// Force: a tile's owned cells sum in f64 per sampled step (warp shuffles, then the warps in order) into
-// one partial per step and tile; after the launches of a run sum_samples2_kernel adds the tiles up in
-// order into the ring.
+// Where every tile is resident at once, a step waits for the tile with the most boundary: with the rules
+// inside each cell's code a step of 128x128 cells took 1.1 us without boundaries and 2.7 with a cylinder. There
+// (LIST) a block first collects its flagged directions into a list of links; a step works the list off, one
+// link per thread, into the places that the pulls read, and then every cell takes the same plain path: 2.05
+// us, and 400x100 2.8 -> 2.4. With more tiles than SMs the work counts, and the rules stay with the cells.
+//
+// Force: a tile's owned cells, each summed link by link, sum in f64 per sampled step (warp shuffles, then
+// the warps in order) into one partial per step and tile; after the launches of a run sum_samples2_kernel
+// adds the tiles up in order into the ring.
 #include <algorithm>
 
 #include "step2d.cuh"
@@ -78,6 +84,100 @@ __device__ __forceinline__ void rules2(uint32_t w, const Tunnel2& T, const Sourc
   }
 }
 
+// A flagged direction of a tile's cell, collected when the block starts: offsets in the tile's buffer of f_j
+// (a, low 15 bits), of the place that the pull reads, population i of x - c_i, solid or outside (a, next 15
+// bits), and of the rule's second source (b, low 15 bits); the rule (b, bits 15-17); c_j + 1 in x and y (b, bits
+// 18-19 and 20-21); on the first link of a cell whose force counts in this tile, the number of the cell's
+// links (b, bits 22-25); and the Bouzidi coefficients, or the moving wall's term in c1.
+template <class R>
+struct __align__(16) Link2 {
+  uint32_t a, b;
+  R c1, c2;
+};
+
+// Links per tile: what 64 x 48 cells of f32 leave of shared memory, or a tile's walls and a body of its size.
+template <int RX, int RY>
+constexpr int kTileLinks2 = RX * RY >= 3072 ? 352 : 512;
+
+// The links of the cell at offset c with rule word w, the first of which is number pos.
+template <class R, int RX, int RY>
+__device__ __forceinline__ void write_links2(Link2<R>* links, int pos, uint32_t w, int c, uint32_t head, R ulid,
+                                             const typename Vec2T<R>::T* __restrict__ coef) {
+  constexpr int cells = RX * RY;
+#pragma unroll
+  for (int i = 1; i < Q2; i++) {
+    const uint32_t rule = (w >> (3 * (i - 1))) & 7u;
+    if (rule == RULE2_PULL) continue;
+    const int j = opp2(i);
+    int g = j * cells + c;
+    if (rule == RULE2_SLIP) g = mirror_y2(i) * cells + c - cx2(i);
+    if (rule == RULE2_SLIP_HERE) g = mirror_y2(i) * cells + c;
+    if (rule == RULE2_BODY_N) g = j * cells + c + cy2(i) * RX + cx2(i);
+    if (rule == RULE2_BODY_H) g = i * cells + c;
+    Link2<R> L;
+    L.a = (uint32_t)(j * cells + c) | (uint32_t)(i * cells + c - cy2(i) * RX - cx2(i)) << 15;
+    L.b = (uint32_t)g | rule << 15 | (uint32_t)(cx2(j) + 1) << 18 | (uint32_t)(cy2(j) + 1) << 20;
+    L.c1 = R(6) * w2<R>(i) * R(cx2(i)) * ulid;
+    L.c2 = R(0);
+    if (rule == RULE2_BODY_N || rule == RULE2_BODY_H) {
+      L.c1 = coef[i - 1].x;
+      L.c2 = coef[i - 1].y;
+    }
+    L.b |= head << 22;
+    head = 0u;
+    links[pos++] = L;
+  }
+}
+
+// One link of a step: the pulled value goes where the pull reads it -- the cell is that place's only reader;
+// a slip row that mirrors a solid's population reads one that points out of the grid, which no link writes --
+// and the momentum exchange f_j + f_i is returned.
+template <class S, class R>
+__device__ __forceinline__ R link2(const Link2<R>& L, S* cur) {
+  const uint32_t rule = (L.b >> 15) & 7u;
+  if (rule == RULE2_PULL) return R(0);
+  const R fj = (R)cur[L.a & 0x7fffu], g = (R)cur[L.b & 0x7fffu];
+  R v = fj;
+  if (rule == RULE2_SLIP || rule == RULE2_SLIP_HERE) v = g;
+  if (rule == RULE2_MOVING) v = fj + L.c1;
+  if (rule == RULE2_BODY_N) v = L.c1 * fj + L.c2 * g;
+  if (rule == RULE2_BODY_H) v = fj / L.c1 + L.c2 * g;
+  cur[L.a >> 15] = (S)v;
+  return fj + v;
+}
+
+// The force on the cell whose links begin with number l, in their order.
+template <class R>
+__device__ __forceinline__ void cell_force2(const Link2<R>* links, const R* linkT, int l, R& fx, R& fy) {
+  const int count = (int)((links[l].b >> 22) & 0xfu);
+  fx = fy = R(0);
+  if (count == 0) return;
+  uint32_t b[Q2 - 1];
+  R t[Q2 - 1];
+#pragma unroll
+  for (int q = 0; q < Q2 - 1; q++) {
+    const int e = q < count ? l + q : l;
+    b[q] = links[e].b;
+    t[q] = linkT[e];
+  }
+#pragma unroll
+  for (int q = 0; q < Q2 - 1; q++) {
+    if (q >= count || ((b[q] >> 15) & 7u) < RULE2_BODY_N) continue;
+    fx += R((int)((b[q] >> 18) & 3u) - 1) * t[q];
+    fy += R((int)((b[q] >> 20) & 3u) - 1) * t[q];
+  }
+}
+
+// The warp's sum of (x, y): x in the even lanes, y in the odd ones.
+__device__ __forceinline__ double warp_sum2(double x, double y, int lane) {
+  const double send = (lane & 1) ? x : y;
+  double keep = (lane & 1) ? y : x;
+  keep += __shfl_xor_sync(0xffffffffu, send, 1);
+#pragma unroll
+  for (int o = 2; o < 32; o <<= 1) keep += __shfl_xor_sync(0xffffffffu, keep, o);
+  return keep;
+}
+
 // A coordinate v in [-k, n - 1 + k] of the margin's frame as one of the grid, or -1 outside it.
 __device__ __forceinline__ int real_coord2(int v, int n, bool wrapLow, bool wrapHigh) {
   if (v < 0) return wrapLow ? v + n : -1;
@@ -86,7 +186,7 @@ __device__ __forceinline__ int real_coord2(int v, int n, bool wrapLow, bool wrap
 }
 
 // Region RX x RY cells, ROWS rows per thread; tiles of (RX - 2 K) x (RY - 2 K) cells.
-template <class C, int RX, int RY, int ROWS>
+template <class C, int RX, int RY, int ROWS, bool LIST>
 __global__ void __launch_bounds__(RX * RY / ROWS, 1)
     block2d_kernel(const Tunnel2* __restrict__ tunnels, const Block2Tunnel* __restrict__ layout,
                    const unsigned short* __restrict__ tileTunnel, int K, int k, int par, double2* __restrict__ partials,
@@ -96,7 +196,8 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
   extern __shared__ __align__(16) unsigned char smemRaw[];
   __shared__ double sU[kBlockSteps2];
   __shared__ unsigned sStep;
-  __shared__ double2 sWarp[kBlockSteps2][32];
+  __shared__ double sWarp[kBlockSteps2][32][2];
+  __shared__ int sLinkCount[32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int b = blockIdx.x;
   const int t = __ldg(&tileTunnel[b]);
@@ -134,6 +235,51 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
   const Geo2 g{W, H, T.left, T.right, T.bottom, T.top};
   const int forcing = T.forcing, every = partials ? T.forceEvery : 0;
   const R smagC2 = prm<R>(T, P2_SMAGC2), lambda = prm<R>(T, P2_LAMBDA);
+  const int parabolic = T.parabolic;
+  // The tile's links, cell by cell and direction by direction, in a fixed order: a scan over the block's
+  // counts. A listed cell drops its rules; where the list is full they stay with the cell (rules2).
+  constexpr int LINKS = kTileLinks2<RX, RY>, WARPS = RX * BY / 32;
+  Link2<R>* const links = (Link2<R>*)(smemRaw + 2 * Q2 * cells * sizeof(S));
+  R* const linkT = (R*)(links + LINKS);  // each link's momentum exchange in the current step
+  int nLinks = 0;
+  if constexpr (LIST) {
+    int mine[ROWS], sum = 0;
+#pragma unroll
+    for (int m = 0; m < ROWS; m++) {
+      const uint32_t w = fl[m] & CODE2_RULES;
+      // only of cells that a step computes: their neighbours are places in the tile
+      const int r = threadIdx.y + m * BY;
+      const bool steps = (int)threadIdx.x > cut && (int)threadIdx.x < RX - 1 - cut && r > cut && r < RY - 1 - cut;
+      mine[m] = !steps || (fl[m] & CODE2_SOLID) ? 0 : __popc((w | w >> 1 | w >> 2) & 0x249249u);
+      sum += mine[m];
+    }
+    int incl = sum;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const int v = __shfl_up_sync(0xffffffffu, incl, o);
+      if ((tid & 31) >= o) incl += v;
+    }
+    if ((tid & 31) == 31) sLinkCount[tid >> 5] = incl;
+    __syncthreads();
+    const int n = (tid & 31) < WARPS ? sLinkCount[tid & 31] : 0;
+    int pos = __reduce_add_sync(0xffffffffu, (tid & 31) < (tid >> 5) ? n : 0) + incl - sum;
+    nLinks = min(__reduce_add_sync(0xffffffffu, n), LINKS);
+#pragma unroll
+    for (int m = 0; m < ROWS; m++) {
+      if (mine[m] == 0) continue;
+      if (pos + mine[m] <= LINKS) {
+        const auto* coef = (const typename Vec2T<R>::T*)T.qCoef;
+        if (fl[m] & CODE2_SLOT) coef += ((size_t)(__ldg(&flags[ry[m] * W + rx]) >> BIDX2_SHIFT) - 1) * 8;
+        const int r = threadIdx.y + m * BY;
+        const bool counts = (fl[m] & CODE2_SLOT) && colOwn && r >= K && r < RY - K && oy + r < H;
+        write_links2<R, RX, RY>(links, pos, fl[m], r * RX + threadIdx.x, counts ? mine[m] : 0, prm<R>(T, P2_ULID), coef);
+        fl[m] &= CODE2_INLET | CODE2_OUTLET;
+      } else {
+        for (int q = pos; q < LINKS; q++) links[q].b = RULE2_PULL << 15;
+      }
+      pos += mine[m];
+    }
+  }
   DevState2* st = T.st;
   // what the launch before wrote: populations, step counter and inlet speed
   asm volatile("griddepcontrol.wait;" ::: "memory");
@@ -172,13 +318,38 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
       for (int i = 0; i < Q2; i++) buf[(Q2 + i) * cells + c] = v[i];
     }
   }
+  // whether the tile has cells with a force, and whether some of them are not in the list
+  bool unlisted = false;
+#pragma unroll
+  for (int m = 0; m < ROWS; m++) unlisted = unlisted || (!(fl[m] & CODE2_SOLID) && (fl[m] & CODE2_SLOT));
   slots = __syncthreads_or(slots ? 1 : 0) != 0;
+  unlisted = LIST ? __syncthreads_or(unlisted ? 1 : 0) != 0 : slots;
   for (int j = 0; j < k; j++) {
-    const S* cur = buf + (j & 1) * (Q2 * cells);
+    S* cur = buf + (j & 1) * (Q2 * cells);
     S* nxt = buf + ((j + 1) & 1) * (Q2 * cells);
     const int lo = cut + j + 1;  // the margin that is still exact after this step begins here
     const bool colOn = (int)threadIdx.x >= lo && (int)threadIdx.x < RX - lo;
     const R u = (R)sU[j];
+    auto sampled = [&]() { return slots && every > 0 && (sStep + (unsigned)j + 1u) % (unsigned)every == 0u; };
+    if (LIST && nLinks > 0) {
+      for (int l = tid; l < nLinks; l += RX * BY) linkT[l] = link2<S, R>(links[l], cur);
+      __syncthreads();
+    }
+    const bool listed = LIST && sampled();  // without a list it is asked late, for want of registers
+    if (listed) {
+      double v = 0.0;
+      if ((tid & ~31) < nLinks) {
+        double ax = 0.0, ay = 0.0;
+        for (int l = tid; l < nLinks; l += RX * BY) {
+          R lx, ly;
+          cell_force2<R>(links, linkT, l, lx, ly);
+          ax += (double)lx;
+          ay += (double)ly;
+        }
+        v = warp_sum2(ax, ay, tid & 31);
+      }
+      if ((tid & 31) < 2) sWarp[j][tid >> 5][tid & 31] = v;
+    }
     double fx = 0.0, fy = 0.0;
 #pragma unroll
     for (int m = 0; m < ROWS; m++) {
@@ -205,7 +376,7 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
             if (flag & CODE2_SLOT) coef += ((size_t)(__ldg(&flags[idx]) >> BIDX2_SHIFT) - 1) * 8;
             rules2<C>(flag, T, ts, coef, f, force);
           }
-          if (flag & (CODE2_INLET | CODE2_OUTLET)) zou_he2<C>(T, H, (flag & CODE2_INLET) != 0u, u, y, f);
+          if (flag & (CODE2_INLET | CODE2_OUTLET)) zou_he2<C>(LIST ? parabolic : T.parabolic, H, (flag & CODE2_INLET) != 0u, u, y, f);
         }
         if ((flag & CODE2_SLOT) && colOwn && r >= K && r < RY - K && oy + r < H) {
           fx += (double)force[0];
@@ -215,7 +386,7 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
       if constexpr (kExact2)
         collide2<C>(T, xt, forcing, smagC2, H, u, y, f, o);
       else
-        collide2_lean<R>(T, xt, forcing, smagC2, lambda, H, u, y, f, o);
+        collide2_lean<R>(T, xt, forcing, smagC2, lambda, H, LIST ? parabolic : T.parabolic, u, y, f, o);
       if (j + 1 < k) {
 #pragma unroll
         for (int i = 0; i < Q2; i++) nxt[i * cells + r * RX + threadIdx.x] = (S)o[i];
@@ -224,22 +395,18 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
         for (int i = 0; i < Q2; i++) dst[i * N + idx] = (S)o[i];
       }
     }
-    if (slots && every > 0 && (sStep + (unsigned)j + 1u) % (unsigned)every == 0u) {
-#pragma unroll
-      for (int s = 16; s > 0; s >>= 1) {
-        fx += __shfl_down_sync(0xffffffffu, fx, s);
-        fy += __shfl_down_sync(0xffffffffu, fy, s);
-      }
-      if ((tid & 31) == 0) sWarp[j][tid >> 5] = make_double2(fx, fy);
+    if (LIST ? listed && unlisted : sampled()) {
+      const double v = warp_sum2(fx, fy, tid & 31);
+      if ((tid & 31) < 2) sWarp[j][tid >> 5][tid & 31] = LIST ? sWarp[j][tid >> 5][tid & 31] + v : v;
     }
     __syncthreads();
   }
   if (every > 0 && tid < k && (sStep + (unsigned)tid + 1u) % (unsigned)every == 0u) {
     double ax = 0.0, ay = 0.0;
     if (slots) {
-      for (int w = 0; w < RX * BY / 32; w++) {
-        ax += sWarp[tid][w].x;
-        ay += sWarp[tid][w].y;
+      for (int w = 0; w < WARPS; w++) {
+        ax += sWarp[tid][w][0];
+        ay += sWarp[tid][w][1];
       }
     }
     partials[(size_t)(j0 + tid) * gridDim.x + b] = make_double2(ax, ay);
@@ -288,19 +455,21 @@ static cudaError_t launch_block2_t(const Block2Launch& a, cudaStream_t s) {
   const int shape = a.regionX * 1000 + a.regionY * 10 + a.rows;
   if constexpr (sizeof(typename C::R) == 4) {
     switch (shape) {
-      case 32281: fn = block2d_kernel<C, 32, 28, 1>; break;
-      case 32321: fn = block2d_kernel<C, 32, 32, 1>; break;
-      case 64322: fn = block2d_kernel<C, 64, 32, 2>; break;
-      case 64483: fn = block2d_kernel<C, 64, 48, 3>; break;
+      case 32241: fn = block2d_kernel<C, 32, 24, 1, true>; break;
+      case 32321: fn = block2d_kernel<C, 32, 32, 1, true>; break;
+      case 64322: fn = block2d_kernel<C, 64, 32, 2, true>; break;
+      case 64483: fn = a.list ? block2d_kernel<C, 64, 48, 3, true> : block2d_kernel<C, 64, 48, 3, false>; break;
     }
   } else {
     switch (shape) {
-      case 32242: fn = block2d_kernel<C, 32, 24, 2>; break;
-      case 32322: fn = block2d_kernel<C, 32, 32, 2>; break;
+      case 32242: fn = block2d_kernel<C, 32, 24, 2, true>; break;
+      case 32322: fn = a.list ? block2d_kernel<C, 32, 32, 2, true> : block2d_kernel<C, 32, 32, 2, false>; break;
     }
   }
   if (!fn) return cudaErrorInvalidValue;
-  const size_t smem = 2 * Q2 * sizeof(typename C::S) * (size_t)a.regionX * a.regionY;
+  const size_t links = !a.list ? 0 : (size_t)a.regionX * a.regionY >= 3072 ? kTileLinks2<64, 48> : kTileLinks2<32, 32>;
+  const size_t smem = 2 * Q2 * sizeof(typename C::S) * (size_t)a.regionX * a.regionY +
+                      links * (sizeof(Link2<typename C::R>) + sizeof(typename C::R));
   cudaError_t e = cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
   if (e != cudaSuccess) return e;
   cudaLaunchAttribute attr[1];
@@ -312,7 +481,7 @@ static cudaError_t launch_block2_t(const Block2Launch& a, cudaStream_t s) {
   cfg.dynamicSmemBytes = smem;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = a.first ? 0 : 1;  // a run's first launch waits for everything before it: the tables are read early
   return cudaLaunchKernelEx(&cfg, fn, a.tunnels, a.layout, a.tileTunnel, a.K, a.k, a.par, a.partials, a.j0);
 }
 

@@ -36,10 +36,12 @@ struct Block2Launch {
   const unsigned short* tileTunnel;  // device array: the tunnel of each tile
   int nTiles;
   int regionX, regionY, rows;        // region of a block and cell rows per thread
+  bool list;                         // the tile's boundary links are collected and go ahead of the cells
   int K, k;
   int par;                           // parity of the first step
   double2* partials;                 // force partials [step of the run][tile]; NULL: no sampling
   int j0;                            // the launch's first step in the run
+  bool first;                        // the first launch of a run: it starts after all work before it
 };
 
 // precision: 0 f32, 3 f64. fast: FMA contraction allowed; exact: every operation rounds as written.

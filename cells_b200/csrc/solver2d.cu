@@ -127,7 +127,7 @@ struct Cells2DBatch : HandleBase {
   // several steps per launch (block2d.cu): the default way to take two steps or more, unless a launch
   // shape was asked for or the autotuner found another one faster
   bool blockWanted = false, blockOn = false;  // blockOn: wanted and possible (tables, periodic sides >= 3)
-  int blockK = 0, regionX = 0, regionY = 0, regionRows = 1;
+  int blockK = 0, blockList = 0, regionX = 0, regionY = 0, regionRows = 1;
   int nBlockTiles = 0;
   Block2Tunnel* dLayout = nullptr;
   unsigned short* dBlockTiles = nullptr;
@@ -336,26 +336,26 @@ void Cells2DBatch::rebuild_flags(int k) {
 // The block kernel's tables. A device without room for them steps one launch at a time.
 void Cells2DBatch::alloc_rules() {
   if (dev.fake) return;
-  unsigned long long total = 1u << 22;
+  auto room = [](unsigned long long bytes) { return (bytes + 255) / 256 * 256; };
+  unsigned long long total = 0;
   for (Tunnel2Host& T : t) {
     // coefficient slots for the cells around a body: a few times the grid's outline (further body cells
     // keep the general rules)
     T.qCap = (int)std::min<long long>(T.N, 4LL * (T.W + T.H));
-    total += (unsigned long long)T.N * 4 + (unsigned long long)T.qCap * 16 * bpp;
+    total += room((unsigned long long)T.N * 4) + room((unsigned long long)T.qCap * 16 * bpp);
   }
-  if (total > dev.free_bytes()) return;
+  if (total + (1u << 22) > dev.free_bytes()) return;
+  char* p = nullptr;
   try {
-    for (Tunnel2Host& T : t) {
-      T.qCoef = dev.alloc((size_t)T.qCap * 16 * bpp, "boundary coefficients");
-      T.code = (uint32_t*)dev.alloc((size_t)T.N * 4, "boundary rules");
-    }
+    p = (char*)dev.alloc(total, "boundary rules");
   } catch (const AllocError&) {
-    for (Tunnel2Host& T : t) {
-      if (T.qCoef) dev.release(T.qCoef);
-      if (T.code) dev.release(T.code);
-      T.qCoef = nullptr;
-      T.code = nullptr;
-    }
+    return;
+  }
+  for (Tunnel2Host& T : t) {
+    T.code = (uint32_t*)p;
+    p += room((unsigned long long)T.N * 4);
+    T.qCoef = p;
+    p += room((unsigned long long)T.qCap * 16 * bpp);
   }
 }
 
@@ -367,25 +367,31 @@ void Cells2DBatch::resolve_rules(int k) {
   dev.launches++;
 }
 
-// A region of the block kernel, the steps K per launch, and the number of tiles up to which it is taken.
+// A region of the block kernel, the steps K per launch, whether boundary links are listed, and the number of
+// tiles up to which it is taken.
 struct Region2 {
-  int x, y, rows, K, maxTiles;
+  int x, y, rows, K, list, maxTiles;
 };
-// us per step of one tunnel with a circle and Smagorinsky off, FP32 [one step per launch before]:
-//                 128x128  400x100  500x140  700x180  1000x250  1500x400  2000x500  4000x1000
-//   32x28x1 K=7     2.70     2.83     3.65     4.96      8.53     18.78     30.68     119.81
-//   32x32x1 K=5     3.14     3.19     3.16     3.75      6.36     13.85     22.07      86.06
-//   64x32x2 K=5     4.62     4.88     5.11     5.09      5.37     10.41     16.71      63.49
-//   64x48x3 K=5     6.51     5.97     6.42     7.55      7.63     10.29     15.18      57.63
-//   [before         9.48    12.13    11.98    14.47     21.72     29.90     45.48     192.38]
-// and for 64 NACA tunnels with Smagorinsky: 189, 138, 102 to 105, 95 [117]. A grid whose tiles fit on the SMs
-// at once pays for the latency of a launch, spread over its steps: small regions, many steps. A larger one
-// is bound by issue, and the margins are computed twice: (x - 2K)(y - 2K) / xy of the work is kept, so the
-// region grows with the number of tiles until shared memory is full (64x48 in two buffers).
-// FP64, same order: 32x24x2 K=7 3.62 (128x128), 4.26 (400x100), 7.89 (700x180), 14.3 (1000x250), 209 (4000x1000);
-// 32x32x2 K=5 4.35, 5.28, 5.15, 9.06, 129; 32x32x2 K=3 5.53, 4.32, 6.08, 8.58, 126 [9.09, 12.3, 15.9, 25.0, 312].
-constexpr Region2 kRegions32[] = {{32, 28, 1, 7, 222}, {32, 32, 1, 5, 296}, {64, 32, 2, 5, 444}, {64, 48, 3, 5, INT_MAX}};
-constexpr Region2 kRegions64[] = {{32, 24, 2, 7, 296}, {32, 32, 2, 5, 296}, {32, 32, 2, 3, INT_MAX}};
+// us per step of one tunnel with a circle, FP32 [one step per launch before]:
+//                 64x64  128x128  300x80  400x100  500x140  700x180  1000x250  1500x400  2000x500
+//   32x24x1 K=7    1.96     2.05    2.04     2.50     3.60     5.79     10.77     24.40     40.76
+//   32x32x1 K=7    2.43     2.47    2.26     2.36     3.21     4.82      8.95     20.07     32.61
+//   64x32x2 K=7    3.26     3.44    2.88     3.06     3.02     3.04      5.42     12.17     19.14
+//   64x48x3 K=5    4.62     4.99    5.04     4.60     4.66     4.78      4.63     11.19     17.00
+//     no list      6.33     6.51    5.07     5.97     6.42     7.55      7.63     10.29     15.18
+//   [before        8.88     9.48    8.57    12.13    11.98    14.47     21.72     29.90     45.48]
+// and for 64 NACA tunnels with Smagorinsky 64x48x3 K=5 103 with a list, 95 without [117]. Tiles that are all
+// resident at once (148 SMs, one block each) step at the pace of the slowest, the one with the body: the
+// smallest region that gives one wave, and its links listed. With more waves the work counts: the margins
+// are computed twice, so (x - 2K)(y - 2K) / xy of it is kept, the region is the largest that shared memory
+// holds in two buffers, and the list's registers and barriers cost more than they save.
+// FP64: 32x24x2 K=7 2.70 (128x128), 3.58 (400x100); 32x32x2 K=7 3.11, 2.79; without a list K=5 5.15 (700x180),
+// 9.06 (1000x250), 129 (4000x1000), K=3 6.08, 8.58, 126 [9.09, 12.3, 15.9, 25.0, 312].
+constexpr int kWave2 = 148;
+constexpr Region2 kRegions32[] = {{32, 24, 1, 7, 1, kWave2}, {32, 32, 1, 7, 1, kWave2}, {64, 32, 2, 7, 1, kWave2},
+                                  {64, 48, 3, 5, 1, kWave2}, {64, 48, 3, 5, 0, INT_MAX}};
+constexpr Region2 kRegions64[] = {{32, 24, 2, 7, 1, kWave2}, {32, 32, 2, 7, 1, kWave2}, {32, 32, 2, 5, 0, 2 * kWave2},
+                                  {32, 32, 2, 3, 0, INT_MAX}};
 
 // The block kernel's region and step count, its tiles numbered tunnel by tunnel, and the tile -> tunnel map.
 void Cells2DBatch::choose_block() {
@@ -412,7 +418,7 @@ void Cells2DBatch::choose_block() {
     if (tiles <= r.maxTiles || r.maxTiles == INT_MAX) break;
   }
   if (tiles > INT_MAX) return;
-  if (dLayout && r.x == regionX && r.y == regionY && K == blockK) {
+  if (dLayout && r.x == regionX && r.y == regionY && K == blockK && r.list == blockList) {
     blockOn = true;
     return;
   }
@@ -448,6 +454,7 @@ void Cells2DBatch::choose_block() {
   regionY = r.y;
   regionRows = r.rows;
   blockK = K;
+  blockList = r.list;
   nBlockTiles = (int)map.size();
   dev.h2d(dLayout, layout.data(), layout.size() * sizeof(Block2Tunnel));
   dev.h2d(dBlockTiles, map.data(), map.size() * sizeof(unsigned short));
@@ -486,8 +493,10 @@ void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
   a.regionY = regionY;
   a.rows = regionRows;
   a.K = blockK;
+  a.list = blockList != 0;
   a.partials = sampled ? runPartials : nullptr;
   a.j0 = 0;
+  a.first = true;
   while (n > 0) {
     a.k = (int)std::min<int64_t>(std::min<int64_t>(n, blockK), kRunSteps2 - a.j0);
     if (a.k % 2 == 0) a.k--;
@@ -495,6 +504,7 @@ void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
     check_cuda(ex ? exact::launch_block2(prec, a, dev.stream) : fast::launch_block2(prec, a, dev.stream),
                "block step kernel");
     dev.launches++;
+    a.first = false;
     par ^= 1;
     n -= a.k;
     a.j0 += a.k;

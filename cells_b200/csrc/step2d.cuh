@@ -155,11 +155,11 @@ __device__ __forceinline__ typename C::R pull_slow2(int i, const Geo2& g, const 
 
 // Zou-He inlet and outlet (populations stored shifted by w_i)
 template <class C>
-__device__ __forceinline__ void zou_he2(const Tunnel2& T, int H, bool inlet, typename C::R uIn, int y,
+__device__ __forceinline__ void zou_he2(int parabolic, int H, bool inlet, typename C::R uIn, int y,
                                         typename C::R (&f)[Q2]) {
   using R = typename C::R;
   if (inlet) {
-    const R u = inlet_velocity2<R>(T.parabolic, uIn, H, y);
+    const R u = inlet_velocity2<R>(parabolic, uIn, H, y);
     const R r = (R(1) + f[0] + f[2] + f[4] + R(2) * (f[3] + f[6] + f[7])) / (R(1) - u);
     f[1] = f[3] + (R)(2.0 / 3.0) * r * u;
     f[5] = f[7] - R(0.5) * (f[2] - f[4]) + (R)(1.0 / 6.0) * r * u;
@@ -193,7 +193,7 @@ __device__ __forceinline__ bool boundary2(const Tunnel2& T, const Geo2& g, const
       if (fl & (1u << i)) f[i] = pull_slow2<C>(i, g, src, flags, T.sdf, x, y, idx, uLid, force);
     slot = (fl >> BIDX2_SHIFT) != 0u;
   }
-  if (fl & (FLAG2_INLET | FLAG2_OUTLET)) zou_he2<C>(T, g.H, (fl & FLAG2_INLET) != 0u, uIn, y, f);
+  if (fl & (FLAG2_INLET | FLAG2_OUTLET)) zou_he2<C>(T.parabolic, g.H, (fl & FLAG2_INLET) != 0u, uIn, y, f);
   return slot;
 }
 
@@ -210,7 +210,7 @@ __device__ __forceinline__ bool boundary2(const Tunnel2& T, const Geo2& g, const
 // the NACA section take 102 us per step like this and 163 to 190 us packed (spills at 64 and 128 registers).
 template <class R>
 __device__ __forceinline__ void collide2_lean(const Tunnel2& T, const typename XTab2<R>::T& xt, int forcing, R smagC2,
-                                              R lambda, int H, R uIn, int y, const R (&f)[Q2], R (&o)[Q2]) {
+                                              R lambda, int H, int parabolic, R uIn, int y, const R (&f)[Q2], R (&o)[Q2]) {
   constexpr int A[4] = {1, 2, 5, 6}, B[4] = {3, 4, 7, 8};
   R s[4], d[4];
 #pragma unroll
@@ -267,7 +267,7 @@ __device__ __forceinline__ void collide2_lean(const Tunnel2& T, const typename X
   // absorbing-layer and Guo body-force sources (src/shaders/step.ts:65-91)
   const R sig = xt.z;
   if (sig > R(0)) {
-    const R ut = inlet_velocity2<R>(T.parabolic, uIn, H, y);
+    const R ut = inlet_velocity2<R>(parabolic, uIn, H, y);
     const R dq = R(1.5) * rho * (ut * ut - uu);
     o0 -= sig * w2<R>(0) * dq;
 #pragma unroll

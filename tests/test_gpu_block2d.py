@@ -53,7 +53,7 @@ def compare(W, H, cfg, precision, counts, edit=None):
     s.destroy()
 
 
-# 18 x 14 (FP32) and 18 x 10 (FP64) cells per tile of a small tunnel: exact, one over, one short, one row, one cell
+# 18 x 10 cells per tile of a small tunnel: exact, one over, one short, one row, one cell
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
 @pytest.mark.parametrize("size", [(36, 28), (37, 29), (35, 41), (50, 1), (3, 3), (64, 7)])
 @pytest.mark.parametrize("modes", [CHANNEL, PERIODIC, CAVITY, SLIP])
@@ -61,9 +61,10 @@ def test_tile_edges(precision, size, modes):
     compare(*size, case(modes, every=3, smag=0.1), precision, (2, 7, 1, 130, 4))
 
 
-# small grids take 32x28 (FP64 32x24) regions; larger ones 32x32, 64x32 and 64x48 (FP64 32x32 with 5 and 3 steps)
+# the smallest grids take 32x24 regions; larger ones 32x32, 64x32, 64x48 with and without a list of links (FP64 32x32
+# with 7 steps and a list, with 5 and with 3 steps without)
 @pytest.mark.parametrize("precision", ["fp32", "fp64"])
-@pytest.mark.parametrize("size", [(300, 200), (500, 300), (905, 605)])
+@pytest.mark.parametrize("size", [(400, 100), (300, 200), (500, 300), (905, 605)])
 @pytest.mark.parametrize("modes", [CHANNEL, PERIODIC])
 def test_region_shapes(precision, size, modes):
     compare(*size, case(modes, smag=0.1), precision, (7, 6))
