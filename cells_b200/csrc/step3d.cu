@@ -1142,9 +1142,9 @@ __device__ __forceinline__ void prefetch_tile_ahead(const StepArgs3<C>& a) {
   }
 }
 
-// ALT: a.reverse may be set. f64 has kernels with and without it: what it changes in the interior code costs
-// grids that never reverse 3-4% (200x100x96 97.9 -> 102.5 us a step); the f32 kernel and the 16-bit x-pairs
-// lose nothing.
+// ALT: a.reverse may be set. f64 and the 16-bit x-pairs have kernels with and without it: what it changes in the
+// interior code costs grids that never reverse 3-4% in f64 (200x100x96 97.9 -> 102.5 us a step), 1-2% in bf16
+// (256x128x128 59.2 -> 60.6), nothing in f32.
 template <class C, bool SMAG, int PAIR, bool ALT>
 __global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR != 0))
     step3d_kernel(const __grid_constant__ StepArgs3<C> a) {
@@ -1282,9 +1282,10 @@ static cudaError_t launch_step3_t(const StepLaunch3& L, cudaStream_t s) {
   //   16    160x80x80 18.1 -> 17.6, 192x96x96 (67 MB) 28.9 -> 27.6, 224x112x112 (107 MB) 46.7 -> 47.1,
   //         256x128x128 (159 MB) 61.0 -> 61.7; one cell per thread is bound by issue (fp16 255x127x127
   //         121.5 -> 123.2)
-  //   f64   112x56x56 (53 MB) 23.5 -> 20.7, 128x64x64 (80 MB) 28.9 -> 27.9, 136x70x66 (96 MB) 34.6 -> 36.2
+  //   f64   112x56x56 (53 MB) 23.5 -> 20.7, 128x64x64 (80 MB) 28.9 -> 27.9, 129x65x65 (83 MB) 33.8 -> 34.1,
+  //         136x70x66 (96 MB) 34.6 -> 36.2
   const unsigned long long altMax = sizeof(S) == 4 ? 150ull << 20
-                                                   : (sizeof(S) == 8 || pair ? 84ull << 20 : 0ull);
+                                                   : (sizeof(S) == 8 ? 78ull << 20 : (pair ? 84ull << 20 : 0ull));
   const bool alternate = 19ull * (unsigned long long)L.N * sizeof(S) <= altMax;
   a.reverse = L.par && alternate;
   // prefetch distance, measured on B200 at 192x96x96 and 256x128x128 (sphere tunnel, 1000 steps):
@@ -1305,6 +1306,8 @@ static cudaError_t launch_step3_t(const StepLaunch3& L, cudaStream_t s) {
   void (*fn)(StepArgs3<C>) = nullptr;
   if (pair) {
     if constexpr (sizeof(S) <= 4) fn = smag ? step3d_kernel<C, true, 1, true> : step3d_kernel<C, false, 1, true>;
+    if constexpr (sizeof(S) == 2)
+      if (!alternate) fn = smag ? step3d_kernel<C, true, 1, false> : step3d_kernel<C, false, 1, false>;
     if constexpr (sizeof(S) == 4 && !kExact)
       if (L.W % 2) fn = smag ? step3d_kernel<C, true, kFarPair, true> : step3d_kernel<C, false, kFarPair, true>;
   } else if (sizeof(S) != 2 && (sizeof(S) == 4 || alternate)) {
