@@ -345,6 +345,8 @@ void Cells2DBatch::alloc_rules() {
     total += room((unsigned long long)T.N * 4) + room((unsigned long long)T.qCap * 16 * bpp);
   }
   if (total + (1u << 22) > dev.free_bytes()) return;
+  for (const Tunnel2Host& T : t)
+    if (T.cfg.max_buffer_bytes > 0 && total > T.cfg.max_buffer_bytes) return;
   char* p = nullptr;
   try {
     p = (char*)dev.alloc(total, "boundary rules");

@@ -116,3 +116,21 @@ def test_fast_build_and_batches_match_single_steps(precision, eps, modes):
         assert len(t.readForces()) == len(one.readForces()) == n // 2
         one.destroy()
     batch.destroy()
+
+
+# a periodic side bounds the steps per launch; below 3 cells steps go one by one, as they do for a fixed block size
+@pytest.mark.parametrize("size", [(40, 2), (40, 4), (5, 30)])
+def test_new_modes_choose_again(size):
+    out = []
+    for workgroup in (0, 128):
+        s = Solver.create(width=size[0], height=size[1], exactArithmetic=True, workgroupSize=workgroup, **case(CHANNEL, 2))
+        s.initField(perturbed_rest2(*size, 1e-3))
+        s.encodeSteps(9)
+        s.update(left=0, right=0, bottom=0, top=0, uIn=0.0)
+        s.encodeSteps(9)
+        s.update(left=2, right=2, bottom=2, top=2, uIn=0.05)
+        s.encodeSteps(11)
+        out.append(s.readPopulations())
+        s.destroy()
+    assert np.all(np.isfinite(out[0]))
+    assert np.array_equal(out[0], out[1])
