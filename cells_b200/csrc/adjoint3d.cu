@@ -234,8 +234,9 @@ __device__ __forceinline__ void block_du_partial(double du, double* part, int sl
 // reader, and f^n asked for before the dependency wait.
 
 // Programmatic dependent launch: waits for the boundary-element kernel of the step before to complete.
-// f^n, the tables and the flags do not depend on it (the recompute that wrote f^n ended before the
-// segment's first adjoint step, which follows an ordinary event), so the roles ask for them first.
+// f^n, the tables and the flags do not depend on it, so the roles ask for them first: a segment's first adjoint
+// step is launched without the attribute (launch_adjoint_step3's `first`), after all work before it, the recompute
+// that wrote the segment's states included.
 __device__ __forceinline__ void adj_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class R>
@@ -611,8 +612,9 @@ __global__ void __launch_bounds__(256) adj_du3_kernel(const double* __restrict__
   }
 }
 
+// A programmatic dependent of the launch before it, or (dependent = false) an ordinary launch.
 template <class... Args>
-cudaError_t launch_dependent(void (*fn)(Args...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+cudaError_t launch_dependent(void (*fn)(Args...), dim3 grid, dim3 block, cudaStream_t s, bool dependent, Args... args) {
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
@@ -621,7 +623,7 @@ cudaError_t launch_dependent(void (*fn)(Args...), dim3 grid, dim3 block, cudaStr
   cfg.blockDim = block;
   cfg.stream = s;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = dependent ? 1 : 0;
   return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 
@@ -644,7 +646,7 @@ int adj_face_blocks(int precision, int W, int H, int D, dim3 cells) {
 }
 
 template <class R>
-cudaError_t launch_adjoint_step3_t(AdjLaunch3 a, cudaStream_t s) {
+cudaError_t launch_adjoint_step3_t(AdjLaunch3 a, bool first, cudaStream_t s) {
   const int precision = sizeof(R) == 4 ? 0 : 3;
   const dim3 cells = adj_cell_grid(precision, a.W, a.H, a.D);
   a.nCellBlocks = (int)(cells.x * cells.y * cells.z);
@@ -668,19 +670,19 @@ cudaError_t launch_adjoint_step3_t(AdjLaunch3 a, cudaStream_t s) {
       if (adj_pairs(precision, a.W)) fn = adj_step3_kernel<R, true>;
     }
     const cudaError_t e = launch_dependent(fn, dim3(cells.x, cells.y, a.roleZ + cells.z),
-                                           dim3(kAdjTileX, kAdjThreads / kAdjTileX), s, a);
+                                           dim3(kAdjTileX, kAdjThreads / kAdjTileX), s, !first, a);
     if (e != cudaSuccess) return e;
   }
   if (a.nRows == 0) return cudaSuccess;
-  return launch_dependent(adj_rows3_kernel<R>, dim3((unsigned)((a.nRows + 255) / 256)), dim3(256), s, a);
+  return launch_dependent(adj_rows3_kernel<R>, dim3((unsigned)((a.nRows + 255) / 256)), dim3(256), s, true, a);
 }
 
 }  // namespace
 
 namespace cells {
-cudaError_t launch_adjoint_step3(int precision, const AdjLaunch3& a, cudaStream_t s) {
-  if (precision == 0) return launch_adjoint_step3_t<float>(a, s);
-  if (precision == 3) return launch_adjoint_step3_t<double>(a, s);
+cudaError_t launch_adjoint_step3(int precision, const AdjLaunch3& a, bool first, cudaStream_t s) {
+  if (precision == 0) return launch_adjoint_step3_t<float>(a, first, s);
+  if (precision == 3) return launch_adjoint_step3_t<double>(a, first, s);
   return cudaErrorInvalidValue;
 }
 }  // namespace cells
@@ -1197,7 +1199,7 @@ void enqueue_sweep(Cells3D* h, Adjoint3D* A, AdjLaunch3& a, int64_t sgi, int set
     a.blockPart = A->blockPart + (size_t)t * A->nParts;
     a.u = A->uStep[(size_t)n];
     a.w = label >= A->w0 && label <= A->w1 ? A->scale / (double)(A->w1 - A->w0 + 1) : 0.0;
-    check_cuda(launch_adjoint_step3(h->prec, a, s), "adjoint step kernel");
+    check_cuda(launch_adjoint_step3(h->prec, a, t == len - 1, s), "adjoint step kernel");
     h->dev.launches += 2;
     // elements that nothing reads keep zero, which a terminal adjoint in the first buffer is not
     if (terminal && n + 1 == A->steps) h->dev.memset0(A->lam[c], 19 * h->bpp * (size_t)h->N);

@@ -140,7 +140,8 @@ struct AdjTables3 {
 constexpr int kAdjThreads = 128;
 constexpr int kAdjTileX = 32;
 // One adjoint step (precision 0 or 3): the interior and flagged cells in one launch, then the
-// boundary-element kernel.
-cudaError_t launch_adjoint_step3(int precision, const AdjLaunch3& a, cudaStream_t s);
+// boundary-element kernel. The step reads f^n before it waits for the launch before it; first: the step starts
+// after all work before it on the stream (the recompute of its segment's states).
+cudaError_t launch_adjoint_step3(int precision, const AdjLaunch3& a, bool first, cudaStream_t s);
 
 }  // namespace cells
