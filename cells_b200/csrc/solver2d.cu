@@ -26,7 +26,7 @@ namespace {
 
 constexpr int kGraphSteps2 = 100;
 constexpr int kPersistentChunk = 500;
-constexpr int kRunSteps2 = 126;  // steps whose force partials wait for one sum: 18 launches of 7
+constexpr int kRunSteps2 = 126;  // most steps whose force partials wait for one sum: 18 launches of 7
 
 struct Shape2 {
   int tx, ty;
@@ -131,9 +131,11 @@ struct Cells2DBatch : HandleBase {
   int nBlockTiles = 0;
   Block2Tunnel* dLayout = nullptr;
   unsigned short* dBlockTiles = nullptr;
-  double2* runPartials = nullptr;  // force partials of a run of kRunSteps2 steps
+  double2* runPartials = nullptr;  // force partials of a run of runSteps steps
+  int runSteps = 0;
   bool runPartialsOff = false;     // they did not fit
   void alloc_rules();
+  unsigned long long buffer_limit() const;
   void choose_block();
   bool samples_force() const;
   bool run_partials();
@@ -333,32 +335,53 @@ void Cells2DBatch::rebuild_flags(int k) {
   resolve_rules(k);
 }
 
-// The block kernel's tables. A device without room for them steps one launch at a time.
+// The block kernel's tables: one buffer for the batch, or, where that exceeds the largest buffer that a tunnel's
+// caller allows, one for each table. A device without room for them steps one launch at a time.
 void Cells2DBatch::alloc_rules() {
   if (dev.fake) return;
   auto room = [](unsigned long long bytes) { return (bytes + 255) / 256 * 256; };
-  unsigned long long total = 0;
+  unsigned long long total = 0, limit = buffer_limit();
   for (Tunnel2Host& T : t) {
     // coefficient slots for the cells around a body: a few times the grid's outline (further body cells
     // keep the general rules)
     T.qCap = (int)std::min<long long>(T.N, 4LL * (T.W + T.H));
+    if (T.cfg.max_buffer_bytes > 0)
+      T.qCap = (int)std::min<unsigned long long>((unsigned long long)T.qCap, T.cfg.max_buffer_bytes / (16 * bpp));
     total += room((unsigned long long)T.N * 4) + room((unsigned long long)T.qCap * 16 * bpp);
   }
   if (total + (1u << 22) > dev.free_bytes()) return;
-  for (const Tunnel2Host& T : t)
-    if (T.cfg.max_buffer_bytes > 0 && total > T.cfg.max_buffer_bytes) return;
+  std::vector<void*> taken;
   char* p = nullptr;
+  auto place = [&](unsigned long long bytes) {
+    if (total > limit) {
+      taken.push_back(dev.alloc(std::max<unsigned long long>(bytes, 1), "boundary rules"));
+      return taken.back();
+    }
+    void* at = p;
+    p += room(bytes);
+    return at;
+  };
   try {
-    p = (char*)dev.alloc(total, "boundary rules");
+    if (total <= limit) p = (char*)dev.alloc(total, "boundary rules");
+    for (Tunnel2Host& T : t) {
+      T.code = (uint32_t*)place((unsigned long long)T.N * 4);  // below the tunnel's own limit: 36 N is
+      T.qCoef = place((unsigned long long)T.qCap * 16 * bpp);
+    }
   } catch (const AllocError&) {
-    return;
+    for (void* q : taken) dev.release(q);
+    for (Tunnel2Host& T : t) {
+      T.code = nullptr;
+      T.qCoef = nullptr;
+    }
   }
-  for (Tunnel2Host& T : t) {
-    T.code = (uint32_t*)p;
-    p += room((unsigned long long)T.N * 4);
-    T.qCoef = p;
-    p += room((unsigned long long)T.qCap * 16 * bpp);
-  }
+}
+
+// The largest single buffer that every tunnel's caller allows.
+unsigned long long Cells2DBatch::buffer_limit() const {
+  unsigned long long limit = ULLONG_MAX;
+  for (const Tunnel2Host& T : t)
+    if (T.cfg.max_buffer_bytes > 0) limit = std::min<unsigned long long>(limit, T.cfg.max_buffer_bytes);
+  return limit;
 }
 
 // The block kernel's rules follow the flags and the SDF.
@@ -473,8 +496,14 @@ bool Cells2DBatch::samples_force() const {
 bool Cells2DBatch::run_partials() {
   if (runPartials) return true;
   if (runPartialsOff) return false;
+  const unsigned long long perStep = (unsigned long long)nBlockTiles * sizeof(double2);
+  runSteps = (int)std::min<unsigned long long>(kRunSteps2, buffer_limit() / perStep);
+  if (runSteps < blockK) {
+    runPartialsOff = true;
+    return false;
+  }
   try {
-    runPartials = (double2*)dev.alloc((size_t)nBlockTiles * kRunSteps2 * sizeof(double2), "force partials of a run");
+    runPartials = (double2*)dev.alloc((size_t)(perStep * (unsigned)runSteps), "force partials of a run");
   } catch (const AllocError&) {
     runPartialsOff = true;
   }
@@ -482,7 +511,7 @@ bool Cells2DBatch::run_partials() {
 }
 
 // n steps from parity par, an odd number at most blockK per launch; the force partials of up to
-// kRunSteps2 steps are summed together.
+// runSteps steps are summed together.
 void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
   const bool sampled = allowSample && samples_force();
   const bool ex = arithmetic == CELLS_ARITH_EXACT;
@@ -500,7 +529,8 @@ void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
   a.j0 = 0;
   a.first = true;
   while (n > 0) {
-    a.k = (int)std::min<int64_t>(std::min<int64_t>(n, blockK), kRunSteps2 - a.j0);
+    a.k = (int)std::min<int64_t>(n, blockK);
+    if (sampled) a.k = std::min(a.k, runSteps - a.j0);
     if (a.k % 2 == 0) a.k--;
     a.par = par;
     check_cuda(ex ? exact::launch_block2(prec, a, dev.stream) : fast::launch_block2(prec, a, dev.stream),
@@ -510,7 +540,7 @@ void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
     par ^= 1;
     n -= a.k;
     a.j0 += a.k;
-    if (sampled && (n == 0 || a.j0 == kRunSteps2)) {
+    if (sampled && (n == 0 || a.j0 == runSteps)) {
       check_cuda(fast::launch_sum_samples2(dTunnels, dLayout, (int)t.size(), runPartials, nBlockTiles, a.j0, par,
                                            dev.stream),
                  "force sum kernel");
