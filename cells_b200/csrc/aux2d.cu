@@ -37,7 +37,8 @@ __device__ __forceinline__ void wrap2a(const AuxLaunch2& a, int& x, int& y) {
 template <class C>
 __global__ void flags2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, uint32_t* __restrict__ flags,
                               typename C::S* __restrict__ fA, typename C::S* __restrict__ fB,
-                              const float4* __restrict__ mac, unsigned* __restrict__ counter) {
+                              const float4* __restrict__ mac, unsigned* __restrict__ counter,
+                              typename C::S* __restrict__ prev, int older) {
   using R = typename C::R;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= a.N) return;
@@ -51,6 +52,10 @@ __global__ void flags2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, uint3
   };
   const uint32_t old = flags[idx];
   if (solidAt(x, y)) {
+    if (prev && !(old & FLAG2_SOLID)) {
+      typename C::S* f = older ? fB : fA;
+      for (int i = 0; i < Q2; i++) f[i * (long long)a.N + idx] = prev[i * (long long)a.N + idx];
+    }
     flags[idx] = FLAG2_SOLID;
     return;
   }
@@ -99,6 +104,7 @@ __global__ void flags2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, uint3
       const typename C::S v = (typename C::S)feq2a<R>(i, rho, ux, uy);
       fA[i * (long long)a.N + idx] = v;
       fB[i * (long long)a.N + idx] = v;
+      if (prev) prev[i * (long long)a.N + idx] = v;
     }
   }
 }
@@ -296,9 +302,10 @@ cudaError_t launch_rules2(int precision, const AuxLaunch2& a, const float* sdf, 
 }
 
 cudaError_t launch_flags2(int precision, const AuxLaunch2& a, const float* sdf, uint32_t* flags, void* fA, void* fB,
-                          const float4* mac, unsigned* counter, cudaStream_t s) {
+                          const float4* mac, unsigned* counter, void* prev, int older, cudaStream_t s) {
   CELLS2_DISPATCH(precision, (flags2_kernel<C><<<blocks_for2(a.N, 256), 256, 0, s>>>(
-                                 a, sdf, flags, (typename C::S*)fA, (typename C::S*)fB, mac, counter)));
+                                 a, sdf, flags, (typename C::S*)fA, (typename C::S*)fB, mac, counter,
+                                 (typename C::S*)prev, older)));
   return cudaGetLastError();
 }
 

@@ -185,8 +185,9 @@ __device__ __forceinline__ int real_coord2(int v, int n, bool wrapLow, bool wrap
   return v;
 }
 
-// Region RX x RY cells, ROWS rows per thread; tiles of (RX - 2 K) x (RY - 2 K) cells.
-template <class C, int RX, int RY, int ROWS, bool LIST>
+// Region RX x RY cells, ROWS rows per thread; tiles of (RX - 2 K) x (RY - 2 K) cells. LAST: a run's last launch, of
+// several steps.
+template <class C, int RX, int RY, int ROWS, bool LIST, bool LAST>
 __global__ void __launch_bounds__(RX * RY / ROWS, 1)
     block2d_kernel(const Tunnel2* __restrict__ tunnels, const Block2Tunnel* __restrict__ layout,
                    const unsigned short* __restrict__ tileTunnel, int K, int k, int par, double2* __restrict__ partials,
@@ -313,9 +314,12 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
     for (int i = 0; i < Q2; i++) v[i] = C::ld(src + (i * N + idx));
 #pragma unroll
     for (int i = 0; i < Q2; i++) buf[i * cells + c] = v[i];
-    if (fl[m] & CODE2_SOLID) {  // a slip row may mirror a solid's populations: they are in both halves
+    if ((fl[m] & CODE2_SOLID) && (ry[m] == 0 || ry[m] == H - 1)) {
+      // A slip row may mirror a solid's populations. No step writes them, and the two buffers differ where the cell
+      // became solid between steps: the steps find them in turn, as step by step. (Not through the read-only
+      // path: this launch writes that buffer's other cells.)
 #pragma unroll
-      for (int i = 0; i < Q2; i++) buf[(Q2 + i) * cells + c] = v[i];
+      for (int i = 0; i < Q2; i++) buf[(Q2 + i) * cells + c] = __ldcg((const S*)T.f[par ^ 1] + (i * N + idx));
     }
   }
   // whether the tile has cells with a force, and whether some of them are not in the list
@@ -411,6 +415,22 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
     }
     partials[(size_t)(j0 + tid) * gridDim.x + b] = make_double2(ax, ay);
   }
+  // The step before the last, still in the half that the last one read. The source buffer should hold it, as after
+  // single steps, for the cells that become solid next (flags2_kernel); it holds the k-th before, and other
+  // blocks may still read it. Bound by its stores, once a run: 100 steps of 2000x500 1,431 -> 1,437 us, 5 steps of
+  // 4000x1000 288 -> 316. A variant of its own, because as a branch it cost the launches that skip it (400x100
+  // 2.40 -> 2.45 us a step).
+  if constexpr (LAST) {
+    const S* cur = buf + ((k - 1) & 1) * (Q2 * cells);
+    S* __restrict__ prev = (S*)T.prev;
+#pragma unroll
+    for (int m = 0; m < ROWS; m++) {
+      const int r = threadIdx.y + m * BY;
+      if (!colOwn || r < K || r >= RY - K || oy + r >= H) continue;
+#pragma unroll
+      for (int i = 0; i < Q2; i++) __stcs(&prev[i * N + ry[m] * W + rx], cur[i * cells + r * RX + threadIdx.x]);
+    }
+  }
 }
 
 // After a run of n steps that ended on parity par: one block per tunnel, one warp per sampled step, adds
@@ -453,19 +473,23 @@ static cudaError_t launch_block2_t(const Block2Launch& a, cudaStream_t s) {
   using Kernel = void (*)(const Tunnel2*, const Block2Tunnel*, const unsigned short*, int, int, int, double2*, int);
   Kernel fn = nullptr;
   const int shape = a.regionX * 1000 + a.regionY * 10 + a.rows;
+  const bool last = a.last && a.k > 1;
+#define SHAPE2(RX, RY, ROWS, LIST) \
+  (last ? block2d_kernel<C, RX, RY, ROWS, LIST, true> : block2d_kernel<C, RX, RY, ROWS, LIST, false>)
   if constexpr (sizeof(typename C::R) == 4) {
     switch (shape) {
-      case 32241: fn = block2d_kernel<C, 32, 24, 1, true>; break;
-      case 32321: fn = block2d_kernel<C, 32, 32, 1, true>; break;
-      case 64322: fn = block2d_kernel<C, 64, 32, 2, true>; break;
-      case 64483: fn = a.list ? block2d_kernel<C, 64, 48, 3, true> : block2d_kernel<C, 64, 48, 3, false>; break;
+      case 32241: fn = SHAPE2(32, 24, 1, true); break;
+      case 32321: fn = SHAPE2(32, 32, 1, true); break;
+      case 64322: fn = SHAPE2(64, 32, 2, true); break;
+      case 64483: fn = a.list ? SHAPE2(64, 48, 3, true) : SHAPE2(64, 48, 3, false); break;
     }
   } else {
     switch (shape) {
-      case 32242: fn = block2d_kernel<C, 32, 24, 2, true>; break;
-      case 32322: fn = a.list ? block2d_kernel<C, 32, 32, 2, true> : block2d_kernel<C, 32, 32, 2, false>; break;
+      case 32242: fn = SHAPE2(32, 24, 2, true); break;
+      case 32322: fn = a.list ? SHAPE2(32, 32, 2, true) : SHAPE2(32, 32, 2, false); break;
     }
   }
+#undef SHAPE2
   if (!fn) return cudaErrorInvalidValue;
   const size_t links = !a.list ? 0 : (size_t)a.regionX * a.regionY >= 3072 ? kTileLinks2<64, 48> : kTileLinks2<32, 32>;
   const size_t smem = 2 * Q2 * sizeof(typename C::S) * (size_t)a.regionX * a.regionY +

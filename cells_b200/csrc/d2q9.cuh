@@ -95,6 +95,7 @@ struct Tunnel2 {
   const float* sdf;       // N
   const uint32_t* code;   // N, the block kernel's rules of each cell
   const void* qCoef;      // (c1, c2) of the body rules, [slot - 1][direction - 1], in the arithmetic type
+  void* prev;             // 9 N: the populations one step before the last, from a run's last block launch
   double2* partials;      // one force partial per tile
   double2* history;       // HISTORY2_LEN force samples
   DevState2* st;

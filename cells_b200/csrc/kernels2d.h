@@ -42,6 +42,7 @@ struct Block2Launch {
   double2* partials;                 // force partials [step of the run][tile]; NULL: no sampling
   int j0;                            // the launch's first step in the run
   bool first;                        // the first launch of a run: it starts after all work before it
+  bool last;                         // the last one: it leaves the step before its last in Tunnel2::prev
 };
 
 // precision: 0 f32, 3 f64. fast: FMA contraction allowed; exact: every operation rounds as written.
@@ -73,8 +74,11 @@ struct AuxLaunch2 {
 
 // flagsShader (src/shaders/aux.ts:22-88): flags with force slots from *counter (zeroed first) and
 // the refill of uncovered cells from mac.
+// A cell that becomes solid keeps the populations of the last step and of the one before it, one in each buffer.
+// prev: those of the step before it, where the buffer that should hold them (older: 0 fA, 1 fB) holds an earlier
+// step because the last launch took several; else NULL. It is kept in step with the refill of uncovered cells.
 cudaError_t launch_flags2(int precision, const AuxLaunch2& a, const float* sdf, uint32_t* flags, void* fA, void* fB,
-                          const float4* mac, unsigned* counter, cudaStream_t s);
+                          const float4* mac, unsigned* counter, void* prev, int older, cudaStream_t s);
 // The block kernel's rule words and Bouzidi coefficients from the flags and the SDF; cells whose force
 // slot exceeds qCap keep the general rules.
 cudaError_t launch_rules2(int precision, const AuxLaunch2& a, const float* sdf, const uint32_t* flags, uint32_t* code,

@@ -44,6 +44,8 @@ struct Tunnel2Host {
   uint32_t* code = nullptr;  // the block kernel's rules (Tunnel2::code, qCoef)
   void* qCoef = nullptr;
   int qCap = 0;
+  void* prev = nullptr;      // Tunnel2::prev
+  bool prevValid = false;    // it holds the step before the last; f[parity ^ 1] holds an earlier one
   float4* macro = nullptr;
   double2* partials = nullptr;
   int partialsCap = 0;
@@ -260,6 +262,7 @@ void Cells2DBatch::upload_tunnel(int k) {
   d.sdf = T.sdf;
   d.code = T.code;
   d.qCoef = T.qCoef;
+  d.prev = T.prev;
   d.partials = T.partials;
   d.history = T.history;
   d.st = T.st;
@@ -330,7 +333,9 @@ void Cells2DBatch::rebuild_flags(int k) {
   const AuxLaunch2 a = aux(k);
   check_cuda(launch_macro2(prec, a, T.f[parity], T.flags, T.macro, T.st, dev.stream), "macro kernel");
   dev.memset0(dCounter, sizeof(unsigned));
-  check_cuda(launch_flags2(prec, a, T.sdf, T.flags, T.f[0], T.f[1], T.macro, dCounter, dev.stream), "flags kernel");
+  check_cuda(launch_flags2(prec, a, T.sdf, T.flags, T.f[0], T.f[1], T.macro, dCounter, T.prevValid ? T.prev : nullptr,
+                           parity ^ 1, dev.stream),
+             "flags kernel");
   dev.launches += 2;
   resolve_rules(k);
 }
@@ -347,7 +352,8 @@ void Cells2DBatch::alloc_rules() {
     T.qCap = (int)std::min<long long>(T.N, 4LL * (T.W + T.H));
     if (T.cfg.max_buffer_bytes > 0)
       T.qCap = (int)std::min<unsigned long long>((unsigned long long)T.qCap, T.cfg.max_buffer_bytes / (16 * bpp));
-    total += room((unsigned long long)T.N * 4) + room((unsigned long long)T.qCap * 16 * bpp);
+    total += room((unsigned long long)T.N * 4) + room((unsigned long long)T.qCap * 16 * bpp) +
+             room(9ull * bpp * (unsigned long long)T.N);
   }
   if (total + (1u << 22) > dev.free_bytes()) return;
   std::vector<void*> taken;
@@ -364,14 +370,15 @@ void Cells2DBatch::alloc_rules() {
   try {
     if (total <= limit) p = (char*)dev.alloc(total, "boundary rules");
     for (Tunnel2Host& T : t) {
-      T.code = (uint32_t*)place((unsigned long long)T.N * 4);  // below the tunnel's own limit: 36 N is
+      T.code = (uint32_t*)place((unsigned long long)T.N * 4);
       T.qCoef = place((unsigned long long)T.qCap * 16 * bpp);
+      T.prev = place(9ull * bpp * (unsigned long long)T.N);
     }
   } catch (const AllocError&) {
     for (void* q : taken) dev.release(q);
     for (Tunnel2Host& T : t) {
       T.code = nullptr;
-      T.qCoef = nullptr;
+      T.qCoef = T.prev = nullptr;
     }
   }
 }
@@ -511,7 +518,7 @@ bool Cells2DBatch::run_partials() {
 }
 
 // n steps from parity par, an odd number at most blockK per launch; the force partials of up to
-// runSteps steps are summed together.
+// runSteps steps are summed together. allowSample 0: a trial, whose state is restored after it.
 void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
   const bool sampled = allowSample && samples_force();
   const bool ex = arithmetic == CELLS_ARITH_EXACT;
@@ -533,12 +540,15 @@ void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
     if (sampled) a.k = std::min(a.k, runSteps - a.j0);
     if (a.k % 2 == 0) a.k--;
     a.par = par;
+    n -= a.k;
+    a.last = n == 0 && allowSample;
     check_cuda(ex ? exact::launch_block2(prec, a, dev.stream) : fast::launch_block2(prec, a, dev.stream),
                "block step kernel");
     dev.launches++;
     a.first = false;
     par ^= 1;
-    n -= a.k;
+    if (a.last)
+      for (Tunnel2Host& T : t) T.prevValid = a.k > 1;
     a.j0 += a.k;
     if (sampled && (n == 0 || a.j0 == runSteps)) {
       check_cuda(fast::launch_sum_samples2(dTunnels, dLayout, (int)t.size(), runPartials, nBlockTiles, a.j0, par,
@@ -557,6 +567,8 @@ void Cells2DBatch::launch_raw(int64_t n, int par, int allowSample) {
     launch_blocks(n, par, allowSample);
     return;
   }
+  if (allowSample)
+    for (Tunnel2Host& T : t) T.prevValid = false;
   Step2Launch a;
   a.tunnels = dTunnels;
   a.tileTunnel = dTileTunnel;
@@ -1053,6 +1065,7 @@ int cells2d_init_field(Cells2D* h, const float* macro4n) {
   }
   b->dev.sync();
   T.step = 0;
+  T.prevValid = false;  // both buffers hold the new flow
   // a new flow clears the divergence status, as recoverFromBlowup's re-init starts over
   b->write_state(h->k, 1 | 2 | 4 | 8);
   T.forceSamplesRead = 0;
