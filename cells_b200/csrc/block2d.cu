@@ -129,9 +129,10 @@ __device__ __forceinline__ void write_links2(Link2<R>* links, int pos, uint32_t 
   }
 }
 
-// One link of a step: the pulled value goes where the pull reads it -- the cell is that place's only reader;
-// a slip row that mirrors a solid's population reads one that points out of the grid, which no link writes --
-// and the momentum exchange f_j + f_i is returned.
+// One link of a step: the pulled value goes where the pull reads it, and the momentum exchange f_j + f_i is
+// returned. The cell is that place's only reader: the place is solid or outside the grid (cells at the seam of a
+// side that is periodic alone are not listed), and a slip row that mirrors a solid's population reads one that
+// points out of the grid, which no link writes.
 template <class S, class R>
 __device__ __forceinline__ R link2(const Link2<R>& L, S* cur) {
   const uint32_t rule = (L.b >> 15) & 7u;
@@ -245,13 +246,20 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
   int nLinks = 0;
   if constexpr (LIST) {
     int mine[ROWS], sum = 0;
+    const bool left = T.left == X2_PERIODIC, right = T.right == X2_PERIODIC;
+    const bool bottom = T.bottom == Y2_PERIODIC, top = T.top == Y2_PERIODIC;
 #pragma unroll
     for (int m = 0; m < ROWS; m++) {
       const uint32_t w = fl[m] & CODE2_RULES;
       // only of cells that a step computes: their neighbours are places in the tile
-      const int r = threadIdx.y + m * BY;
+      const int r = threadIdx.y + m * BY, vy = oy + r;
       const bool steps = (int)threadIdx.x > cut && (int)threadIdx.x < RX - 1 - cut && r > cut && r < RY - 1 - cut;
-      mine[m] = !steps || (fl[m] & CODE2_SOLID) ? 0 : __popc((w | w >> 1 | w >> 2) & 0x249249u);
+      // With one side of an axis periodic, the margin behind it continues the grid with cells whose own far side is
+      // a wall or open: what they would pull from there is a real cell in the tile, no place for a link's value.
+      // The cells on both sides of that seam keep their rules.
+      const bool seam = (left != right && (left ? vx == -1 || vx == 0 : vx == W - 1 || vx == W)) ||
+                        (bottom != top && (bottom ? vy == -1 || vy == 0 : vy == H - 1 || vy == H));
+      mine[m] = !steps || seam || (fl[m] & CODE2_SOLID) ? 0 : __popc((w | w >> 1 | w >> 2) & 0x249249u);
       sum += mine[m];
     }
     int incl = sum;
