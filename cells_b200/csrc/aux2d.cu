@@ -2,6 +2,8 @@
 // writer. Reference: src/shaders/aux.ts:14-194. They run once per set_sdf / init_field / readback,
 // not per step, so they use a flat one-thread-per-cell launch. Compiled with -fmad=false: the
 // equilibria they write round exactly as the reference's expressions state.
+#include <type_traits>
+
 #include "kernels2d.h"
 
 namespace cells {
@@ -33,13 +35,92 @@ __device__ __forceinline__ void wrap2a(const AuxLaunch2& a, int& x, int& y) {
   if (y >= a.H && a.top == Y2_PERIODIC) y -= a.H;
 }
 
-// flagsShader, src/shaders/aux.ts:22-88
+// The word of a fluid cell with flags fl: the rules of pullSlow (src/shaders/step.ts:119-175) for every flagged
+// direction (Rule2), its Bouzidi coefficients into qCoef. solid(x, y): whether a cell of the grid is solid. The loads
+// of all eight directions go out together.
+template <class R, class R2, class Solid>
+__device__ __forceinline__ uint32_t rules_of2(const AuxLaunch2& a, int x, int y, uint32_t fl, const float* __restrict__ sdf,
+                                              R2* __restrict__ qCoef, int qCap, const Solid& solid) {
+  const int W = a.W, H = a.H;
+  const int slot = (int)(fl >> BIDX2_SHIFT);
+  uint32_t w = ((fl & FLAG2_INLET) ? CODE2_INLET : 0u) | ((fl & FLAG2_OUTLET) ? CODE2_OUTLET : 0u) |
+               (slot ? CODE2_SLOT : 0u);
+  // an inlet (outlet) cell whose only flagged directions are the three that Zou-He replaces needs no rule
+  constexpr uint32_t kInletPlain = FLAG2_INLET | (1u << 1) | (1u << 5) | (1u << 8);
+  constexpr uint32_t kOutletPlain = FLAG2_OUTLET | (1u << 3) | (1u << 6) | (1u << 7);
+  if (fl == kInletPlain || fl == kOutletPlain) return w;
+  // whether the source of each flagged direction is solid, its SDF, and whether there is fluid on the other side
+  const R dF = (R)sdf[(long long)y * W + x];
+  bool source[Q2], behind[Q2];
+  float dSource[Q2];
+#pragma unroll
+  for (int i = 1; i < Q2; i++) {
+    source[i] = behind[i] = false;
+    dSource[i] = 0.0f;
+    int sx = x - cx2(i), sy = y - cy2(i), nx = x + cx2(i), ny = y + cy2(i);
+    wrap2a(a, sx, sy);
+    wrap2a(a, nx, ny);
+    if ((fl & (1u << i)) && sx >= 0 && sx < W && sy >= 0 && sy < H) {
+      source[i] = solid(sx, sy);
+      dSource[i] = sdf[(long long)sy * W + sx];
+      behind[i] = nx >= 0 && nx < W && ny >= 0 && ny < H && !solid(nx, ny);
+    }
+  }
+#pragma unroll
+  for (int i = 1; i < Q2; i++) {
+    if (!(fl & (1u << i))) continue;
+    int sx = x - cx2(i), sy = y - cy2(i);
+    wrap2a(a, sx, sy);
+    const bool inX = sx >= 0 && sx < W, inY = sy >= 0 && sy < H;
+    uint32_t rule = RULE2_BOUNCE;
+    if (inX && inY) {
+      if (!source[i]) {
+        rule = RULE2_PULL;
+      } else if (slot == 0 || slot > qCap) {
+        w |= CODE2_GENERAL;
+      } else {
+        const R dS = (R)dSource[i];
+        const R den = (dF - dS) < (R)1e-6 ? (R)1e-6 : (dF - dS);
+        R q = dF / den;
+        q = q < (R)1e-3 ? (R)1e-3 : (R(1) < q ? R(1) : q);
+        R2 c;
+        c.x = R(2) * q;
+        c.y = R(0);
+        if (q < R(0.5)) {
+          rule = RULE2_BODY_0;
+          if (behind[i]) {
+            rule = RULE2_BODY_N;
+            c.y = R(1) - R(2) * q;
+          }
+        } else {
+          rule = RULE2_BODY_H;
+          c.y = (R(2) * q - R(1)) / (R(2) * q);
+        }
+        qCoef[(long long)(slot - 1) * 8 + (i - 1)] = c;
+      }
+    } else if (!inY) {
+      const int mode = sy < 0 ? a.bottom : a.top;
+      if (mode == Y2_SLIP) rule = inX ? RULE2_SLIP : RULE2_SLIP_HERE;
+      if (mode == Y2_MOVING) rule = RULE2_MOVING;
+    }
+    w |= rule << (3 * (i - 1));
+  }
+  if (w & CODE2_GENERAL) w &= ~CODE2_RULES;
+  return w;
+}
+
+// flagsShader, src/shaders/aux.ts:22-88, and the block kernel's rules with it: a rebuild waits for the latency of
+// this pass on a small grid and for its memory on a large one, and a kernel of its own for the rules added to both.
+// us, without rules / with a kernel of their own / here: setSdf of 400x100 41.7 / 49.0 / 43.6, brush with a
+// rebuild on 4000x1000 117 / 142 / 122. Six blocks per SM for the cells without a boundary: 152 with the 65
+// registers that the rules would take.
 template <class C>
-__global__ void flags2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, uint32_t* __restrict__ flags,
-                              typename C::S* __restrict__ fA, typename C::S* __restrict__ fB,
-                              const float4* __restrict__ mac, unsigned* __restrict__ counter,
-                              typename C::S* __restrict__ prev, int older) {
+__global__ void __launch_bounds__(256, 6)
+    flags2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, uint32_t* __restrict__ flags,
+                  typename C::S* __restrict__ fA, typename C::S* __restrict__ fB, const float4* __restrict__ mac,
+                  unsigned* __restrict__ counter, typename C::S* __restrict__ prev, int older, Rules2 rules) {
   using R = typename C::R;
+  using R2 = std::conditional_t<sizeof(R) == 4, float2, double2>;
   const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= a.N) return;
   const int W = a.W, H = a.H;
@@ -57,6 +138,7 @@ __global__ void flags2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, uint3
       for (int i = 0; i < Q2; i++) f[i * (long long)a.N + idx] = prev[i * (long long)a.N + idx];
     }
     flags[idx] = FLAG2_SOLID;
+    if (rules.code) rules.code[idx] = CODE2_SOLID;
     return;
   }
   uint32_t bits = 0;
@@ -80,6 +162,7 @@ __global__ void flags2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, uint3
     if (slot < (1u << (32 - BIDX2_SHIFT))) bits |= slot << BIDX2_SHIFT;
   }
   flags[idx] = bits;
+  if (rules.code) rules.code[idx] = bits ? rules_of2<R>(a, x, y, bits, sdf, (R2*)rules.qCoef, rules.qCap, solidAt) : 0u;
   if ((old & FLAG2_SOLID) != 0u) {
     R rho = R(0), ux = R(0), uy = R(0), n = R(0);
     for (int i = 1; i < Q2; i++) {
@@ -109,69 +192,24 @@ __global__ void flags2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, uint3
   }
 }
 
-// The rules of pullSlow (src/shaders/step.ts:119-175) for every flagged direction, as words (Rule2).
+// The words of a box's cells (which may reach one cell over the grid's edges, to its other side) after an edit of the
+// SDF that leaves the flags.
 template <class R, class R2>
-__global__ void rules2_kernel(AuxLaunch2 a, const float* __restrict__ sdf, const uint32_t* __restrict__ flags,
-                              uint32_t* __restrict__ code, R2* __restrict__ qCoef, int qCap) {
-  const long long idx = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= a.N) return;
+__global__ void rules2_kernel(AuxLaunch2 a, Box2 box, const float* __restrict__ sdf, const uint32_t* __restrict__ flags,
+                              Rules2 rules) {
+  const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+  if (t >= (long long)box.w * box.h) return;
+  const int by = (int)(t / box.w);
+  int x = box.x0 + (int)(t - (long long)by * box.w), y = box.y0 + by;
+  // over every edge: with one side periodic, the cells behind it have links into the box as well
+  x += x < 0 ? a.W : (x >= a.W ? -a.W : 0);
+  y += y < 0 ? a.H : (y >= a.H ? -a.H : 0);
+  const long long idx = (long long)y * a.W + x;
   const uint32_t fl = flags[idx];
-  if (fl == 0u || (fl & FLAG2_SOLID)) {
-    code[idx] = fl == 0u ? 0u : CODE2_SOLID;
-    return;
-  }
-  const int W = a.W, H = a.H;
-  const int y = (int)(idx / W);
-  const int x = (int)(idx - (long long)y * W);
-  const int slot = (int)(fl >> BIDX2_SHIFT);
-  uint32_t w = ((fl & FLAG2_INLET) ? CODE2_INLET : 0u) | ((fl & FLAG2_OUTLET) ? CODE2_OUTLET : 0u) |
-               (slot ? CODE2_SLOT : 0u);
-  // an inlet (outlet) cell whose only flagged directions are the three that Zou-He replaces needs no rule
-  constexpr uint32_t kInletPlain = FLAG2_INLET | (1u << 1) | (1u << 5) | (1u << 8);
-  constexpr uint32_t kOutletPlain = FLAG2_OUTLET | (1u << 3) | (1u << 6) | (1u << 7);
-  for (int i = 1; i < Q2 && fl != kInletPlain && fl != kOutletPlain; i++) {
-    if (!(fl & (1u << i))) continue;
-    int sx = x - cx2(i), sy = y - cy2(i);
-    wrap2a(a, sx, sy);
-    const bool inX = sx >= 0 && sx < W, inY = sy >= 0 && sy < H;
-    uint32_t rule = RULE2_BOUNCE;
-    if (inX && inY) {
-      const long long s = (long long)sy * W + sx;
-      if ((flags[s] & FLAG2_SOLID) == 0u) {
-        rule = RULE2_PULL;
-      } else if (slot == 0 || slot > qCap) {
-        w |= CODE2_GENERAL;
-      } else {
-        const R dF = (R)sdf[idx], dS = (R)sdf[s];
-        const R den = (dF - dS) < (R)1e-6 ? (R)1e-6 : (dF - dS);
-        R q = dF / den;
-        q = q < (R)1e-3 ? (R)1e-3 : (R(1) < q ? R(1) : q);
-        R2 c;
-        c.x = R(2) * q;
-        c.y = R(0);
-        if (q < R(0.5)) {
-          rule = RULE2_BODY_0;
-          int nx = x + cx2(i), ny = y + cy2(i);
-          wrap2a(a, nx, ny);
-          if (nx >= 0 && nx < W && ny >= 0 && ny < H && (flags[(long long)ny * W + nx] & FLAG2_SOLID) == 0u) {
-            rule = RULE2_BODY_N;
-            c.y = R(1) - R(2) * q;
-          }
-        } else {
-          rule = RULE2_BODY_H;
-          c.y = (R(2) * q - R(1)) / (R(2) * q);
-        }
-        qCoef[(long long)(slot - 1) * 8 + (i - 1)] = c;
-      }
-    } else if (!inY) {
-      const int mode = sy < 0 ? a.bottom : a.top;
-      if (mode == Y2_SLIP) rule = inX ? RULE2_SLIP : RULE2_SLIP_HERE;
-      if (mode == Y2_MOVING) rule = RULE2_MOVING;
-    }
-    w |= rule << (3 * (i - 1));
-  }
-  if (w & CODE2_GENERAL) w &= ~CODE2_RULES;
-  code[idx] = w;
+  if (fl == 0u || (fl & FLAG2_SOLID)) return;  // no rules
+  rules.code[idx] = rules_of2<R>(a, x, y, fl, sdf, (R2*)rules.qCoef, rules.qCap, [&](int qx, int qy) {
+    return (flags[(long long)qy * a.W + qx] & FLAG2_SOLID) != 0u;
+  });
 }
 
 // initShader, src/shaders/aux.ts:92-111
@@ -292,20 +330,22 @@ __global__ void set_state2_kernel(DevState2* st, int which, unsigned step, doubl
     }                                                    \
   } while (0)
 
-cudaError_t launch_rules2(int precision, const AuxLaunch2& a, const float* sdf, const uint32_t* flags, uint32_t* code,
-                          void* qCoef, int qCap, cudaStream_t s) {
+cudaError_t launch_rules2(int precision, const AuxLaunch2& a, const Box2& box, const float* sdf, const uint32_t* flags,
+                          const Rules2& rules, cudaStream_t s) {
+  const unsigned blocks = blocks_for2((long long)box.w * box.h, 256);
   if (precision == 0)
-    rules2_kernel<float, float2><<<blocks_for2(a.N, 256), 256, 0, s>>>(a, sdf, flags, code, (float2*)qCoef, qCap);
+    rules2_kernel<float, float2><<<blocks, 256, 0, s>>>(a, box, sdf, flags, rules);
   else
-    rules2_kernel<double, double2><<<blocks_for2(a.N, 256), 256, 0, s>>>(a, sdf, flags, code, (double2*)qCoef, qCap);
+    rules2_kernel<double, double2><<<blocks, 256, 0, s>>>(a, box, sdf, flags, rules);
   return cudaGetLastError();
 }
 
 cudaError_t launch_flags2(int precision, const AuxLaunch2& a, const float* sdf, uint32_t* flags, void* fA, void* fB,
-                          const float4* mac, unsigned* counter, void* prev, int older, cudaStream_t s) {
+                          const float4* mac, unsigned* counter, void* prev, int older, const Rules2& rules,
+                          cudaStream_t s) {
   CELLS2_DISPATCH(precision, (flags2_kernel<C><<<blocks_for2(a.N, 256), 256, 0, s>>>(
                                  a, sdf, flags, (typename C::S*)fA, (typename C::S*)fB, mac, counter,
-                                 (typename C::S*)prev, older)));
+                                 (typename C::S*)prev, older, rules)));
   return cudaGetLastError();
 }
 

@@ -6,7 +6,7 @@
 //
 // Boundary rules read within one cell of their own, so they need nothing beyond the margin; a periodic
 // seam is a margin loaded from the other side. What a flagged direction pulls is resolved per cell into
-// a rule word and Bouzidi coefficients when the SDF is set (rules2_kernel), because evaluating the
+// a rule word and Bouzidi coefficients when the SDF is set (rules_of2), because evaluating the
 // general rules -- eight directions with dependent flag and SDF loads -- took most of a step: 400x100
 // cylinder 5.0 us a step with them. The arithmetic is the one-step kernel's (step2d.cuh); k is odd, so
 // a launch ends in the other population buffer as a single step does.

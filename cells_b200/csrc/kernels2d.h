@@ -72,17 +72,28 @@ struct AuxLaunch2 {
   double fx, fy;
 };
 
-// flagsShader (src/shaders/aux.ts:22-88): flags with force slots from *counter (zeroed first) and
-// the refill of uncovered cells from mac.
+// The block kernel's rule words and Bouzidi coefficients (Tunnel2::code, qCoef); cells whose force slot exceeds qCap
+// keep the general rules. code NULL: there are none.
+struct Rules2 {
+  uint32_t* code;
+  void* qCoef;
+  int qCap;
+};
+// flagsShader (src/shaders/aux.ts:22-88): flags with force slots from *counter (zeroed first), the rules that follow
+// from them, and the refill of uncovered cells from mac.
 // A cell that becomes solid keeps the populations of the last step and of the one before it, one in each buffer.
 // prev: those of the step before it, where the buffer that should hold them (older: 0 fA, 1 fB) holds an earlier
 // step because the last launch took several; else NULL. It is kept in step with the refill of uncovered cells.
 cudaError_t launch_flags2(int precision, const AuxLaunch2& a, const float* sdf, uint32_t* flags, void* fA, void* fB,
-                          const float4* mac, unsigned* counter, void* prev, int older, cudaStream_t s);
-// The block kernel's rule words and Bouzidi coefficients from the flags and the SDF; cells whose force
-// slot exceeds qCap keep the general rules.
-cudaError_t launch_rules2(int precision, const AuxLaunch2& a, const float* sdf, const uint32_t* flags, uint32_t* code,
-                          void* qCoef, int qCap, cudaStream_t s);
+                          const float4* mac, unsigned* counter, void* prev, int older, const Rules2& rules,
+                          cudaStream_t s);
+// Cells of a tunnel; x0 and y0 may be -1 and the far ends one beyond the grid: its other side.
+struct Box2 {
+  int x0, y0, w, h;
+};
+// The rules of a box's cells from the flags and the SDF, for edits of the SDF that leave the flags.
+cudaError_t launch_rules2(int precision, const AuxLaunch2& a, const Box2& box, const float* sdf, const uint32_t* flags,
+                          const Rules2& rules, cudaStream_t s);
 // initShader (src/shaders/aux.ts:92-111): both buffers to feq(rho, ux, uy) of mac.
 cudaError_t launch_init2(int precision, const AuxLaunch2& a, const float4* mac, void* fA, void* fB, cudaStream_t s);
 // macroShader (src/shaders/aux.ts:115-140); sets status bit 1 on a non-finite value.

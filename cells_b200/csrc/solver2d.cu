@@ -153,7 +153,7 @@ struct Cells2DBatch : HandleBase {
   void upload_tunnel(int k);
   void write_state(int k, int which);
   void rebuild_flags(int k);
-  void resolve_rules(int k);
+  void resolve_rules(int k, const Box2& box);
   AuxLaunch2 aux(int k) const;
   void launch_raw(int64_t n, int par, int allowSample);
   void launch_steps(int64_t n);
@@ -334,10 +334,9 @@ void Cells2DBatch::rebuild_flags(int k) {
   check_cuda(launch_macro2(prec, a, T.f[parity], T.flags, T.macro, T.st, dev.stream), "macro kernel");
   dev.memset0(dCounter, sizeof(unsigned));
   check_cuda(launch_flags2(prec, a, T.sdf, T.flags, T.f[0], T.f[1], T.macro, dCounter, T.prevValid ? T.prev : nullptr,
-                           parity ^ 1, dev.stream),
+                           parity ^ 1, Rules2{T.code, T.qCoef, T.qCap}, dev.stream),
              "flags kernel");
   dev.launches += 2;
-  resolve_rules(k);
 }
 
 // The block kernel's tables: one buffer for the batch, or, where that exceeds the largest buffer that a tunnel's
@@ -391,11 +390,11 @@ unsigned long long Cells2DBatch::buffer_limit() const {
   return limit;
 }
 
-// The block kernel's rules follow the flags and the SDF.
-void Cells2DBatch::resolve_rules(int k) {
+// The rules of a box's cells follow an edit of the SDF that leaves the flags.
+void Cells2DBatch::resolve_rules(int k, const Box2& box) {
   Tunnel2Host& T = t[(size_t)k];
   if (!T.code) return;
-  check_cuda(launch_rules2(prec, aux(k), T.sdf, T.flags, T.code, T.qCoef, T.qCap, dev.stream), "rules kernel");
+  check_cuda(launch_rules2(prec, aux(k), box, T.sdf, T.flags, Rules2{T.code, T.qCoef, T.qCap}, dev.stream), "rules kernel");
   dev.launches++;
 }
 
@@ -1004,8 +1003,9 @@ int cells2d_read_sdf(Cells2D* h, float* out, size_t n) {
   C2_CATCH(h, kAllocPrefix)
 }
 
-// the bounding box of brush (src/solver.ts:249-255), then the SDF kernel
-static void brush_one(Cells2D* h, double cx, double cy, double r, int erase) {
+// the bounding box of brush (src/solver.ts:249-255), then the SDF kernel. rules: the flags are not rebuilt after it,
+// and the links' fractions follow the SDF at once.
+static void brush_one(Cells2D* h, double cx, double cy, double r, int erase, bool rules) {
   Tunnel2Host& T = h->T();
   const int pad = 2;
   const int x0 = std::max(0, (int)std::floor(cx - r - pad));
@@ -1027,13 +1027,16 @@ static void brush_one(Cells2D* h, double cx, double cy, double r, int erase) {
                            y1 - y0 + 1, h->b->dev.stream),
              "brush kernel");
   h->b->dev.launches++;
-  h->b->resolve_rules(h->k);  // the links' fractions follow the SDF at once, the flags on the next rebuild
+  if (rules) {  // of the cells that have a link with a node of the box
+    const int w = std::min(T.W, x1 - x0 + 3), hh = std::min(T.H, y1 - y0 + 3);
+    h->b->resolve_rules(h->k, Box2{w == T.W ? 0 : x0 - 1, hh == T.H ? 0 : y0 - 1, w, hh});
+  }
 }
 
 int cells2d_brush(Cells2D* h, double cx, double cy, double r, int erase, int rebuild) {
   if (!h) return CELLS_E_INVALID;
   C2_TRY
-  brush_one(h, cx, cy, r, erase);
+  brush_one(h, cx, cy, r, erase, !rebuild);
   if (rebuild) h->b->rebuild_flags(h->k);
   C2_CATCH(h, kAllocPrefix)
 }
@@ -1041,7 +1044,7 @@ int cells2d_brush(Cells2D* h, double cx, double cy, double r, int erase, int reb
 int cells2d_brush_stroke(Cells2D* h, const double* xy, size_t n_points, double r, int erase) {
   if (!h || (!xy && n_points)) return CELLS_E_INVALID;
   C2_TRY
-  for (size_t p = 0; p < n_points; p++) brush_one(h, xy[2 * p], xy[2 * p + 1], r, erase);
+  for (size_t p = 0; p < n_points; p++) brush_one(h, xy[2 * p], xy[2 * p + 1], r, erase, false);
   h->b->rebuild_flags(h->k);
   C2_CATCH(h, kAllocPrefix)
 }
