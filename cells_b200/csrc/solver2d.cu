@@ -28,6 +28,12 @@ constexpr int kGraphSteps2 = 100;
 constexpr int kPersistentChunk = 500;
 constexpr int kRunSteps2 = 126;  // most steps whose force partials wait for one sum: 18 launches of 7
 
+// A region of the block kernel, the steps K per launch, whether boundary links are listed, and the number of
+// tiles up to which it is taken.
+struct Region2 {
+  int x, y, rows, K, list, maxTiles;
+};
+
 struct Shape2 {
   int tx, ty;
 };
@@ -136,7 +142,14 @@ struct Cells2DBatch : HandleBase {
   double2* runPartials = nullptr;  // force partials of a run of runSteps steps
   int runSteps = 0;
   bool runPartialsOff = false;     // they did not fit
+  char* spare = nullptr;           // room for the layout and the force partials behind the rules
+  size_t spareBytes = 0, spareUsed = 0;
+  std::vector<void*> blockOwn;     // their own buffers where it does not suffice
+  static unsigned long long room(unsigned long long bytes) { return (bytes + 255) / 256 * 256; }
+  bool pick_region(Region2& r, int& K, long long& tiles) const;
+  unsigned long long partial_bytes(long long tiles, int K, int& steps) const;
   void alloc_rules();
+  void* block_alloc(size_t bytes, const char* what);
   unsigned long long buffer_limit() const;
   void choose_block();
   bool samples_force() const;
@@ -339,11 +352,61 @@ void Cells2DBatch::rebuild_flags(int k) {
   dev.launches += 2;
 }
 
-// The block kernel's tables: one buffer for the batch, or, where that exceeds the largest buffer that a tunnel's
-// caller allows, one for each table. A device without room for them steps one launch at a time.
+// The regions (Region2). us per step of one tunnel with a circle, FP32 [one step per launch before]:
+//                 64x64  128x128  300x80  400x100  500x140  700x180  1000x250  1500x400  2000x500
+//   32x24x1 K=7    1.96     2.05    2.04     2.50     3.60     5.79     10.77     24.40     40.76
+//   32x32x1 K=7    2.43     2.47    2.26     2.36     3.21     4.82      8.95     20.07     32.61
+//   64x32x2 K=7    3.26     3.44    2.88     3.06     3.02     3.04      5.42     12.17     19.14
+//   64x48x3 K=5    4.62     4.99    5.04     4.60     4.66     4.78      4.63     11.19     17.00
+//     no list      6.33     6.51    5.07     5.97     6.42     7.55      7.63     10.29     15.18
+//   [before        8.88     9.48    8.57    12.13    11.98    14.47     21.72     29.90     45.48]
+// and for 64 NACA tunnels with Smagorinsky 64x48x3 K=5 103 with a list, 95 without [117]. Tiles that are all
+// resident at once (148 SMs, one block each) step at the pace of the slowest, the one with the body: the
+// smallest region that gives one wave, and its links listed. With more waves the work counts: the margins
+// are computed twice, so (x - 2K)(y - 2K) / xy of it is kept, the region is the largest that shared memory
+// holds in two buffers, and the list's registers and barriers cost more than they save.
+// FP64: 32x24x2 K=7 2.70 (128x128), 3.58 (400x100); 32x32x2 K=7 3.11, 2.79; without a list K=5 5.15 (700x180),
+// 9.06 (1000x250), 129 (4000x1000), K=3 6.08, 8.58, 126 [9.09, 12.3, 15.9, 25.0, 312].
+constexpr int kWave2 = 148;
+constexpr Region2 kRegions32[] = {{32, 24, 1, 7, 1, kWave2}, {32, 32, 1, 7, 1, kWave2}, {64, 32, 2, 7, 1, kWave2},
+                                  {64, 48, 3, 5, 1, kWave2}, {64, 48, 3, 5, 0, INT_MAX}};
+constexpr Region2 kRegions64[] = {{32, 24, 2, 7, 1, kWave2}, {32, 32, 2, 7, 1, kWave2}, {32, 32, 2, 5, 0, 2 * kWave2},
+                                  {32, 32, 2, 3, 0, INT_MAX}};
+
+// The block kernel's region and step count for the batch's grids and boundary modes, and its number of tiles. False
+// where there are none.
+bool Cells2DBatch::pick_region(Region2& r, int& K, long long& tiles) const {
+  int limit = kBlockSteps2;
+  for (const Tunnel2Host& T : t) {
+    // a periodic margin is loaded from the other side once
+    if (T.cfg.left == CELLS_X_PERIODIC || T.cfg.right == CELLS_X_PERIODIC) limit = std::min(limit, T.W);
+    if (T.cfg.bottom == CELLS_Y_PERIODIC || T.cfg.top == CELLS_Y_PERIODIC) limit = std::min(limit, T.H);
+  }
+  limit = (limit - 1) | 1;  // the largest odd number up to it
+  if (limit < 3) return false;
+  for (const Region2* c = prec == CELLS_FP64 ? kRegions64 : kRegions32;; c++) {
+    r = *c;
+    K = std::min(r.K, limit);
+    tiles = 0;
+    for (const Tunnel2Host& T : t)
+      tiles += (long long)((T.W + r.x - 2 * K - 1) / (r.x - 2 * K)) * ((T.H + r.y - 2 * K - 1) / (r.y - 2 * K));
+    if (tiles <= r.maxTiles || r.maxTiles == INT_MAX) break;
+  }
+  return tiles <= INT_MAX;
+}
+
+// What a run's force partials take for `tiles` tiles, and its steps; 0 where the buffer limit leaves no room.
+unsigned long long Cells2DBatch::partial_bytes(long long tiles, int K, int& steps) const {
+  const unsigned long long perStep = (unsigned long long)tiles * sizeof(double2);
+  steps = (int)std::min<unsigned long long>(kRunSteps2, buffer_limit() / perStep);
+  return steps < K ? 0 : perStep * (unsigned)steps;
+}
+
+// The block kernel's tables: one buffer for the batch, the layout and a run's force partials behind them, or, where
+// that exceeds the largest buffer that a tunnel's caller allows, one for each table. A device without room for them
+// steps one launch at a time.
 void Cells2DBatch::alloc_rules() {
   if (dev.fake) return;
-  auto room = [](unsigned long long bytes) { return (bytes + 255) / 256 * 256; };
   unsigned long long total = 0, limit = buffer_limit();
   for (Tunnel2Host& T : t) {
     // coefficient slots for the cells around a body: a few times the grid's outline (further body cells
@@ -353,6 +416,17 @@ void Cells2DBatch::alloc_rules() {
       T.qCap = (int)std::min<unsigned long long>((unsigned long long)T.qCap, T.cfg.max_buffer_bytes / (16 * bpp));
     total += room((unsigned long long)T.N * 4) + room((unsigned long long)T.qCap * 16 * bpp) +
              room(9ull * bpp * (unsigned long long)T.N);
+  }
+  Region2 r;
+  int K, steps;
+  long long tiles;
+  if (blockWanted && pick_region(r, K, tiles))
+    spareBytes = room(t.size() * sizeof(Block2Tunnel)) + room((unsigned long long)tiles * sizeof(unsigned short)) +
+                 (samples_force() ? room(partial_bytes(tiles, K, steps)) : 0);
+  total += spareBytes;
+  if (total > limit) {
+    total -= spareBytes;
+    spareBytes = 0;
   }
   if (total + (1u << 22) > dev.free_bytes()) return;
   std::vector<void*> taken;
@@ -373,7 +447,9 @@ void Cells2DBatch::alloc_rules() {
       T.qCoef = place((unsigned long long)T.qCap * 16 * bpp);
       T.prev = place(9ull * bpp * (unsigned long long)T.N);
     }
+    spare = p;
   } catch (const AllocError&) {
+    spareBytes = 0;
     for (void* q : taken) dev.release(q);
     for (Tunnel2Host& T : t) {
       T.code = nullptr;
@@ -398,57 +474,15 @@ void Cells2DBatch::resolve_rules(int k, const Box2& box) {
   dev.launches++;
 }
 
-// A region of the block kernel, the steps K per launch, whether boundary links are listed, and the number of
-// tiles up to which it is taken.
-struct Region2 {
-  int x, y, rows, K, list, maxTiles;
-};
-// us per step of one tunnel with a circle, FP32 [one step per launch before]:
-//                 64x64  128x128  300x80  400x100  500x140  700x180  1000x250  1500x400  2000x500
-//   32x24x1 K=7    1.96     2.05    2.04     2.50     3.60     5.79     10.77     24.40     40.76
-//   32x32x1 K=7    2.43     2.47    2.26     2.36     3.21     4.82      8.95     20.07     32.61
-//   64x32x2 K=7    3.26     3.44    2.88     3.06     3.02     3.04      5.42     12.17     19.14
-//   64x48x3 K=5    4.62     4.99    5.04     4.60     4.66     4.78      4.63     11.19     17.00
-//     no list      6.33     6.51    5.07     5.97     6.42     7.55      7.63     10.29     15.18
-//   [before        8.88     9.48    8.57    12.13    11.98    14.47     21.72     29.90     45.48]
-// and for 64 NACA tunnels with Smagorinsky 64x48x3 K=5 103 with a list, 95 without [117]. Tiles that are all
-// resident at once (148 SMs, one block each) step at the pace of the slowest, the one with the body: the
-// smallest region that gives one wave, and its links listed. With more waves the work counts: the margins
-// are computed twice, so (x - 2K)(y - 2K) / xy of it is kept, the region is the largest that shared memory
-// holds in two buffers, and the list's registers and barriers cost more than they save.
-// FP64: 32x24x2 K=7 2.70 (128x128), 3.58 (400x100); 32x32x2 K=7 3.11, 2.79; without a list K=5 5.15 (700x180),
-// 9.06 (1000x250), 129 (4000x1000), K=3 6.08, 8.58, 126 [9.09, 12.3, 15.9, 25.0, 312].
-constexpr int kWave2 = 148;
-constexpr Region2 kRegions32[] = {{32, 24, 1, 7, 1, kWave2}, {32, 32, 1, 7, 1, kWave2}, {64, 32, 2, 7, 1, kWave2},
-                                  {64, 48, 3, 5, 1, kWave2}, {64, 48, 3, 5, 0, INT_MAX}};
-constexpr Region2 kRegions64[] = {{32, 24, 2, 7, 1, kWave2}, {32, 32, 2, 7, 1, kWave2}, {32, 32, 2, 5, 0, 2 * kWave2},
-                                  {32, 32, 2, 3, 0, INT_MAX}};
-
 // The block kernel's region and step count, its tiles numbered tunnel by tunnel, and the tile -> tunnel map.
 void Cells2DBatch::choose_block() {
   const bool on = blockOn;
   blockOn = false;
   if (!t[0].code) return;
-  int limit = kBlockSteps2;
-  for (const Tunnel2Host& T : t) {
-    // a periodic margin is loaded from the other side once
-    if (T.cfg.left == CELLS_X_PERIODIC || T.cfg.right == CELLS_X_PERIODIC) limit = std::min(limit, T.W);
-    if (T.cfg.bottom == CELLS_Y_PERIODIC || T.cfg.top == CELLS_Y_PERIODIC) limit = std::min(limit, T.H);
-  }
-  limit = (limit - 1) | 1;  // the largest odd number up to it
-  if (limit < 3) return;
   Region2 r = {};
   int K = 0;
   long long tiles = 0;
-  for (const Region2* c = prec == CELLS_FP64 ? kRegions64 : kRegions32;; c++) {
-    r = *c;
-    K = std::min(r.K, limit);
-    tiles = 0;
-    for (const Tunnel2Host& T : t)
-      tiles += (long long)((T.W + r.x - 2 * K - 1) / (r.x - 2 * K)) * ((T.H + r.y - 2 * K - 1) / (r.y - 2 * K));
-    if (tiles <= r.maxTiles || r.maxTiles == INT_MAX) break;
-  }
-  if (tiles > INT_MAX) return;
+  if (!pick_region(r, K, tiles)) return;
   if (dLayout && r.x == regionX && r.y == regionY && K == blockK && r.list == blockList) {
     blockOn = true;
     return;
@@ -466,19 +500,17 @@ void Cells2DBatch::choose_block() {
     map.insert(map.end(), (size_t)L.tiles, (unsigned short)k);
   }
   if (on) dev.sync();  // launches that read the layout before
-  if (dLayout) dev.release(dLayout);
-  if (dBlockTiles) dev.release(dBlockTiles);
-  if (runPartials) dev.release(runPartials);
+  for (void* p : blockOwn) dev.release(p);
+  blockOwn.clear();
+  spareUsed = 0;
   dLayout = nullptr;
   dBlockTiles = nullptr;
   runPartials = nullptr;
   runPartialsOff = false;
   try {
-    dLayout = (Block2Tunnel*)dev.alloc(layout.size() * sizeof(Block2Tunnel), "block layout");
-    dBlockTiles = (unsigned short*)dev.alloc(map.size() * sizeof(unsigned short), "block tile map");
+    dBlockTiles = (unsigned short*)block_alloc(map.size() * sizeof(unsigned short), "block tile map");
+    dLayout = (Block2Tunnel*)block_alloc(layout.size() * sizeof(Block2Tunnel), "block layout");
   } catch (const AllocError&) {
-    if (dLayout) dev.release(dLayout);
-    dLayout = nullptr;
     return;  // one step per launch
   }
   regionX = r.x;
@@ -491,6 +523,18 @@ void Cells2DBatch::choose_block() {
   dev.h2d(dBlockTiles, map.data(), map.size() * sizeof(unsigned short));
   dev.sync();  // the host vectors die here
   blockOn = true;
+  if (samples_force()) run_partials();  // here, not in the first run
+}
+
+// A buffer of the block kernel's layout: behind the rules while it fits there, else one of its own.
+void* Cells2DBatch::block_alloc(size_t bytes, const char* what) {
+  if (spareUsed + room(bytes) <= spareBytes) {
+    void* p = spare + spareUsed;
+    spareUsed += (size_t)room(bytes);
+    return p;
+  }
+  blockOwn.push_back(dev.alloc(bytes, what));
+  return blockOwn.back();
 }
 
 bool Cells2DBatch::samples_force() const {
@@ -502,17 +546,12 @@ bool Cells2DBatch::samples_force() const {
 bool Cells2DBatch::run_partials() {
   if (runPartials) return true;
   if (runPartialsOff) return false;
-  const unsigned long long perStep = (unsigned long long)nBlockTiles * sizeof(double2);
-  runSteps = (int)std::min<unsigned long long>(kRunSteps2, buffer_limit() / perStep);
-  if (runSteps < blockK) {
-    runPartialsOff = true;
-    return false;
-  }
+  const unsigned long long bytes = partial_bytes(nBlockTiles, blockK, runSteps);
   try {
-    runPartials = (double2*)dev.alloc((size_t)(perStep * (unsigned)runSteps), "force partials of a run");
+    if (bytes) runPartials = (double2*)block_alloc((size_t)bytes, "force partials of a run");
   } catch (const AllocError&) {
-    runPartialsOff = true;
   }
+  runPartialsOff = !runPartials;
   return runPartials != nullptr;
 }
 

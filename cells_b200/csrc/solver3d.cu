@@ -171,6 +171,7 @@ void Cells3D::build_body_list() {
     links.meta = (int*)dev.alloc((size_t)cap * 4, "body links");
     links.cap = cap;
   }
+  if (nBody > 0 && cfg.force_every > 0) run_partials(kGraphSteps);  // here, not in the first run
   if (nBody > 0 && !dev.fake) {
     AuxLaunch3 a{W, H, D, (int)N, current_uin()};
     check_cuda(launch_links3(prec, a, bodyCells, nBody, flags, sdf, links, dev.stream), "links kernel");
@@ -199,19 +200,23 @@ void Cells3D::rebuild_flags() {
 // about 3.6 us of every sampled step). False when they would take too much memory.
 bool Cells3D::run_partials(int samples) {
   const size_t need = (size_t)samples * (size_t)(nBody > 0 ? fast::body_blocks3(nBody) : 0);
-  if (dev.fake || runPartialsOff || need * sizeof(double4) > kRunPartialBytes) return false;
+  size_t most = kRunPartialBytes / sizeof(double4);
+  if (cfg.max_buffer_bytes > 0) most = std::min<size_t>(most, (size_t)(cfg.max_buffer_bytes / sizeof(double4)));
+  if (dev.fake || runPartialsOff || need > most) return false;
   if (need > runPartialCap) {
+    // for as many body cells as the link tables hold, so that both grow together
+    const size_t cap = std::max(need, std::min(most, (size_t)samples * (size_t)fast::body_blocks3(links.cap)));
     dev.release(runPartials);
     runPartials = nullptr;
     runPartialCap = 0;
     argGen++;  // step graphs bake the address
     try {
-      runPartials = (double4*)dev.alloc(need * sizeof(double4), "force partials of a run");
+      runPartials = (double4*)dev.alloc(cap * sizeof(double4), "force partials of a run");
     } catch (const AllocError&) {
       runPartialsOff = true;
       return false;
     }
-    runPartialCap = need;
+    runPartialCap = cap;
   }
   return true;
 }
