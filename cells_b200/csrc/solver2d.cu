@@ -792,8 +792,16 @@ static Cells2DBatch* create_batch(const Cells2DConfig* cfgs, int count) {
       // takes them; on the top row direction 8's pull lands up to W - 1 elements past the nine
       // arrays, so each buffer carries W elements of padding (never used as a population)
       const size_t padBytes = (size_t)T.W * b->bpp;
-      T.f[0] = b->dev.alloc(fBytes + padBytes, "distribution buffer A");
-      T.f[1] = b->dev.alloc(fBytes + padBytes, "distribution buffer B");
+      if (b->dev.fake || cfgs[k].max_buffer_bytes > 0) {
+        T.f[0] = b->dev.alloc(fBytes + padBytes, "distribution buffer A");
+        T.f[1] = b->dev.alloc(fBytes + padBytes, "distribution buffer B");
+      } else {
+        // as one: every 2 MB begun, and every larger allocation, takes the device about 0.35 ms, and the tables of
+        // several steps per launch are one more (a batch of 32 tunnels: 47 ms apart, 38 as one)
+        const size_t each = (size_t)Cells2DBatch::room(fBytes + padBytes);
+        T.f[0] = b->dev.alloc(2 * each, "distribution buffers");
+        T.f[1] = (char*)T.f[0] + each;
+      }
       T.flags = (uint32_t*)b->dev.alloc((size_t)T.N * 4, "flags");
       T.sdf = (float*)b->dev.alloc((size_t)T.N * 4, "sdf");
       T.macro = (float4*)b->dev.alloc((size_t)T.N * 16, "macro");
