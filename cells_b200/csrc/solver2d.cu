@@ -154,7 +154,8 @@ struct Cells2DBatch : HandleBase {
   void choose_block();
   bool samples_force() const;
   bool run_partials();
-  void launch_blocks(int64_t n, int par, int allowSample);
+  int64_t block_steps(int64_t n, bool sampled) const;
+  void launch_blocks(int64_t n, int par, int allowSample, bool end);
 
   struct StepGraph {
     cudaGraphExec_t exec = nullptr;
@@ -556,8 +557,9 @@ bool Cells2DBatch::run_partials() {
 }
 
 // n steps from parity par, an odd number at most blockK per launch; the force partials of up to
-// runSteps steps are summed together. allowSample 0: a trial, whose state is restored after it.
-void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
+// runSteps steps are summed together. allowSample 0: a trial, whose state is restored after it. end: the run ends
+// with these steps.
+void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample, bool end) {
   const bool sampled = allowSample && samples_force();
   const bool ex = arithmetic == CELLS_ARITH_EXACT;
   Block2Launch a;
@@ -579,7 +581,7 @@ void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
     if (a.k % 2 == 0) a.k--;
     a.par = par;
     n -= a.k;
-    a.last = n == 0 && allowSample;
+    a.last = n == 0 && allowSample && end;
     check_cuda(ex ? exact::launch_block2(prec, a, dev.stream) : fast::launch_block2(prec, a, dev.stream),
                "block step kernel");
     dev.launches++;
@@ -599,11 +601,30 @@ void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample) {
   }
 }
 
+// How many of n steps the block kernel takes: all, or all but the one or two that no odd number of steps holds. A
+// launch of a single step costs it the margins and a load through shared memory: with samples it still beats
+// the one-step kernel (which counts its blocks), and on the small regions it does by the overlap of the launches.
+// us for 2 steps without samples, one-step / block: 128x128 11.8 / 10.2, 400x100 14.7 / 12.6; 1000x250 (64x48 with a
+// list) 19.7 / 22.9, 2000x500 39 / 64, 4000x1000 137 / 281; FP64 1000x250 (without a list) 21.9 / 30.4. With
+// samples: 1000x250 43 / 28, 4000x1000 383 / 295, FP64 620 / 533. Without a list FP32 needs a launch of K steps to
+// gain: 3 steps 2000x500 58.5 / 62.1, 4000x1000 205 / 234, 4 steps 78 / 82, 273 / 291, 8 steps 156 / 136, 545 / 503
+// (FP64 4000x1000, 3 steps 561 / 421).
+int64_t Cells2DBatch::block_steps(int64_t n, bool sampled) const {
+  if (sampled || (blockList && regionX * regionY < 64 * 48)) return n;
+  if (n < blockK && !blockList && prec == CELLS_FP32) return 0;
+  const int64_t full = n / blockK * blockK, rest = n - full;
+  return full + (rest < 3 ? 0 : (rest - 1) | 1);
+}
+
 // n steps from parity par on the device only (no host bookkeeping).
 void Cells2DBatch::launch_raw(int64_t n, int par, int allowSample) {
-  if (blockOn && n >= 2 && (!(allowSample && samples_force()) || run_partials())) {
-    launch_blocks(n, par, allowSample);
-    return;
+  if (blockOn && n >= 2) {
+    const bool sampled = allowSample && samples_force();
+    const int64_t m = !sampled || run_partials() ? block_steps(n, sampled) : 0;
+    if (m > 0) launch_blocks(m, par, allowSample, m == n);
+    par ^= (int)(m & 1);
+    n -= m;
+    if (n == 0) return;
   }
   if (allowSample)
     for (Tunnel2Host& T : t) T.prevValid = false;
@@ -1553,9 +1574,9 @@ int cells2d_batch_autotune(Cells2DBatch* b, int32_t trial_steps, Cells2DInfo* in
       float blockMs = 1e30f;
       b->choose_block();
       if (b->blockOn) {
-        b->launch_blocks(warm, par0, 0);
+        b->launch_blocks(warm, par0, 0, false);
         check_cuda(cudaEventRecord(b->dev.ev0, b->dev.stream), "cudaEventRecord");
-        b->launch_blocks(trial_steps, par0 ^ (warm & 1), 0);
+        b->launch_blocks(trial_steps, par0 ^ (warm & 1), 0, false);
         check_cuda(cudaEventRecord(b->dev.ev1, b->dev.stream), "cudaEventRecord");
         check_cuda(cudaEventSynchronize(b->dev.ev1), "cudaEventSynchronize");
         check_cuda(cudaEventElapsedTime(&blockMs, b->dev.ev0, b->dev.ev1), "cudaEventElapsedTime");

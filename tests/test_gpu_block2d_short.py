@@ -1,0 +1,40 @@
+"""Short 2D runs without force samples on grids of many tiles: steps that no launch of three or more takes go through
+the one-step kernel. Bit for bit against the oracle in the exact build, for every remainder, with a body drawn onto
+a slip wall after each run (solid cells keep what both buffers held, whichever kernel took the last steps)."""
+import numpy as np
+import pytest
+
+import cells_b200.geometry as g
+from cells_b200 import Solver
+from cells_b200.rng import perturbed_rest2
+from oracle.oracle import OracleSolver2D
+
+pytestmark = pytest.mark.gpu
+
+
+# FP32: 64x48 with a list, without one; FP64: 32x32 without a list, with 5 and with 3 steps
+@pytest.mark.parametrize("precision,size,K", [("fp32", (500, 300), 5), ("fp32", (905, 605), 5), ("fp64", (300, 200), 5),
+                                              ("fp64", (905, 605), 3)])
+def test_remainders(precision, size, K):
+    W, H = size
+    cfg = dict(left=2, right=2, bottom=2, top=2, tau=0.56, uIn=0.05, forceEvery=0)
+    s = Solver.create(width=W, height=H, precision=precision, exactArithmetic=True, **cfg)
+    o = OracleSolver2D(width=W, height=H, precision=precision, **cfg)
+    for x in (s, o):
+        sdf = g.empty_sdf(W, H)
+        g.add_circle(sdf, W, H, W / 4, H / 2, H / 9)
+        x.setSdf(sdf)
+        x.initField(perturbed_rest2(W, H, 1e-3))
+    for k, n in enumerate((2, 4, 6, 7, 9, 1, 12, 3)):
+        before = s.launchCount()
+        s.encodeSteps(n)
+        few = precision == "fp32" and W > 500 and n < K  # one by one
+        assert s.launchCount() - before == (n if few else n // K + (0, 1, 2, 1, 2)[n % K])
+        o.encodeSteps(n)
+        for x in (s, o):
+            x.brush(40 + 40 * k, H - 1 if k % 2 else 0, 3.3, False, True)
+    s.encodeSteps(5)
+    o.encodeSteps(5)
+    a, b = s.readPopulations(), np.ascontiguousarray(o.populations())
+    assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
+    s.destroy()
