@@ -41,7 +41,7 @@ struct Vec2T<double> {
 template <class C, int RX, int RY>
 struct TileSource2 {
   const typename C::S* p;  // population 0 of the cell
-  __device__ __forceinline__ typename C::R at(int pop, int, int, int dx, int dy) const {
+  __device__ __forceinline__ typename C::R at(int pop, long long, int, int, int dx, int dy) const {
     return (typename C::R)p[pop * (RX * RY) + dy * RX + dx];
   }
 };
@@ -59,10 +59,10 @@ __device__ __forceinline__ void rules2(uint32_t w, const Tunnel2& T, const Sourc
     if (rule == RULE2_PULL) continue;
     const int j = opp2(i);
     if (rule == RULE2_SLIP || rule == RULE2_SLIP_HERE) {
-      f[i] = src.at(mirror_y2(i), 0, 0, rule == RULE2_SLIP ? -cx2(i) : 0, 0);
+      f[i] = src.at(mirror_y2(i), 0, 0, 0, rule == RULE2_SLIP ? -cx2(i) : 0, 0);
       continue;
     }
-    const R fj = src.at(j, 0, 0, 0, 0);
+    const R fj = src.at(j, 0, 0, 0, 0, 0);
     R fi = fj;
     if (rule == RULE2_MOVING) {
       f[i] = fj + R(6) * w2<R>(i) * R(cx2(i)) * prm<R>(T, P2_ULID);
@@ -72,9 +72,9 @@ __device__ __forceinline__ void rules2(uint32_t w, const Tunnel2& T, const Sourc
       if (rule != RULE2_BODY_0) {
         const auto c = coef[i - 1];
         if (rule == RULE2_BODY_N)
-          fi = c.x * fj + c.y * src.at(j, 0, 0, cx2(i), cy2(i));
+          fi = c.x * fj + c.y * src.at(j, 0, 0, 0, cx2(i), cy2(i));
         else
-          fi = fj / c.x + c.y * src.at(i, 0, 0, 0, 0);
+          fi = fj / c.x + c.y * src.at(i, 0, 0, 0, 0, 0);
       }
       const R t = fj + fi;
       force[0] += R(cx2(j)) * t;
@@ -396,7 +396,7 @@ __global__ void __launch_bounds__(RX * RY / ROWS, 1)
         }
       }
       if constexpr (kExact2)
-        collide2<C>(T, xt, forcing, smagC2, H, u, y, f, o);
+        collide2<C>(T, xt, forcing, smagC2, H, u, y, f, [&](int i, R v) { o[i] = v; });
       else
         collide2_lean<R>(T, xt, forcing, smagC2, lambda, H, LIST ? parabolic : T.parabolic, u, y, f, o);
       if (j + 1 < k) {
