@@ -266,9 +266,10 @@ class Solver:
 
 
 class Batch2D:
-    """Independent D2Q9 tunnels of different sizes stepped together: one launch per step for all
-    of them (graph-replayed), or persistent launches, as the autotuner decides. ``tunnels[k]`` is
-    a Solver for the per-tunnel calls; step with ``step(n)`` / ``run(n)`` on the batch."""
+    """Independent D2Q9 tunnels of different sizes stepped together: up to seven steps of all of them per
+    launch, or one launch per step (graph-replayed) or persistent launches where the autotuner or
+    ``setLaunch`` chose them. ``tunnels[k]`` is a Solver for the per-tunnel calls; step with
+    ``step(n)`` / ``run(n)`` on the batch."""
 
     def __init__(self, configs: Sequence[dict]):
         cfgs = [_full_config(c) for c in configs]

@@ -392,7 +392,10 @@ int cells2d_read_sdf(Cells2D* h, float* out, size_t n);
 int cells2d_init_field(Cells2D* h, const float* macro4n);
 int cells2d_reset_forces(Cells2D* h);
 /* encodeSteps / encodeMacro / run (src/solver.ts:270-307); tunnels of a multi-tunnel batch step
- * with cells2d_batch_step. */
+ * with cells2d_batch_step. Single steps and runs go through kernels that round differently in fast
+ * arithmetic (see cells2d_batch_step): how a caller groups its steps then changes the populations by
+ * roundings of a step. In exact arithmetic they do not depend on it, nor with a workgroup_size; force
+ * samples are f64 sums whose order may depend on it. */
 int cells2d_step(Cells2D* h, int64_t n);
 int cells2d_update_macro(Cells2D* h);
 int cells2d_run(Cells2D* h, int64_t n, int64_t chunk);
@@ -430,7 +433,8 @@ void cells2d_batch_destroy(Cells2DBatch* b);
 int cells2d_batch_tunnel(Cells2DBatch* b, int32_t k, Cells2D** out);
 /* n steps of every tunnel: up to seven steps per launch, or, after cells2d_batch_set_launch, with a
  * workgroup_size, or when the autotuner found it faster, one launch per step (replayed from CUDA
- * graphs of 100 steps) or persistent launches of many steps. */
+ * graphs of 100 steps) or persistent launches of many steps. A single step, and the one or two last
+ * steps of a run without samples on a large grid, take one launch each as well. */
 int cells2d_batch_step(Cells2DBatch* b, int64_t n);
 /* n steps, then every tunnel's macro refresh, then wait. */
 int cells2d_batch_run(Cells2DBatch* b, int64_t n);

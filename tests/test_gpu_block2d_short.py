@@ -38,3 +38,29 @@ def test_remainders(precision, size, K):
     a, b = s.readPopulations(), np.ascontiguousarray(o.populations())
     assert np.array_equal(a.view(np.uint8), b.view(np.uint8))
     s.destroy()
+
+
+# How a caller groups its steps: in the fast build, single steps and runs round differently. Each step leaves at most 18
+# roundings of the largest population, which relaxation does not amplify. A fixed workgroup size takes one kernel.
+@pytest.mark.parametrize("workgroup", [0, 128])
+@pytest.mark.parametrize("precision,eps", [("fp32", 6e-8), ("fp64", 1.1e-16)])
+@pytest.mark.parametrize("size", [(64, 48), (400, 100), (905, 605)])
+def test_grouping_of_steps(workgroup, precision, eps, size):
+    W, H = size
+    out, n = [], 60
+    for counts in ((n,), (1,) * n, (7, 1, 2, 1, 1, 13, 5, 30)):
+        s = Solver.create(width=W, height=H, precision=precision, workgroupSize=workgroup, left=2, right=2, bottom=2,
+                          top=2, tau=0.56, uIn=0.05, smagorinsky=0.1)
+        sdf = g.empty_sdf(W, H)
+        g.add_circle(sdf, W, H, W / 4, H / 2, H / 9)
+        s.setSdf(sdf)
+        s.initField(perturbed_rest2(W, H, 1e-3))
+        for k in counts:
+            s.encodeSteps(k)
+        assert [v["step"] for v in s.readForces()] == list(range(1, n + 1))
+        out.append(s.readPopulations())
+        s.destroy()
+    for a in out[1:]:
+        if workgroup:
+            assert np.array_equal(a, out[0])
+        assert np.max(np.abs(a - out[0])) <= 2 * n * 18 * eps * np.max(np.abs(out[0]))
