@@ -53,6 +53,8 @@ void Device::close() {
   }
   for (void* p : owned) cudaFree(p);
   owned.clear();
+  arena = nullptr;
+  arenaBytes = arenaUsed = 0;
   if (ev0) cudaEventDestroy(ev0);
   if (ev1) cudaEventDestroy(ev1);
   if (evRead) cudaEventDestroy(evRead);
@@ -73,6 +75,11 @@ void* Device::alloc(size_t bytes, const char* what) {
     g_fake_live_buffers++;
     return p;
   }
+  if (reserved(bytes)) {
+    void* p = arena + arenaUsed;
+    arenaUsed += room(bytes);
+    return p;
+  }
   void* p = nullptr;
   cudaError_t e = cudaMalloc(&p, bytes);
   if (e != cudaSuccess) {
@@ -81,6 +88,15 @@ void* Device::alloc(size_t bytes, const char* what) {
   }
   owned.push_back(p);
   return p;
+}
+
+void Device::reserve(size_t bytes) {
+  if (fake || arena) return;
+  try {
+    arena = (char*)alloc(bytes, "buffers");
+    arenaBytes = bytes;
+  } catch (const AllocError&) {
+  }
 }
 
 void Device::h2d(void* d, const void* h, size_t bytes) {
@@ -162,7 +178,7 @@ void* Device::host_pinned(size_t bytes) {
 }
 
 void Device::release(void* d) {
-  if (!d) return;
+  if (!d || (arena && (char*)d >= arena && (char*)d < arena + arenaBytes)) return;  // the arena goes as a whole
   for (size_t k = 0; k < owned.size(); k++) {
     if (owned[k] != d) continue;
     owned.erase(owned.begin() + (long)k);

@@ -39,6 +39,13 @@ struct Device {
   void open(int device_ordinal, int fail_alloc_at);
   void close();
   void* alloc(size_t bytes, const char* what);
+  // One allocation that the following alloc() calls take their buffers from, until close, while they fit (a
+  // buffer's share of it is room(bytes)). A device that cannot give it allocates them one by one.
+  void reserve(size_t bytes);
+  bool reserved(size_t bytes) const { return arena && arenaUsed + room(bytes) <= arenaBytes; }
+  static size_t room(size_t bytes) { return (bytes + 255) / 256 * 256; }
+  char* arena = nullptr;
+  size_t arenaBytes = 0, arenaUsed = 0;
   void h2d(void* d, const void* h, size_t bytes);
   void d2h(void* h, const void* d, size_t bytes);
   // Device-to-host copy of a large buffer into pageable memory, waiting for it: through two pinned

@@ -145,9 +145,11 @@ struct Cells2DBatch : HandleBase {
   char* spare = nullptr;           // room for the layout and the force partials behind the rules
   size_t spareBytes = 0, spareUsed = 0;
   std::vector<void*> blockOwn;     // their own buffers where it does not suffice
-  static unsigned long long room(unsigned long long bytes) { return (bytes + 255) / 256 * 256; }
+  unsigned long long ruleBytes = 0;  // of the tables, the room behind them included
+  static unsigned long long room(unsigned long long bytes) { return Device::room((size_t)bytes); }
   bool pick_region(Region2& r, int& K, long long& tiles) const;
   unsigned long long partial_bytes(long long tiles, int K, int& steps) const;
+  void size_rules();
   void alloc_rules();
   void* block_alloc(size_t bytes, const char* what);
   unsigned long long buffer_limit() const;
@@ -406,17 +408,16 @@ unsigned long long Cells2DBatch::partial_bytes(long long tiles, int K, int& step
 // The block kernel's tables: one buffer for the batch, the layout and a run's force partials behind them, or, where
 // that exceeds the largest buffer that a tunnel's caller allows, one for each table. A device without room for them
 // steps one launch at a time.
-void Cells2DBatch::alloc_rules() {
-  if (dev.fake) return;
-  unsigned long long total = 0, limit = buffer_limit();
+void Cells2DBatch::size_rules() {
+  ruleBytes = spareBytes = 0;
   for (Tunnel2Host& T : t) {
     // coefficient slots for the cells around a body: a few times the grid's outline (further body cells
     // keep the general rules)
     T.qCap = (int)std::min<long long>(T.N, 4LL * (T.W + T.H));
     if (T.cfg.max_buffer_bytes > 0)
       T.qCap = (int)std::min<unsigned long long>((unsigned long long)T.qCap, T.cfg.max_buffer_bytes / (16 * bpp));
-    total += room((unsigned long long)T.N * 4) + room((unsigned long long)T.qCap * 16 * bpp) +
-             room(9ull * bpp * (unsigned long long)T.N);
+    ruleBytes += room((unsigned long long)T.N * 4) + room((unsigned long long)T.qCap * 16 * bpp) +
+                 room(9ull * bpp * (unsigned long long)T.N);
   }
   Region2 r;
   int K, steps;
@@ -424,12 +425,17 @@ void Cells2DBatch::alloc_rules() {
   if (blockWanted && pick_region(r, K, tiles))
     spareBytes = room(t.size() * sizeof(Block2Tunnel)) + room((unsigned long long)tiles * sizeof(unsigned short)) +
                  (samples_force() ? room(partial_bytes(tiles, K, steps)) : 0);
-  total += spareBytes;
-  if (total > limit) {
-    total -= spareBytes;
+  if (ruleBytes + spareBytes > buffer_limit()) spareBytes = 0;
+  ruleBytes += spareBytes;
+}
+
+void Cells2DBatch::alloc_rules() {
+  if (dev.fake) return;
+  const unsigned long long total = ruleBytes, limit = buffer_limit();
+  if (!dev.reserved(total) && total + (1u << 22) > dev.free_bytes()) {
     spareBytes = 0;
+    return;
   }
-  if (total + (1u << 22) > dev.free_bytes()) return;
   std::vector<void*> taken;
   char* p = nullptr;
   auto place = [&](unsigned long long bytes) {
@@ -765,6 +771,21 @@ void Cells2DBatch::free_all() {
 
 // ---------------- creation ----------------
 
+// The one-step kernel's tiles of a tunnel in the shape that has most.
+static int most_tiles(const Tunnel2Host& T) {
+  int most = 0;
+  for (const Shape2& sh : kShapes) most = std::max(most, ((T.W + sh.tx - 1) / sh.tx) * ((T.H + sh.ty - 1) / sh.ty));
+  return most;
+}
+
+// What create_batch allocates for a tunnel.
+static unsigned long long tunnel_bytes(const Tunnel2Host& T, size_t bpp) {
+  const unsigned long long N = (unsigned long long)T.N, W = (unsigned long long)T.W;
+  return 2 * Device::room((9 * N + W) * bpp) + 2 * Device::room(N * 4) + Device::room(N * 16) +
+         Device::room((size_t)most_tiles(T) * sizeof(double2)) + Device::room((size_t)HISTORY2_LEN * sizeof(double2)) +
+         Device::room(sizeof(DevState2)) + Device::room(W * 4 * bpp);
+}
+
 static Cells2DBatch* create_batch(const Cells2DConfig* cfgs, int count) {
   if (!cfgs || count <= 0) throw Error(CELLS_E_INVALID, "need at least one config");
   if (count > 65535) throw Error(CELLS_E_INVALID, "at most 65535 tunnels per batch");
@@ -806,6 +827,18 @@ static Cells2DBatch* create_batch(const Cells2DConfig* cfgs, int count) {
       maxTiles = std::max(maxTiles, tiles);
     }
     b->maxTiles = maxTiles;
+    b->blockWanted = cfgs[0].workgroup_size == 0;
+    b->size_rules();
+    // All buffers from one allocation: each of 2 MB or more takes the device 0.35 ms, smaller ones share pieces of 2 MB
+    // that earlier handles may have left. us to create a tunnel, one by one / together: 64x24 (0.5 MB) 337 / 240,
+    // 128x128 (2.3 MB) 390 / 610, 400x100 (6 MB) 750 / 600, 1000x250 (35 MB) 1,850 / 700, 4000x1000 4,400 / 2,600;
+    // a batch of 32 tunnels 48,000 / 12,000.
+    if (!b->dev.fake && b->buffer_limit() == ULLONG_MAX && total + b->ruleBytes <= freeB) {
+      unsigned long long bytes = b->ruleBytes + Cells2DBatch::room((size_t)count * sizeof(Tunnel2)) +
+                                 Cells2DBatch::room((size_t)maxTiles * sizeof(unsigned short)) + (1u << 14);
+      for (const Tunnel2Host& T : b->t) bytes += tunnel_bytes(T, b->bpp);
+      if (bytes < (2u << 20) || bytes >= (4u << 20)) b->dev.reserve((size_t)bytes);
+    }
     for (int k = 0; k < count; k++) {
       Tunnel2Host& T = b->t[(size_t)k];
       const size_t fBytes = 9ull * b->bpp * (size_t)T.N;
@@ -813,23 +846,13 @@ static Cells2DBatch* create_batch(const Cells2DConfig* cfgs, int count) {
       // takes them; on the top row direction 8's pull lands up to W - 1 elements past the nine
       // arrays, so each buffer carries W elements of padding (never used as a population)
       const size_t padBytes = (size_t)T.W * b->bpp;
-      if (b->dev.fake || cfgs[k].max_buffer_bytes > 0) {
-        T.f[0] = b->dev.alloc(fBytes + padBytes, "distribution buffer A");
-        T.f[1] = b->dev.alloc(fBytes + padBytes, "distribution buffer B");
-      } else {
-        // as one: every 2 MB begun, and every larger allocation, takes the device about 0.35 ms, and the tables of
-        // several steps per launch are one more (a batch of 32 tunnels: 47 ms apart, 38 as one)
-        const size_t each = (size_t)Cells2DBatch::room(fBytes + padBytes);
-        T.f[0] = b->dev.alloc(2 * each, "distribution buffers");
-        T.f[1] = (char*)T.f[0] + each;
-      }
+      T.f[0] = b->dev.alloc(fBytes + padBytes, "distribution buffer A");
+      T.f[1] = b->dev.alloc(fBytes + padBytes, "distribution buffer B");
       T.flags = (uint32_t*)b->dev.alloc((size_t)T.N * 4, "flags");
       T.sdf = (float*)b->dev.alloc((size_t)T.N * 4, "sdf");
       T.macro = (float4*)b->dev.alloc((size_t)T.N * 16, "macro");
-      int cap = 0;
-      for (const Shape2& sh : kShapes) cap = std::max(cap, ((T.W + sh.tx - 1) / sh.tx) * ((T.H + sh.ty - 1) / sh.ty));
-      T.partialsCap = cap;
-      T.partials = (double2*)b->dev.alloc((size_t)cap * sizeof(double2), "force partials");
+      T.partialsCap = most_tiles(T);
+      T.partials = (double2*)b->dev.alloc((size_t)T.partialsCap * sizeof(double2), "force partials");
       T.history = (double2*)b->dev.alloc((size_t)HISTORY2_LEN * sizeof(double2), "force history");
       T.st = (DevState2*)b->dev.alloc(sizeof(DevState2), "state");
       T.xtab = b->dev.alloc((size_t)T.W * 4 * b->bpp, "x table");
@@ -855,7 +878,6 @@ static Cells2DBatch* create_batch(const Cells2DConfig* cfgs, int count) {
     // 64 x 2, which the autotuner picked for a single 400 x 100 tunnel (cells2d_batch_autotune
     // retunes a batch for its own sizes)
     const int wg = cfgs[0].workgroup_size;
-    b->blockWanted = wg == 0;
     b->alloc_rules();
     if (wg == 0) {
       b->set_layout(64, 2, 0);
