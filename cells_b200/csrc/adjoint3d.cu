@@ -236,7 +236,8 @@ __device__ __forceinline__ void block_du_partial(double du, double* part, int sl
 // Programmatic dependent launch: waits for the boundary-element kernel of the step before to complete.
 // f^n, the tables and the flags do not depend on it, so the roles ask for them first: a segment's first adjoint
 // step is launched without the attribute (launch_adjoint_step3's `first`), after all work before it, the recompute
-// that wrote the segment's states included.
+// that wrote the segment's states included. lambda^{n+1} comes through L2 (__ldcg): the launch before may still write it
+// while these blocks are resident, which the read-only path does not allow for.
 __device__ __forceinline__ void adj_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 template <class R>
@@ -259,7 +260,7 @@ __device__ __forceinline__ double adj_cells_role(const AdjLaunch3& a, int tz) {
   const uint32_t fl = __ldg(&a.flags[idx]);
   adj_wait();
 #pragma unroll
-  for (int i = 0; i < Q3; i++) lp[i] = __ldg(&lamNext[i * N + idx]);
+  for (int i = 0; i < Q3; i++) lp[i] = __ldcg(&lamNext[i * N + idx]);
   if (fl != 0u) return 0.0;
   // interior cell: plain pulls, the collision's transposed Jacobian, plain pushes
   R lg[Q3];
@@ -296,7 +297,7 @@ __device__ __forceinline__ double adj_pairs_role(const AdjLaunch3& a, int tz) {
   const uint2 fl = __ldg(reinterpret_cast<const uint2*>(a.flags + idx));
   adj_wait();
 #pragma unroll
-  for (int i = 0; i < Q3; i++) lp[i] = __ldg(reinterpret_cast<const float2*>(lamNext + (i * N + idx)));
+  for (int i = 0; i < Q3; i++) lp[i] = __ldcg(reinterpret_cast<const float2*>(lamNext + (i * N + idx)));
   if (fl.x != 0u && fl.y != 0u) return 0.0;
   const float4* xt = (const float4*)a.xTab + x0;
   const float4 t0 = __ldg(xt), t1 = __ldg(xt + 1);
@@ -367,7 +368,7 @@ __device__ __forceinline__ double adj_face_pairs_role(const AdjLaunch3& a, int f
   }
   adj_wait();
 #pragma unroll
-  for (int i = 0; i < Q3; i++) lp[i] = __ldg(reinterpret_cast<const float2*>(lamNext + (i * N + idx)));
+  for (int i = 0; i < Q3; i++) lp[i] = __ldcg(reinterpret_cast<const float2*>(lamNext + (i * N + idx)));
   const float4* xt = (const float4*)a.xTab + x0;
   const float4 t0 = __ldg(xt), t1 = __ldg(xt + 1);
   float2 lg[Q3], dut;
@@ -450,7 +451,7 @@ __device__ __forceinline__ double adj_slow_role(const AdjLaunch3& a, int block, 
 #pragma unroll
   for (int k = 0; k < kItems; k++) {
     const int i = i0 + k * kDirs;
-    lp[k] = on && i < Q3 ? lamNext[i * N + idx] : R(0);
+    lp[k] = on && i < Q3 ? __ldcg(&lamNext[i * N + idx]) : R(0);
   }
 #pragma unroll
   for (int k = 0; k < kItems; k++) {

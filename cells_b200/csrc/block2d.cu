@@ -518,8 +518,10 @@ static cudaError_t launch_block2_t(const Block2Launch& a, cudaStream_t s) {
 }
 
 cudaError_t launch_block2(int precision, const Block2Launch& a, cudaStream_t s) {
-  if (precision == 0) return launch_block2_t<Store2F32>(a, s);
-  if (precision == 3) return launch_block2_t<Store2F64>(a, s);
+  // Populations through L2: a launch is resident while the one before it still writes them, which the read-only
+  // path does not allow for; a block reads each once.
+  if (precision == 0) return launch_block2_t<Store2F32P>(a, s);
+  if (precision == 3) return launch_block2_t<Store2F64P>(a, s);
   return cudaErrorInvalidValue;
 }
 
