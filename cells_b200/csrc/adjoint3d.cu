@@ -528,8 +528,9 @@ __global__ void __launch_bounds__(kAdjThreads, PAIR ? 4 : (sizeof(R) == 4 ? 5 : 
   __shared__ double red[kAdjThreads / 32];
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   const int tid = threadIdx.x + blockDim.x * threadIdx.y;
-  if ((int)blockIdx.z < a.roleZ) {
-    const int r = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
+  const int slice = a.slice0 + blockIdx.z;
+  if (slice < a.roleZ) {
+    const int r = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * slice);
     if (r >= a.nSlowBlocks + a.nFaceBlocks) return;
     double du = 0.0;
     if (r < a.nSlowBlocks) {
@@ -539,7 +540,7 @@ __global__ void __launch_bounds__(kAdjThreads, PAIR ? 4 : (sizeof(R) == 4 ? 5 : 
     }
     block_du_partial(du, a.blockPart, a.nCellBlocks + r, red, tid);
   } else {
-    const int tz = blockIdx.z - a.roleZ;
+    const int tz = slice - a.roleZ;
     if (tz + 1 < a.D - 2) adj_prefetch<R, (PAIR ? 2 : 1) * kAdjTileX>(a, tz + 1, tid);
     double du;
     if constexpr (PAIR)
@@ -628,6 +629,8 @@ cudaError_t launch_dependent(void (*fn)(Args...), dim3 grid, dim3 block, cudaStr
   return cudaLaunchKernelEx(&cfg, fn, args...);
 }
 
+constexpr unsigned kMaxSlices = 65535;  // of a grid's z
+
 // Interior-cell blocks of a step: x tiles of 32 cells (or 32 x-pairs), so each warp still reads
 // 128-byte rows and the tiles before the absorbing layer take the collision code without it.
 bool adj_pairs(int precision, int W) { return precision == 0 && W % 2 == 0; }
@@ -665,13 +668,16 @@ cudaError_t launch_adjoint_step3_t(AdjLaunch3 a, bool first, cudaStream_t s) {
   }
   const unsigned slice = cells.x * cells.y;
   a.roleZ = (int)(((unsigned)(a.nSlowBlocks + a.nFaceBlocks) + slice - 1) / slice);
-  if (a.roleZ + cells.z > 0) {
-    void (*fn)(AdjLaunch3) = adj_step3_kernel<R, false>;
-    if constexpr (sizeof(R) == 4) {
-      if (adj_pairs(precision, a.W)) fn = adj_step3_kernel<R, true>;
-    }
-    const cudaError_t e = launch_dependent(fn, dim3(cells.x, cells.y, a.roleZ + cells.z),
-                                           dim3(kAdjTileX, kAdjThreads / kAdjTileX), s, !first, a);
+  void (*fn)(AdjLaunch3) = adj_step3_kernel<R, false>;
+  if constexpr (sizeof(R) == 4) {
+    if (adj_pairs(precision, a.W)) fn = adj_step3_kernel<R, true>;
+  }
+  // a launch takes 65,535 slices: a thin grid of some 20,000 planes has more
+  const unsigned slices = a.roleZ + cells.z;
+  for (unsigned z0 = 0; z0 < slices; z0 += kMaxSlices) {
+    a.slice0 = (int)z0;
+    const cudaError_t e = launch_dependent(fn, dim3(cells.x, cells.y, std::min(slices - z0, kMaxSlices)),
+                                           dim3(kAdjTileX, kAdjThreads / kAdjTileX), s, !first || z0 > 0, a);
     if (e != cudaSuccess) return e;
   }
   if (a.nRows == 0) return cudaSuccess;

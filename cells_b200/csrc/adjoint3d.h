@@ -106,6 +106,7 @@ struct AdjLaunch3 {
   int absorbX0;          // first x of the absorbing layer (W when there is none)
   int nCellBlocks, nSlowBlocks, nFaceBlocks;  // blocks of the roles
   int roleZ;                                  // grid slices of the last two
+  int slice0;                                 // first slice of this launch
   int foff[4][cells::Q3];                     // face rows: element offset of direction i's source from the cell
   const int* slowCells;  // the flagged fluid cells, in index order
   int nSlow;

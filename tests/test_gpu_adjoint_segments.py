@@ -30,3 +30,24 @@ def test_one_segment_equals_short_segments(precision, W, H, D, steps):
         assert j == out[0][0] and o["du"] == out[0][1]["du"]
         for k in ("adjoint", "dsdf"):
             assert np.array_equal(o[k].view(np.uint8), out[0][1][k].view(np.uint8))
+
+
+# More slices of blocks than one launch holds: the adjoint step of a thin, deep grid goes out in two launches.
+@pytest.mark.parametrize("precision,size", [("fp64", (32, 3, 22000)), ("fp32", (64, 2, 20000))])
+def test_more_slices_than_a_launch_holds(precision, size):
+    W, H, D = size
+    out = []
+    for every in (3, 1):
+        s = Solver3D.create(W, H, D, precision=precision, tau=0.6, uIn=0.05, forceEvery=0)
+        sdf = g.empty_sdf3(W, H, D)
+        g.add_sphere(sdf, W, H, D, W / 3, 0.6, D - 40, 2.2)
+        s.setSdf(sdf)
+        s.initField()
+        s.encodeSteps(2)
+        first = s.step
+        s.adjointForward(3, first + 1, first + 3, checkpointEvery=every, component=0)
+        out.append(s.adjointBackward(wantAdjoint=True))
+        s.destroy()
+    for k in ("adjoint", "dsdf"):
+        assert np.any(out[0][k]) and np.array_equal(out[0][k].view(np.uint8), out[1][k].view(np.uint8))
+    assert out[0]["du"] == out[1]["du"]
