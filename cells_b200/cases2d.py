@@ -357,9 +357,9 @@ def batched_naca_tunnels(count: int = 64, seed: Optional[int] = None):
 
 def batched_naca_throughput(steps: int = 10000, device: int = 0, autotune: bool = True, warmup: int = 200,
                             count: int = 64) -> dict:
-    """MLUPS of the batched tunnels stepped together (one Batch2D, CUDA-graph or persistent
-    launches as the autotuner picks) and of the same tunnels stepped one at a time (one Solver
-    each, graph-replayed), both timed with CUDA events on the solvers' streams; the final
+    """MLUPS of the batched tunnels stepped together (one Batch2D: several steps per launch, CUDA graphs of the
+    one-step kernel or persistent launches, as the autotuner picks) and of the same tunnels stepped one at a
+    time (one Solver each, several steps per launch), both timed with CUDA events on the solvers' streams; the final
     populations of each tunnel, batched and alone, are compared (how many are bit for bit equal,
     and the largest difference)."""
     from .solver2d import Batch2D
@@ -373,9 +373,11 @@ def batched_naca_throughput(steps: int = 10000, device: int = 0, autotune: bool 
     launch = b.autotune(100) if autotune else b.info()
     b.step(warmup)
     b.synchronize()
+    launches = b.launchCount()
     b.timerStart()
     b.step(steps)
     ms_batch = b.timerStop()
+    launches = b.launchCount() - launches
     batched = [t.readPopulations() for t in b.tunnels]
     b.destroy()
     ms_seq = 0.0
@@ -399,7 +401,8 @@ def batched_naca_throughput(steps: int = 10000, device: int = 0, autotune: bool 
             "batched_ms": ms_batch, "sequential_ms": ms_seq,
             "bitwise_identical_tunnels": identical, "max_population_diff": max_diff,
             "finite": bool(all(np.all(np.isfinite(f)) for f in batched)),
-            "launch": {"tile": [launch["tile_x"], launch["tile_y"]], "persistent": bool(launch["persistent"])}}
+            "launch": {"steps_per_launch": round(steps / launches, 2), "one_step_tile": [launch["tile_x"], launch["tile_y"]],
+                       "persistent": bool(launch["persistent"])}}
 
 
 # ---------------------------------------------------------------- the 400 x 100 cylinder tunnel

@@ -1033,9 +1033,9 @@ int adj_parts(const Cells3D* h, int nSlow) {
 unsigned blocks_of(size_t n, unsigned b) { return (unsigned)((n + b - 1) / b); }
 
 // The list of flagged cells, their pull records, the links and the rows for the current flags and SDF.
-// Two ints come back to the host: the links with the cells' number, then the rows'. The per-element
-// scratch (one count and one row number per population element) lies in the recompute buffers, which
-// the sweep fills later.
+// Three ints come back to the host: the numbers of cells, links and rows. The per-element scratch (cnt and rowOf, a
+// count and a row number per population element) lies in the two adjoint states: a backward sweep has to clear them
+// before it starts, as it does.
 template <class R>
 void build_tables(Cells3D* h, Adjoint3D* A, int* cnt, int* rowOf) {
   cells::Device& dev = h->dev;
@@ -1325,7 +1325,7 @@ int cells3d_adjoint_forward(Cells3D* h, const Cells3DAdjointSpec* spec, double* 
   for (int64_t k = 0; k < nSeg; k++) A->ck.push_back(store + (size_t)k * stride);
   for (int set = 0; set < 2; set++)
     for (int k = 0; k < segBufs; k++) A->seg[set].push_back(store + (size_t)(nSeg + set * segBufs + k) * stride);
-  // the per-element scratch: the last checkpoint-sized places of the store (an f32 element is as wide as a
+  // the per-element scratch: the adjoint states' places, the last two of the store (an f32 element is as wide as a
   // count)
   if (h->prec == CELLS_FP64)
     build_tables<double>(h, A, (int*)(store + (size_t)(nSeg + 2 * segBufs) * stride),

@@ -91,7 +91,7 @@ struct AdjLaunch3 {
   const void* lamNext;   // lambda^{n+1}
   void* lamOut;          // lambda^n
   const uint32_t* flags;
-  const void* xTab;      // per x: omega+, omega-, sigma, 0
+  const void* xTab;      // per x: omega+, omega-, sigma, 1 / omega+
   const uint8_t* rowBody;
   const void* lcF;
   const void* lq;

@@ -28,7 +28,7 @@ Cells3D::~Cells3D() = default;
 
 // ---------------- helpers ----------------
 
-// Per-x table (omega+ without Smagorinsky, omega-, sigma, 0). The reference computes these per
+// Per-x table (omega+ without Smagorinsky, omega-, sigma, 1 / omega+). The reference computes these per
 // cell in f32 (src/shaders/step3d.ts:72-74 and :213-219); the same f32 operations in the same order
 // give the same values here (the host build does not contract multiply-adds).
 template <class R>

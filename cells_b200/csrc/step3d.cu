@@ -64,9 +64,9 @@ struct StepArgs3 {
   const uint32_t* flags;
   const float* sdf;
   const uint8_t* rowBody;
-  const typename Vec4<R>::T* xTab;  // per x: (omega+ without Smagorinsky, omega-, sigma, 0)
-  // per x-pair (x0 = 2j, x0 + 1), for f32 rates: entry 2j (omega+ of both, omega- of both),
-  // entry 2j + 1 (sigma of both, 0, 0); the same values as xTab, laid out so a pair's rates load
+  const typename Vec4<R>::T* xTab;  // per x: (omega+ without Smagorinsky, omega-, sigma, 1 / omega+)
+  // per x-pair (x0 = 2j, x0 + 1), for f32 rates: entry 2j (omega+ of both, omega- of both, or with
+  // Smagorinsky 1 / omega+ of both), entry 2j + 1 (sigma of both, 0, 0); the values of xTab, so a pair's rates load
   // as register pairs of the packed f32x2 collision
   const float4* xPair;
   BodyLinks3 links;
@@ -397,18 +397,6 @@ __device__ __noinline__ float2 smag_rates(float q, float ir, float t, float smag
 
 constexpr int kFarPair = 32;  // distance of the two cells of a thread at odd widths (f32)
 
-// The fast TRT collision of the two cells of an x-pair (cell x0 in .x, x0 + 1 in .y) with packed
-// f32x2 instructions, stored as one 32-bit word per population. It evaluates the lean pair form of
-// collide3 per component in f32: with s_p = f_p + f_p+1 and d_p = f_p - f_p+1 (exact for values
-// of 16-bit storage, whose sums and differences fit the f32 significand; rounded once for f32),
-//   o_p = S + T, o_p+1 = S - T,  S = (1 - omega+)/2 s_p + omega+ w (rho cu^2/2 + K0),
-//                                T = (1 - omega-)/2 d_p + omega- w rho cu,   K0 = drho - rho usq,
-// which is f_p + A + B and f_p+1 + A - B of collide3 rearranged, so only s_p and d_p stay live.
-// Only the reciprocal of rho, and with Smagorinsky the relaxation time, run per cell.
-// The inlet cell (x0 = 0, when IN) and the outlet cell (x0 + 1 = W - 1, when OUT) go through the
-// same instructions: with omega+ = omega- = 1, rho = 1, drho = 0 and no absorbing source the update
-// is exactly the equilibrium feq(1, u), at u = (uIn, 0, 0) for the inlet (step3d.ts:190-193) and at
-// the node's own velocity for the outlet.
 // DX: the distance of the two cells. 1: an x-pair, both stored as one word; kFarPair: cells of their own,
 // each stored when act0 / act1 is set (the other's values are computed and dropped).
 template <class C, int DX>
@@ -421,6 +409,18 @@ __device__ __forceinline__ void store2(typename C::S* p, float2 v, bool act0, bo
   }
 }
 
+// The fast TRT collision of the two cells of an x-pair (cell x0 in .x, x0 + 1 in .y) with packed
+// f32x2 instructions, stored by store2. It evaluates the lean pair form of
+// collide3 per component in f32: with s_p = f_p + f_p+1 and d_p = f_p - f_p+1 (exact for values
+// of 16-bit storage, whose sums and differences fit the f32 significand; rounded once for f32),
+//   o_p = S + T, o_p+1 = S - T,  S = (1 - omega+)/2 s_p + omega+ w (rho cu^2/2 + K0),
+//                                T = (1 - omega-)/2 d_p + omega- w rho cu,   K0 = drho - rho usq,
+// which is f_p + A + B and f_p+1 + A - B of collide3 rearranged, so only s_p and d_p stay live.
+// Only the reciprocal of rho runs per cell.
+// The inlet cell (x = 0, when IN) and the outlet cell (x = W - 1, when OUT) go through the
+// same instructions: with omega+ = omega- = 1, rho = 1, drho = 0 and no absorbing source the update
+// is exactly the equilibrium feq(1, u), at u = (uIn, 0, 0) for the inlet (step3d.ts:190-193) and at
+// the node's own velocity for the outlet.
 template <class C, bool SMAG, bool ABS, bool IN, bool OUT, int DX>
 __device__ __forceinline__ void collide3x2_store(const StepArgs3<C>& a, const typename C::Pair (&r)[Q3], int x0,
                                                  int idx, bool act0, bool act1) {
@@ -1143,8 +1143,8 @@ __device__ __forceinline__ void prefetch_tile_ahead(const StepArgs3<C>& a) {
 }
 
 // ALT: a.reverse may be set. f64 and the 16-bit x-pairs have kernels with and without it: what it changes in the
-// interior code costs grids that never reverse 3-4% in f64 (200x100x96 97.9 -> 102.5 us a step), 1-2% in bf16
-// (256x128x128 59.2 -> 60.6), nothing in f32.
+// interior code costs grids that never reverse 3-4% in f64 (200x100x96 97.9 -> 102.5 us a step), 1.4% in bf16
+// (256x128x128 57.9 -> 58.7, 224x112x112 45.6 -> 46.2), nothing in f16 and f32.
 template <class C, bool SMAG, int PAIR, bool ALT>
 __global__ void __launch_bounds__(kStepThreads, step_min_blocks<C>(PAIR != 0))
     step3d_kernel(const __grid_constant__ StepArgs3<C> a) {
