@@ -1356,6 +1356,7 @@ int cells3d_adjoint_forward(Cells3D* h, const Cells3DAdjointSpec* spec, double* 
   // (launched step by step: a step takes the GPU several times as long as its launch takes the host,
   // and capturing K-step graphs anew for every recorded run cost more than they saved)
   int samples = 0;
+  const bool split = h->split_run(nWin);
   for (int64_t n = 0; n < A->steps; n++) {
     if (n % A->K == 0) {
       const int64_t k = n / A->K;
@@ -1367,7 +1368,7 @@ int cells3d_adjoint_forward(Cells3D* h, const Cells3DAdjointSpec* spec, double* 
     }
     const int64_t label = s0 + n + 1;
     const bool sample = label >= A->w0 && label <= A->w1;
-    h->enqueue_run_step(sample, n + 1 == A->steps, samples);
+    h->enqueue_run_step(sample, n + 1 == A->steps, split, samples);
     h->parity ^= 1;
     h->step++;
     if (sample) h->forceSteps.push_back((uint32_t)h->step);

@@ -235,10 +235,25 @@ void Cells3D::enqueue_step(int par, bool sample, int sampled) {
   launch_step(a, dev.stream);
 }
 
-// The next step of a run of steps launched one by one, `samples` of which wait for their sum; the
-// last one adds them up.
-void Cells3D::enqueue_run_step(bool sample, bool last, int& samples) {
-  const bool split = sample && (!last || samples > 0) && run_partials(kGraphSteps);
+// Whether the force partials of `samples` steps launched one by one are summed by one kernel after them. That kernel
+// takes 4 to 6 us that overlap nothing, and what it saves a step is the block count and the last block's sum, where
+// the step waits for them. us for 2 / 3 / 8 / 100 steps with a sample each, in the step -> after the run:
+//   f32  48x24x24 17 25 67 843 -> 17 21 51 644, 96x48x48 20 30 81 1009 -> 19 27 66 786, 128x64x64 27 40 106 1321 ->
+//        28 40 100 1186, 160x80x80 53 80 213 2666 -> 60 86 220 2679
+//   f16  48x24x24 18 28 74 926 -> 21 31 77 925, 96x48x48 22 33 87 1084 -> 23 33 82 996, 128x64x64 24 36 95 1187 -> 25
+//        35 87 1052, 160x80x80 37 55 147 1842 -> 42 60 152 1827
+//   f64  48x24x24 16 24 64 804 -> 17 22 53 622, 96x48x48 26 38 101 1268 -> 29 41 105 1257
+// Without a body there is nothing to wait for: 64x32x32 12 18 47 -> 15 20 47.
+bool Cells3D::split_run(int64_t samples) {
+  const long long work = bpp == 8 ? 4 * N : N;
+  const bool waits = work <= 600000 && (bpp != 2 || N >= 100000);
+  return nBody > 0 && samples >= (!waits ? 48 : (bpp != 2 && work <= 300000 ? 2 : 3)) && run_partials(kGraphSteps);
+}
+
+// The next step of a run of steps launched one by one, `samples` of which wait for their sum (split: split_run of
+// the run); the last one adds them up.
+void Cells3D::enqueue_run_step(bool sample, bool last, bool split, int& samples) {
+  split = split && sample;
   enqueue_step(parity, sample, split ? samples : -1);
   dev.launches++;
   if (split) samples++;
@@ -336,6 +351,7 @@ void Cells3D::launch_steps(int64_t n) {
   const int every = cfg.force_every;
   const int period = graph_period();
   int samples = 0;  // sampled steps launched one by one, whose partials wait for their sum
+  bool alone = false, split = false;
   while (n > 0) {
     if (!dev.fake && useGraphs && period <= kMaxGraphPeriod && n >= kGraphSteps) {
       // kGraphSteps steps as one graph launch: parity and sampling depend on step % period only
@@ -360,8 +376,9 @@ void Cells3D::launch_steps(int64_t n) {
         st->sample = s + 1;
       }
     } else {
-      // a single step reduces its force itself; the partials of a run are summed once
-      enqueue_run_step(sample, n == 1, samples);
+      if (!alone) split = every > 0 && split_run((step + n) / every - step / every);
+      alone = true;  // the rest of the run goes out step by step
+      enqueue_run_step(sample, n == 1, split, samples);
     }
     parity ^= 1;
     step++;

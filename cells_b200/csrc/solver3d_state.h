@@ -129,7 +129,8 @@ struct Cells3D : cells::HandleBase {
   // runPartials (run_partials), or reduce them in the step itself when sampled is -1
   void enqueue_step(int par, bool sample, int sampled);
   bool run_partials(int samples);
-  void enqueue_run_step(bool sample, bool last, int& samples);
+  bool split_run(int64_t samples);
+  void enqueue_run_step(bool sample, bool last, bool split, int& samples);
   void sum_samples(int samples);
   cells::StepLaunch3 step_launch(const void* src, void* dst, int par, bool sample) const;
   void launch_step(const cells::StepLaunch3& a, cudaStream_t stream);
