@@ -616,7 +616,18 @@ void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample, bool end) 
 // gain: 3 steps 2000x500 58.5 / 62.1, 4000x1000 205 / 234, 4 steps 78 / 82, 273 / 291, 8 steps 156 / 136, 545 / 503
 // (FP64 4000x1000, 3 steps 561 / 421).
 int64_t Cells2DBatch::block_steps(int64_t n, bool sampled) const {
-  if (sampled || (blockList && regionX * regionY < 64 * 48)) return n;
+  if (blockList && regionX * regionY < 64 * 48) return n;
+  if (sampled) {
+    // The one-step kernel counts a tunnel's blocks one after another, 7 ns each; a launch of a single step costs about
+    // its time without samples (18 ps a cell) again. Two steps of a large batch of small tunnels are the case for it:
+    // 64 NACA tunnels 313 / 442 (FP64 768 / 807), six of them 45 / 42, 4000x1000 383 / 295.
+    long long cells = 0, most = 0;
+    for (const Tunnel2Host& T : t) {
+      cells += T.N;
+      most = std::max<long long>(most, T.nTiles);
+    }
+    return n == 2 && cells >= 2000000 && most * 390 < cells ? 0 : n;
+  }
   if (n < blockK && !blockList && prec == CELLS_FP32) return 0;
   const int64_t full = n / blockK * blockK, rest = n - full;
   return full + (rest < 3 ? 0 : (rest - 1) | 1);

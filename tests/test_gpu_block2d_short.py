@@ -5,7 +5,7 @@ import numpy as np
 import pytest
 
 import cells_b200.geometry as g
-from cells_b200 import Solver
+from cells_b200 import Batch2D, Solver
 from cells_b200.rng import perturbed_rest2
 from oracle.oracle import OracleSolver2D
 
@@ -64,3 +64,31 @@ def test_grouping_of_steps(workgroup, precision, eps, size):
         if workgroup:
             assert np.array_equal(a, out[0])
         assert np.max(np.abs(a - out[0])) <= 2 * n * 18 * eps * np.max(np.abs(out[0]))
+
+
+# Two sampled steps of a large batch of small tunnels: one by one, as a single tunnel of as many cells does not
+@pytest.mark.parametrize("sizes,one_by_one", [([(500, 200)] * 24, True), ([(2400, 1000)], False)])
+def test_two_sampled_steps(sizes, one_by_one):
+    cfg = dict(left=2, right=2, bottom=2, top=2, tau=0.56, uIn=0.05, exactArithmetic=True)
+    b = Batch2D([dict(cfg, width=W, height=H) for W, H in sizes])
+    W, H = sizes[0]
+    sdf = g.empty_sdf(W, H)
+    g.add_circle(sdf, W, H, W / 4, H / 2, H / 9)
+    m = perturbed_rest2(W, H, 1e-3)
+    for t in b.tunnels:
+        t.setSdf(sdf)
+        t.initField(m)
+    before = b.launchCount()
+    b.step(2)
+    assert b.launchCount() - before == (2 if one_by_one else 3)  # and the force sums
+    b.step(7)
+    b.step(2)
+    o = OracleSolver2D(width=W, height=H, **{k: v for k, v in cfg.items() if k != "exactArithmetic"})
+    o.setSdf(sdf)
+    o.initField(m)
+    o.encodeSteps(11)
+    f = np.ascontiguousarray(o.populations())
+    for t in {0: b.tunnels[0], len(sizes) - 1: b.tunnels[-1]}.values():
+        assert np.array_equal(t.readPopulations().view(np.uint8), f.view(np.uint8))
+        assert [v["step"] for v in t.readForces()] == list(range(1, 12))
+    b.destroy()
