@@ -130,7 +130,11 @@ __global__ void links3_kernel(AuxLaunch3 a, const int* __restrict__ cells, int n
     uint8_t kind = LINK_LOAD;
     long long e1 = 0, e2 = -1;
     R k1 = R(0), k2 = R(0);
-    if ((fl & (1u << i)) == 0u) {
+    if (fl & FLAG3_INLET) {
+      // the inlet stores the inflow equilibrium: its pulls are dropped, and their sources before x = 0 lie outside
+      // the grid, for the cell (0, 0, 0) outside the buffers
+      e1 = (long long)i * N + idx;
+    } else if ((fl & (1u << i)) == 0u) {
       e1 = (long long)i * N + at(sx, sy, sz);
     } else {
       const bool outX = sx < 0 || sx >= W;
