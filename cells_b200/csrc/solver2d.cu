@@ -1598,6 +1598,13 @@ int cells2d_batch_autotune(Cells2DBatch* b, int32_t trial_steps, Cells2DInfo* in
         check_cuda(cudaMemcpyAsync((char*)p + 9ull * b->bpp * (size_t)T.N, T.st, sizeof(DevState2),
                                    cudaMemcpyDeviceToDevice, b->dev.stream),
                    "snapshot copy");
+        // the trials write the other buffer: what cells that become solid next keep of it is saved as well
+        if (T.prev && !T.prevValid) {
+          check_cuda(cudaMemcpyAsync(T.prev, T.f[b->parity ^ 1], 9ull * b->bpp * (size_t)T.N, cudaMemcpyDeviceToDevice,
+                                     b->dev.stream),
+                     "snapshot copy");
+          T.prevValid = true;
+        }
       }
       float best = 1e30f;
       Shape2 bestShape = {b->tileX, b->tileY};

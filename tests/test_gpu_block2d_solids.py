@@ -6,7 +6,7 @@ import numpy as np
 import pytest
 
 import cells_b200.geometry as g
-from cells_b200 import Solver
+from cells_b200 import Batch2D, Solver
 from cells_b200.rng import perturbed_rest2
 from oracle.oracle import OracleSolver2D
 
@@ -94,3 +94,25 @@ def test_rebuilds_between_runs(precision, before):
         x.encodeSteps(5)
     assert equal(s, o)
     s.destroy()
+
+
+# the autotuner's trials step the flow and restore it: a body drawn after them finds both buffers as they were
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+@pytest.mark.parametrize("before", [4, 7])
+def test_body_after_autotune(precision, before):
+    W, H = SMALL
+    cfg = dict(left=2, right=2, bottom=2, top=2, tau=0.56, uIn=0.05)
+    b = Batch2D([dict(cfg, width=W, height=H, precision=precision, exactArithmetic=True)])
+    o = OracleSolver2D(width=W, height=H, precision=precision, **cfg)
+    t, m = b.tunnels[0], perturbed_rest2(W, H, 1e-3)
+    t.initField(m)
+    o.initField(m)
+    b.step(before)
+    o.encodeSteps(before)
+    b.autotune(11)
+    for x in (t, o):
+        x.brush(30, 1, 3.2, False, True)
+    b.step(5)
+    o.encodeSteps(5)
+    assert equal(t, o)
+    b.destroy()
