@@ -243,11 +243,22 @@ void Cells3D::enqueue_step(int par, bool sample, int sampled) {
 //   f16  48x24x24 18 28 74 926 -> 21 31 77 925, 96x48x48 22 33 87 1084 -> 23 33 82 996, 128x64x64 24 36 95 1187 -> 25
 //        35 87 1052, 160x80x80 37 55 147 1842 -> 42 60 152 1827
 //   f64  48x24x24 16 24 64 804 -> 17 22 53 622, 96x48x48 26 38 101 1268 -> 29 41 105 1257
-// Without a body there is nothing to wait for: 64x32x32 12 18 47 -> 15 20 47.
+// Without a body there is nothing to wait for: 64x32x32 12 18 47 -> 15 20 47. These bodies are spheres of 294 to 3,406
+// cells. Where their steps do not wait, those with many body blocks do; a cylinder across the grid, 8 / 40 steps:
+//   f16  64x32x32 (88 blocks) 81 408 -> 73 356, 144x70x70 (391) 151 751 -> 151 734, 192x96x96 (703) 313 1562 -> 313 1525
+//   f32  192x96x96 439 2200 -> 439 2171;  f64  96x48x48 (190) 117 582 -> 116 561
 bool Cells3D::split_run(int64_t samples) {
+  if (nBody == 0) return false;
   const long long work = bpp == 8 ? 4 * N : N;
-  const bool waits = work <= 600000 && (bpp != 2 || N >= 100000);
-  return nBody > 0 && samples >= (!waits ? 48 : (bpp != 2 && work <= 300000 ? 2 : 3)) && run_partials(kGraphSteps);
+  const int blocks = fast::body_blocks3(nBody);
+  int from = 48;
+  if (work <= 600000 && (bpp != 2 || N >= 100000))
+    from = bpp != 2 && work <= 300000 ? 2 : 3;
+  else if (N < 100000 && blocks >= 80)
+    from = 4;
+  else if (blocks >= 160)
+    from = 12;
+  return samples >= from && run_partials(kGraphSteps);
 }
 
 // The next step of a run of steps launched one by one, `samples` of which wait for their sum (split: split_run of

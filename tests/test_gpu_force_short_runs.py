@@ -46,3 +46,24 @@ def test_launches(size, body, launches):
         assert s.launchCount() - before == want
     assert [v["step"] for v in s.readForces()] == list(range(1, sum(launches) + 1))
     s.destroy()
+
+
+# a cylinder across the grid: many body blocks, for whose count the steps of a larger grid or of FP16 wait after all
+@pytest.mark.parametrize("precision,size,launches", [("fp16", (64, 32, 32), {3: 3, 4: 5}), ("fp32", (160, 80, 80), {11: 11, 12: 13})])
+def test_launches_with_a_large_body(precision, size, launches):
+    W, H, D = size
+    x, y = np.meshgrid(np.arange(W), np.arange(H))
+    sdf = np.tile((np.hypot(x - W / 4, y - H / 2 - 0.3) - 0.12 * H).astype(np.float32).reshape(-1), D)
+    out = []
+    for alone in (False, True):
+        s = Solver3D.create(W, H, D, precision=precision, tau=0.56, uIn=0.05, forceEvery=1)
+        s.setSdf(sdf)
+        s.initField()
+        for n, want in launches.items():
+            before = s.launchCount()
+            for _ in range(n if alone else 1):
+                s.encodeSteps(1 if alone else n)
+            assert s.launchCount() - before == (n if alone else want)
+        out.append((s.readPopulations(), s.readForces()))
+        s.destroy()
+    assert np.array_equal(out[0][0].view(np.uint8), out[1][0].view(np.uint8)) and out[0][1] == out[1][1]
