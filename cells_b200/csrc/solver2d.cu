@@ -607,14 +607,15 @@ void Cells2DBatch::launch_blocks(int64_t n, int par, int allowSample, bool end) 
   }
 }
 
-// How many of n steps the block kernel takes: all, or all but the one or two that no odd number of steps holds. A
-// launch of a single step costs it the margins and a load through shared memory: with samples it still beats
+// How many of n steps the block kernel takes: all, or in a short run all but the one or two that no odd number of
+// steps holds. A launch of a single step costs it the margins and a load through shared memory: with samples it still beats
 // the one-step kernel (which counts its blocks), and on the small regions it does by the overlap of the launches.
 // us for 2 steps without samples, one-step / block: 128x128 11.8 / 10.2, 400x100 14.7 / 12.6; 1000x250 (64x48 with a
 // list) 19.7 / 22.9, 2000x500 39 / 64, 4000x1000 137 / 281; FP64 1000x250 (without a list) 21.9 / 30.4. With
 // samples: 1000x250 43 / 28, 4000x1000 383 / 295, FP64 620 / 533. Without a list FP32 needs a launch of K steps to
 // gain: 3 steps 2000x500 58.5 / 62.1, 4000x1000 205 / 234, 4 steps 78 / 82, 273 / 291, 8 steps 156 / 136, 545 / 503
-// (FP64 4000x1000, 3 steps 561 / 421).
+// (FP64 4000x1000, 3 steps 561 / 421). Beyond two launches of K the difference is below 1%, and a run of one kernel
+// rounds in one way.
 int64_t Cells2DBatch::block_steps(int64_t n, bool sampled) const {
   if (blockList && regionX * regionY < 64 * 48) return n;
   if (sampled) {
@@ -628,6 +629,7 @@ int64_t Cells2DBatch::block_steps(int64_t n, bool sampled) const {
     }
     return n == 2 && cells >= 2000000 && most * 390 < cells ? 0 : n;
   }
+  if (n > 2 * blockK + 2) return n;
   if (n < blockK && !blockList && prec == CELLS_FP32) return 0;
   const int64_t full = n / blockK * blockK, rest = n - full;
   return full + (rest < 3 ? 0 : (rest - 1) | 1);

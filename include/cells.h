@@ -433,8 +433,8 @@ void cells2d_batch_destroy(Cells2DBatch* b);
 int cells2d_batch_tunnel(Cells2DBatch* b, int32_t k, Cells2D** out);
 /* n steps of every tunnel: up to seven steps per launch, or, after cells2d_batch_set_launch, with a
  * workgroup_size, or when the autotuner found it faster, one launch per step (replayed from CUDA
- * graphs of 100 steps) or persistent launches of many steps. A single step, and the one or two last
- * steps of a run without samples on a large grid, take one launch each as well. */
+ * graphs of 100 steps) or persistent launches of many steps. A single step, and single
+ * steps of runs of up to twelve without samples on large grids, take one launch each as well. */
 int cells2d_batch_step(Cells2DBatch* b, int64_t n);
 /* n steps, then every tunnel's macro refresh, then wait. */
 int cells2d_batch_run(Cells2DBatch* b, int64_t n);

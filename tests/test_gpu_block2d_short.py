@@ -92,3 +92,18 @@ def test_two_sampled_steps(sizes, one_by_one):
         assert np.array_equal(t.readPopulations().view(np.uint8), f.view(np.uint8))
         assert [v["step"] for v in t.readForces()] == list(range(1, 12))
     b.destroy()
+
+
+# a longer run goes through one kernel whatever its remainder: the same bits as its steps in launches of one
+@pytest.mark.parametrize("size", [(500, 300), (905, 605)])
+def test_longer_runs_take_one_kernel(size):
+    W, H = size
+    out = []
+    for counts in ((16, 17), (15, 13, 5)):
+        s = Solver.create(width=W, height=H, left=2, right=2, bottom=2, top=2, tau=0.56, uIn=0.05, forceEvery=0)
+        s.initField(perturbed_rest2(W, H, 1e-3))
+        for n in counts:
+            s.encodeSteps(n)
+        out.append(s.readPopulations())
+        s.destroy()
+    assert np.array_equal(out[0], out[1])
