@@ -204,8 +204,8 @@ bool Cells3D::run_partials(int samples) {
   if (cfg.max_buffer_bytes > 0) most = std::min<size_t>(most, (size_t)(cfg.max_buffer_bytes / sizeof(double4)));
   if (dev.fake || runPartialsOff || need > most) return false;
   if (need > runPartialCap) {
-    // for as many body cells as the link tables hold, so that both grow together
-    const size_t cap = std::max(need, std::min(most, (size_t)samples * (size_t)fast::body_blocks3(links.cap)));
+    // with room for a body that moves and has now more cells, now fewer
+    const size_t cap = std::max(need, std::min(most, need + need / 4 + 1024));
     dev.release(runPartials);
     runPartials = nullptr;
     runPartialCap = 0;
